@@ -6,9 +6,9 @@
 // saturated regime, where the rank k approaches n and the Jacobi route's
 // O(n k^2)-per-sweep cost dominates).  FormLambda1/FormGamma1/FormGamma2 read
 // only the first chi singular values and vectors, so only those are computed:
-//   1. ZGEBD2 semantics: Q^H Theta P = B, B real upper bidiagonal (ZLARFG makes
-//      beta real), left reflectors H(i) = I - tauq v v^H below the diagonal,
-//      right reflectors G(i) = I - taup u u^H (u also copied column-wise to aux).
+//   1. (gebrd.cu) ZGEBD2 semantics: Q^H Theta P = B, B real upper bidiagonal (ZLARFG
+//      makes beta real), left reflectors H(i) = I - tauq v v^H below the diagonal,
+//      right reflectors G(i) = I - taup u u^H (u column-wise in aux).
 //   2. Singular values of B: bisection with Sturm counts on the Golub-Kahan
 //      tridiagonal (zero diagonal, off-diagonals d0,e0,d1,...,d_{n-1}; its
 //      eigenvalues are +-sigma), one thread per kept value, stopped at relative
@@ -22,7 +22,7 @@
 //   4. U = Q [Ub; 0], V = P Vb by applying the reflectors in reverse, one warp per
 //      kept column; X(:,i) = U(:,i) sigma_i, V(:,i), the same layout the sort and
 //      restore kernels read from the Jacobi routes.
-// All arithmetic is FP64.  Cost: 32/3 n^3 (bidiagonalisation) + 16 (m+n) n chi'
+// Steps 2 to 4 are FP64, step 1 64-bit fixed point.  Cost: 32/3 n^3 (bidiagonalisation) + 16 (m+n) n chi'
 // (back-transformation) instead of the Jacobi route's many O(n k^2) sweeps.
 #include <cooperative_groups.h>
 #include <math.h>
@@ -36,7 +36,6 @@
 namespace tebd {
 
 namespace {
-constexpr int kBW = 16;   // warps per CTA of the bidiagonalisation kernel
 
 __device__ __forceinline__ double bsum(double v) {
 #pragma unroll
@@ -64,738 +63,8 @@ __host__ __device__ __forceinline__ size_t bd_scratch(int n, int kk) {
 
 }  // namespace
 
-// ---------------------------------------------------------------------------
-// 1. Householder bidiagonalisation of the M x N matrix in S.X (ld M), M >= N,
-//    in panels of kPanel columns (the delayed-update scheme of LAPACK's ZGEBRD /
-//    ZLABRD).  Inside a panel the trailing matrix keeps its panel-start values A0
-//    and the current matrix is A0 - V Y^H - Xp U^H, with v_k, u_k the panel's
-//    left/right reflectors, y_k = tauq_k A^H v_k and x_k = taup_k A u_k.  Each
-//    column costs two read-only passes over A0 (z = A0^H v, w = A0 u) plus
-//    rank-2j corrections; at the panel end A0 <- A0 - V Y^H - Xp U^H.
-//    One cluster per bond, four cluster barriers per column:
-//      S1  column i corrected and its norm partials posted
-//      S2  z = A0^H v and the small dots V^H v, Xp^H v posted
-//      S3  y_i and row i corrected, row-norm partials posted, v_i stored
-//      S4  w = A0 u by column chunks, Y^H u and U^H u posted, u_i stored
-//    Every CTA recomputes the reflector scalars from the posted partial norms
-//    (same values, same order), so no barrier waits on a single CTA's scalar work.
-//    Output (as ZGEBD2): d, e in bdws; tauq in S.tau, v_i below the diagonal of
-//    column i; taup in S.taup, u_i in column i of Pv with u_i(i+1) = 1.
-// ---------------------------------------------------------------------------
-constexpr int kDfLoads = 8;  // loads in flight per lane in the double-float passes
-constexpr int kPanel = 8;   // columns per panel (narrow: the per-column corrections grow with it)
-constexpr int kChunk = 32;  // columns per task of the w = A0 u pass
-constexpr int kTile = 64;   // trailing-update tile (rows and columns)
-constexpr int kKc = 16;     // trailing-update k chunk staged in shared memory
-constexpr int kS = kTile + 8;  // staging stride (doubles): a fragment load is two wavefronts
-constexpr size_t kStageDoubles = 4 * (size_t)kKc * kS;
-
-// D += A B on the FP64 tensor pipe: mma m8n8k4, one A element (row lane/4, col lane%4),
-// one B element (row lane%4, col lane/4), two D elements (row lane/4, cols 2(lane%4)+{0,1})
-__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
-struct BdAux {
-  double2 *Pv, *Yb, *Xb, *zb, *s1, *s2, *t1, *t2, *part;
-  double *nrmL, *nrmR;
-};
-
-__host__ __device__ __forceinline__ size_t bd_aux_elems(int M, int N) {
-  const int P = N < kPanel ? N : kPanel;
-  return (size_t)N * N + (size_t)(N + M) * P + N + 4 * (size_t)P +
-         (size_t)((N + kChunk - 1) / kChunk) * M + 16;
-}
-
-__device__ __forceinline__ BdAux bd_aux(double2 *aux, int M, int N) {
-  const int P = min(kPanel, N);
-  BdAux a;
-  size_t o = 0;
-  a.Pv = aux;
-  o += (size_t)N * N;
-  a.Yb = aux + o;  // N x P, ld N
-  o += (size_t)N * P;
-  a.Xb = aux + o;  // M x P, ld M
-  o += (size_t)M * P;
-  a.zb = aux + o;
-  o += N;
-  a.s1 = aux + o;
-  a.s2 = a.s1 + P;
-  a.t1 = a.s2 + P;
-  a.t2 = a.t1 + P;
-  o += 4 * (size_t)P;
-  a.part = aux + o;  // ceil(N / kChunk) x M
-  o += (size_t)((N + kChunk - 1) / kChunk) * M;
-  a.nrmL = reinterpret_cast<double *>(aux + o);  // 8 per-CTA partial norms each
-  a.nrmR = a.nrmL + 8;
-  return a;
-}
-
-__device__ __forceinline__ double2 ldc(const double2 *p) { return __ldcg(p); }
-
-// acc += conj(a) b
-__device__ __forceinline__ void mac_ca(double2 &acc, double2 a, double2 b) {
-  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-// acc += a b
-__device__ __forceinline__ void mac(double2 &acc, double2 a, double2 b) {
-  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
-}
-// acc -= a b
-__device__ __forceinline__ void msub(double2 &acc, double2 a, double2 b) {
-  acc.x = fma(-a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(-a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-// acc -= a conj(b)
-__device__ __forceinline__ void msub_cb(double2 &acc, double2 a, double2 b) {
-  acc.x = fma(-a.x, b.x, fma(-a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-
-// ZLARFG's scalars from alpha and ||x||^2: beta (real), tau, and 1/(alpha - beta),
-// the factor that turns x into the reflector's tail.
-__device__ void larfg_scalars(double2 alpha, double xn2, double &beta, double2 &tau, double2 &sc) {
-  if (xn2 == 0.0 && alpha.y == 0.0) {  // H = I, x left as it is
-    beta = alpha.x;
-    tau = make_double2(0.0, 0.0);
-    sc = make_double2(1.0, 0.0);
-    return;
-  }
-  beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
-  tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-  const double dr = alpha.x - beta, di = alpha.y, den = dr * dr + di * di;
-  sc = make_double2(dr / den, -di / den);
-}
-
-// CTA-wide sum, valid in every thread
-__device__ double block_sum(double v, double *red) {
-  v = bsum(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  return t;
-}
-
-__global__ void __launch_bounds__(kBW * 32) k_gebrd(Slot *slots, const int *path) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;  // uniform per cluster
-  const Slot S = slots[s];
-  int M, N;
-  bd_dims(*S.cp, route, M, N);
-  double2 *A = S.X;
-  double *dd = S.bdws, *ee = S.bdws + N;
-  const BdAux ax = bd_aux(S.aux, M, N);
-  const int C = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int gt = crank * nthr + tid, gthr = C * nthr;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int gw = crank * (nthr >> 5) + warp, nw = C * (nthr >> 5);
-  extern __shared__ double2 sh[];
-  double2 *vec = sh;                    // max(M, N): v or u of the current column
-  double2 *sm = sh + max(M, N);         // 4 kPanel small per-column vectors
-  double *stg = reinterpret_cast<double *>(sm + 4 * kPanel);  // trailing-update staging
-  __shared__ double red[32];
-#define AE(r, c) A[(size_t)(r) + (size_t)M * (c)]
-#define YB(c, k) ax.Yb[(size_t)(c) + (size_t)N * (k)]
-#define XB(r, k) ax.Xb[(size_t)(r) + (size_t)M * (k)]
-#define PV(c, k) ax.Pv[(size_t)(c) + (size_t)N * (k)]
-  {  // norm partials of column 0 below the diagonal
-    double acc = 0.0;
-    for (int r = 1 + gt; r < M; r += gthr) {
-      const double2 a = ldc(&AE(r, 0));
-      acc = fma(a.x, a.x, fma(a.y, a.y, acc));
-    }
-    acc = block_sum(acc, red);
-    if (tid == 0) ax.nrmL[crank] = acc;
-  }
-  cluster.sync();
-  for (int p = 0; p < N; p += kPanel) {
-    const int jb = min(kPanel, N - p);
-    for (int j = 0; j < jb; ++j) {
-      const int i = p + j;
-      // ---- left reflector of column i (every CTA, identical inputs) ----
-      double beta;
-      double2 tau, sc;
-      {
-        double xn2 = 0.0;
-        for (int q = 0; q < C; ++q) xn2 += __ldcg(&ax.nrmL[q]);
-        larfg_scalars(ldc(&AE(i, i)), xn2, beta, tau, sc);
-      }
-      if (crank == 0 && tid == 0) {
-        dd[i] = beta;
-        S.tau[i] = tau;
-      }
-      if (i == N - 1) {  // last column: left reflector only
-        for (int r = i + 1 + gt; r < M; r += gthr) AE(r, i) = cmul(ldc(&AE(r, i)), sc);
-        break;
-      }
-      // ---- S2: z = A0(i:M, i+1:N)^H v, s1 = V^H v, s2 = Xp^H v ----
-      for (int r = i + tid; r < M; r += nthr)
-        vec[r - i] = r == i ? make_double2(1.0, 0.0) : cmul(ldc(&AE(r, i)), sc);
-      __syncthreads();
-      {
-        const int ncol = N - i - 1, items = ncol + 2 * j;
-        for (int it = gw; it < items; it += nw) {
-          const double2 *col = it < ncol       ? &AE(0, i + 1 + it)
-                               : it < ncol + j ? &AE(0, p + (it - ncol))
-                                               : &XB(0, it - ncol - j);
-          double2 acc = make_double2(0.0, 0.0);  // sum_r conj(col(r)) v(r)
-          int r = i + lane;
-          for (; r + 224 < M; r += 256) {
-            double2 c[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) c[q] = ldc(col + r + 32 * q);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) mac_ca(acc, c[q], vec[r + 32 * q - i]);
-          }
-          for (; r < M; r += 32) mac_ca(acc, ldc(col + r), vec[r - i]);
-          acc.x = bsum(acc.x);
-          acc.y = bsum(acc.y);
-          if (lane == 0) {
-            if (it < ncol)
-              ax.zb[i + 1 + it] = acc;
-            else if (it < ncol + j)
-              ax.s1[it - ncol] = acc;
-            else
-              ax.s2[it - ncol - j] = acc;
-          }
-        }
-      }
-      cluster.sync();
-      // ---- S3: y_i = tauq (z - Y s1 - U s2); row i of the current matrix ----
-      if (tid < j) {
-        sm[tid] = ldc(&ax.s1[tid]);
-        sm[kPanel + tid] = ldc(&ax.s2[tid]);
-        sm[2 * kPanel + tid] = ldc(&AE(i, p + tid));  // v_k(i)
-        sm[3 * kPanel + tid] = ldc(&XB(i, tid));      // x_k(i)
-      }
-      __syncthreads();
-      {
-        double acc = 0.0;
-        for (int c = i + 1 + gt; c < N; c += gthr) {
-          double2 y = ldc(&ax.zb[c]);
-          double2 rr = ldc(&AE(i, c));
-          for (int k = 0; k < j; ++k) {
-            const double2 yk = ldc(&YB(c, k)), uk = ldc(&PV(c, p + k));
-            msub(y, yk, sm[k]);
-            msub(y, uk, sm[kPanel + k]);
-            msub_cb(rr, sm[2 * kPanel + k], yk);
-            msub_cb(rr, sm[3 * kPanel + k], uk);
-          }
-          y = cmul(tau, y);
-          YB(c, j) = y;
-          rr.x -= y.x;  // v_i(i) = 1: rr -= conj(y)
-          rr.y += y.y;
-          AE(i, c) = rr;
-          if (c >= i + 2) acc = fma(rr.x, rr.x, fma(rr.y, rr.y, acc));
-        }
-        acc = block_sum(acc, red);
-        if (tid == 0) ax.nrmR[crank] = acc;
-      }
-      for (int r = i + 1 + gt; r < M; r += gthr) AE(r, i) = cmul(ldc(&AE(r, i)), sc);  // v_i
-      cluster.sync();
-      // ---- right reflector of row i (every CTA) ----
-      double beta2;
-      double2 tau2, sc2;
-      {
-        double xn2 = 0.0;
-        for (int q = 0; q < C; ++q) xn2 += __ldcg(&ax.nrmR[q]);
-        larfg_scalars(cconj(ldc(&AE(i, i + 1))), xn2, beta2, tau2, sc2);
-      }
-      if (crank == 0 && tid == 0) {
-        ee[i] = beta2;
-        S.taup[i] = tau2;
-      }
-      // ---- S4: w = A0(i+1:M, i+1:N) u by column chunks, t1 = Y^H u, t2 = U^H u ----
-      for (int c = i + 1 + tid; c < N; c += nthr)
-        vec[c - i - 1] = c == i + 1 ? make_double2(1.0, 0.0) : cmul(cconj(ldc(&AE(i, c))), sc2);
-      __syncthreads();
-      {
-        const int rows = M - i - 1, cols = N - i - 1;
-        const int nrb = (rows + 31) / 32, ncc = (cols + kChunk - 1) / kChunk;
-        const int tasks = nrb * ncc, items = tasks + 2 * j + 1;
-        for (int it = gw; it < items; it += nw) {
-          if (it < tasks) {
-            const int rb = it % nrb, cc = it / nrb;
-            const int r = i + 1 + rb * 32 + lane;
-            const int c0 = i + 1 + cc * kChunk, c1 = min(N, c0 + kChunk);
-            if (r < M) {
-              double2 acc = make_double2(0.0, 0.0);
-              const double2 *rp = &AE(r, 0);
-              int c = c0;
-              for (; c + 7 < c1; c += 8) {
-                double2 a[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) a[q] = ldc(rp + (size_t)M * (c + q));
-#pragma unroll
-                for (int q = 0; q < 8; ++q) mac(acc, a[q], vec[c + q - i - 1]);
-              }
-              for (; c < c1; ++c) mac(acc, ldc(rp + (size_t)M * c), vec[c - i - 1]);
-              ax.part[(size_t)cc * M + r] = acc;
-            }
-          } else {
-            const int k = it - tasks;  // 0..j: t1 over y_k; j+1..2j: t2 over u_(k-j-1)
-            const double2 *cp = k <= j ? &YB(0, k) : &PV(0, p + k - j - 1);
-            double2 acc = make_double2(0.0, 0.0);
-            for (int c = i + 1 + lane; c < N; c += 32) mac_ca(acc, ldc(cp + c), vec[c - i - 1]);
-            acc.x = bsum(acc.x);
-            acc.y = bsum(acc.y);
-            if (lane == 0) {
-              if (k <= j)
-                ax.t1[k] = acc;
-              else
-                ax.t2[k - j - 1] = acc;
-            }
-          }
-        }
-        for (int c = i + 1 + gt; c < N; c += gthr) PV(c, i) = vec[c - i - 1];  // u_i
-      }
-      cluster.sync();
-      // ---- x_i = taup (w - V t1 - Xp t2); then column i+1 of the current matrix ----
-      const bool next_in_panel = j + 1 < jb;
-      if (tid <= j) {
-        sm[tid] = ldc(&ax.t1[tid]);
-        if (tid < j) sm[kPanel + tid] = ldc(&ax.t2[tid]);
-        if (next_in_panel) {
-          sm[2 * kPanel + tid] = ldc(&YB(i + 1, tid));      // y_k(i+1)
-          sm[3 * kPanel + tid] = ldc(&PV(i + 1, p + tid));  // u_k(i+1)
-        }
-      }
-      __syncthreads();
-      {
-        const int ncc = (N - i - 1 + kChunk - 1) / kChunk;
-        double acc = 0.0;
-        for (int r = i + 1 + gt; r < M; r += gthr) {
-          double2 w = make_double2(0.0, 0.0);
-          for (int q = 0; q < ncc; ++q) {  // fixed order
-            const double2 t = ldc(&ax.part[(size_t)q * M + r]);
-            w.x += t.x;
-            w.y += t.y;
-          }
-          for (int k = 0; k <= j; ++k) msub(w, ldc(&AE(r, p + k)), sm[k]);
-          for (int k = 0; k < j; ++k) msub(w, ldc(&XB(r, k)), sm[kPanel + k]);
-          const double2 x = cmul(tau2, w);
-          XB(r, j) = x;
-          if (next_in_panel) {
-            double2 a = ldc(&AE(r, i + 1));
-            for (int k = 0; k <= j; ++k) {
-              msub_cb(a, ldc(&AE(r, p + k)), sm[2 * kPanel + k]);
-              msub_cb(a, k < j ? ldc(&XB(r, k)) : x, sm[3 * kPanel + k]);
-            }
-            AE(r, i + 1) = a;
-            if (r >= i + 2) acc = fma(a.x, a.x, fma(a.y, a.y, acc));
-          }
-        }
-        if (next_in_panel) {
-          acc = block_sum(acc, red);
-          if (tid == 0) ax.nrmL[crank] = acc;
-        }
-      }
-      cluster.sync();
-    }
-    const int q = p + jb;
-    if (q >= N) break;
-    // ---- panel end: A0(q:M, q:N) -= V Y^H + Xp U^H (inner dimension 2 jb) ----
-    // 64 x 64 tiles over the cluster's CTAs; each warp owns a 16 x 16 block and
-    // accumulates its real and imaginary parts with four real DMMAs per k-step:
-    //   Re -= Lr Rr^T + Li Ri^T,  Im -= Li Rr^T - Lr Ri^T   (L = [V Xp], R = [Y U])
-    {
-      const int K2 = 2 * jb;
-      const int ntr = (M - q + kTile - 1) / kTile, ntc = (N - q + kTile - 1) / kTile;
-      double *Lr = stg, *Li = stg + kKc * kS, *Rr = stg + 2 * kKc * kS, *Ri = stg + 3 * kKc * kS;
-      const int wr = (warp & 3) * 16, wc = (warp >> 2) * 16;
-      const int fr = lane >> 2, fk = lane & 3;
-      for (int t = crank; t < ntr * ntc; t += C) {
-        const int r0 = q + (t % ntr) * kTile, c0 = q + (t / ntr) * kTile;
-        double cr[2][2][2], ci[2][2][2];
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-#pragma unroll
-          for (int y = 0; y < 2; ++y)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) cr[x][y][e] = ci[x][y][e] = 0.0;
-        for (int kc = 0; kc < K2; kc += kKc) {
-          __syncthreads();
-          for (int e = tid; e < kKc * kTile; e += nthr) {
-            const int rr = e % kTile, kk = e / kTile, k = kc + kk;
-            const int r = r0 + rr, c = c0 + rr;
-            double2 l = make_double2(0.0, 0.0), g = make_double2(0.0, 0.0);
-            if (k < K2) {
-              if (r < M) l = k < jb ? ldc(&AE(r, p + k)) : ldc(&XB(r, k - jb));
-              if (c < N) g = k < jb ? ldc(&YB(c, k)) : ldc(&PV(c, p + k - jb));
-            }
-            Lr[kk * kS + rr] = l.x;
-            Li[kk * kS + rr] = l.y;
-            Rr[kk * kS + rr] = g.x;
-            Ri[kk * kS + rr] = g.y;
-          }
-          __syncthreads();
-#pragma unroll
-          for (int ks = 0; ks < kKc; ks += 4) {
-            const int ko = (ks + fk) * kS;
-            double ar[2], ai[2], br[2], bi[2];
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              ar[b] = Lr[ko + wr + 8 * b + fr];
-              ai[b] = Li[ko + wr + 8 * b + fr];
-              br[b] = Rr[ko + wc + 8 * b + fr];
-              bi[b] = Ri[ko + wc + 8 * b + fr];
-            }
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-#pragma unroll
-              for (int y = 0; y < 2; ++y) {
-                dmma(cr[x][y][0], cr[x][y][1], -ar[x], br[y]);
-                dmma(cr[x][y][0], cr[x][y][1], -ai[x], bi[y]);
-                dmma(ci[x][y][0], ci[x][y][1], -ai[x], br[y]);
-                dmma(ci[x][y][0], ci[x][y][1], ar[x], bi[y]);
-              }
-          }
-        }
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const int r = r0 + wr + 8 * x + fr;
-          if (r >= M) continue;
-#pragma unroll
-          for (int y = 0; y < 2; ++y)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int c = c0 + wc + 8 * y + 2 * fk + e;
-              if (c >= N) continue;
-              double2 v = ldc(&AE(r, c));
-              v.x += cr[x][y][e];
-              v.y += ci[x][y][e];
-              AE(r, c) = v;
-            }
-        }
-      }
-    }
-    cluster.sync();
-    {  // norm partials of column q below the diagonal
-      double acc = 0.0;
-      for (int r = q + 1 + gt; r < M; r += gthr) {
-        const double2 a = ldc(&AE(r, q));
-        acc = fma(a.x, a.x, fma(a.y, a.y, acc));
-      }
-      acc = block_sum(acc, red);
-      if (tid == 0) ax.nrmL[crank] = acc;
-    }
-    cluster.sync();
-  }
-#undef AE
-#undef YB
-#undef XB
-#undef PV
-}
-
 // warp sum of a double-float, as a double (each lane's pair is exact in FP64)
 __device__ __forceinline__ double df_warp_sum(float h, float l) { return bsum((double)h + (double)l); }
-
-__global__ void __launch_bounds__(kBW * 32) k_gebrd_df(Slot *slots, const int *path) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;  // uniform per cluster
-  const Slot S = slots[s];
-  int M, N;
-  bd_dims(*S.cp, route, M, N);
-  float4 *A = reinterpret_cast<float4 *>(S.X);  // (re_hi, re_lo, im_hi, im_lo)
-  double *dd = S.bdws, *ee = S.bdws + N;
-  const BdAux ax = bd_aux(S.aux, M, N);
-  const int C = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int gt = crank * nthr + tid, gthr = C * nthr;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int gw = crank * (nthr >> 5) + warp, nw = C * (nthr >> 5);
-  extern __shared__ double2 sh[];
-  float4 *vec = reinterpret_cast<float4 *>(sh);  // max(M, N): v or u of the current column
-  double2 *sm = sh + max(M, N);         // 4 kPanel small per-column vectors
-  double *stg = reinterpret_cast<double *>(sm + 4 * kPanel);  // trailing-update staging
-  __shared__ double red[32];
-#define AE(r, c) A[(size_t)(r) + (size_t)M * (c)]
-#define YB(c, k) ax.Yb[(size_t)(c) + (size_t)N * (k)]
-#define XB(r, k) ax.Xb[(size_t)(r) + (size_t)M * (k)]
-#define PV(c, k) ax.Pv[(size_t)(c) + (size_t)N * (k)]
-  {  // norm partials of column 0 below the diagonal
-    double acc = 0.0;
-    for (int r = 1 + gt; r < M; r += gthr) {
-      const double2 a = dfl(&AE(r, 0));
-      acc = fma(a.x, a.x, fma(a.y, a.y, acc));
-    }
-    acc = block_sum(acc, red);
-    if (tid == 0) ax.nrmL[crank] = acc;
-  }
-  cluster.sync();
-  for (int p = 0; p < N; p += kPanel) {
-    const int jb = min(kPanel, N - p);
-    for (int j = 0; j < jb; ++j) {
-      const int i = p + j;
-      // ---- left reflector of column i (every CTA, identical inputs) ----
-      double beta;
-      double2 tau, sc;
-      {
-        double xn2 = 0.0;
-        for (int q = 0; q < C; ++q) xn2 += __ldcg(&ax.nrmL[q]);
-        larfg_scalars(dfl(&AE(i, i)), xn2, beta, tau, sc);
-      }
-      if (crank == 0 && tid == 0) {
-        dd[i] = beta;
-        S.tau[i] = tau;
-      }
-      if (i == N - 1) {  // last column: left reflector only
-        for (int r = i + 1 + gt; r < M; r += gthr) AE(r, i) = dfs(cmul(dfl(&AE(r, i)), sc));
-        break;
-      }
-      // ---- S2: z = A0(i:M, i+1:N)^H v, s1 = V^H v, s2 = Xp^H v ----
-      for (int r = i + tid; r < M; r += nthr)
-        vec[r - i] = dfs(r == i ? make_double2(1.0, 0.0) : cmul(dfl(&AE(r, i)), sc));
-      __syncthreads();
-      {
-        const int ncol = N - i - 1, items = ncol + 2 * j;
-        for (int it = gw; it < items; it += nw) {
-          double2 acc = make_double2(0.0, 0.0);  // sum_r conj(col(r)) v(r)
-          if (it < ncol + j) {  // columns of A0 / of V: double-float on the FP32 pipe
-            const float4 *col = &AE(0, it < ncol ? i + 1 + it : p + (it - ncol));
-            float ar = 0.f, arl = 0.f, ai = 0.f, ail = 0.f;
-            int r = i + lane;
-            for (; r + 32 * (kDfLoads - 1) < M; r += 32 * kDfLoads) {
-              float4 c[kDfLoads];
-#pragma unroll
-              for (int q = 0; q < kDfLoads; ++q) c[q] = __ldcg(col + r + 32 * q);
-#pragma unroll
-              for (int q = 0; q < kDfLoads; ++q) df_cmac_ca(ar, arl, ai, ail, c[q], vec[r + 32 * q - i]);
-            }
-            for (; r < M; r += 32) df_cmac_ca(ar, arl, ai, ail, __ldcg(col + r), vec[r - i]);
-            acc = make_double2(df_warp_sum(ar, arl), df_warp_sum(ai, ail));
-          } else {  // x_k columns (FP64)
-            const double2 *col = &XB(0, it - ncol - j);
-            for (int r = i + lane; r < M; r += 32) mac_ca(acc, ldc(col + r), dfd(vec[r - i]));
-            acc.x = bsum(acc.x);
-            acc.y = bsum(acc.y);
-          }
-          if (lane == 0) {
-            if (it < ncol)
-              ax.zb[i + 1 + it] = acc;
-            else if (it < ncol + j)
-              ax.s1[it - ncol] = acc;
-            else
-              ax.s2[it - ncol - j] = acc;
-          }
-        }
-      }
-      cluster.sync();
-      // ---- S3: y_i = tauq (z - Y s1 - U s2); row i of the current matrix ----
-      if (tid < j) {
-        sm[tid] = ldc(&ax.s1[tid]);
-        sm[kPanel + tid] = ldc(&ax.s2[tid]);
-        sm[2 * kPanel + tid] = dfl(&AE(i, p + tid));  // v_k(i)
-        sm[3 * kPanel + tid] = ldc(&XB(i, tid));      // x_k(i)
-      }
-      __syncthreads();
-      {
-        double acc = 0.0;
-        for (int c = i + 1 + gt; c < N; c += gthr) {
-          double2 y = ldc(&ax.zb[c]);
-          double2 rr = dfl(&AE(i, c));
-          for (int k = 0; k < j; ++k) {
-            const double2 yk = ldc(&YB(c, k)), uk = ldc(&PV(c, p + k));
-            msub(y, yk, sm[k]);
-            msub(y, uk, sm[kPanel + k]);
-            msub_cb(rr, sm[2 * kPanel + k], yk);
-            msub_cb(rr, sm[3 * kPanel + k], uk);
-          }
-          y = cmul(tau, y);
-          YB(c, j) = y;
-          rr.x -= y.x;  // v_i(i) = 1: rr -= conj(y)
-          rr.y += y.y;
-          AE(i, c) = dfs(rr);
-          if (c >= i + 2) acc = fma(rr.x, rr.x, fma(rr.y, rr.y, acc));
-        }
-        acc = block_sum(acc, red);
-        if (tid == 0) ax.nrmR[crank] = acc;
-      }
-      for (int r = i + 1 + gt; r < M; r += gthr) AE(r, i) = dfs(cmul(dfl(&AE(r, i)), sc));  // v_i
-      cluster.sync();
-      // ---- right reflector of row i (every CTA) ----
-      double beta2;
-      double2 tau2, sc2;
-      {
-        double xn2 = 0.0;
-        for (int q = 0; q < C; ++q) xn2 += __ldcg(&ax.nrmR[q]);
-        larfg_scalars(cconj(dfl(&AE(i, i + 1))), xn2, beta2, tau2, sc2);
-      }
-      if (crank == 0 && tid == 0) {
-        ee[i] = beta2;
-        S.taup[i] = tau2;
-      }
-      // ---- S4: w = A0(i+1:M, i+1:N) u by column chunks, t1 = Y^H u, t2 = U^H u ----
-      for (int c = i + 1 + tid; c < N; c += nthr)
-        vec[c - i - 1] = dfs(c == i + 1 ? make_double2(1.0, 0.0) : cmul(cconj(dfl(&AE(i, c))), sc2));
-      __syncthreads();
-      {
-        const int rows = M - i - 1, cols = N - i - 1;
-        const int nrb = (rows + 31) / 32, ncc = (cols + kChunk - 1) / kChunk;
-        const int tasks = nrb * ncc, items = tasks + 2 * j + 1;
-        for (int it = gw; it < items; it += nw) {
-          if (it < tasks) {
-            const int rb = it % nrb, cc = it / nrb;
-            const int r = i + 1 + rb * 32 + lane;
-            const int c0 = i + 1 + cc * kChunk, c1 = min(N, c0 + kChunk);
-            if (r < M) {
-              float ar = 0.f, arl = 0.f, ai = 0.f, ail = 0.f;
-              const float4 *rp = &AE(r, 0);
-              int c = c0;
-              for (; c + kDfLoads - 1 < c1; c += kDfLoads) {
-                float4 a[kDfLoads];
-#pragma unroll
-                for (int q = 0; q < kDfLoads; ++q) a[q] = __ldcg(rp + (size_t)M * (c + q));
-#pragma unroll
-                for (int q = 0; q < kDfLoads; ++q) df_cmac(ar, arl, ai, ail, a[q], vec[c + q - i - 1]);
-              }
-              for (; c < c1; ++c) df_cmac(ar, arl, ai, ail, __ldcg(rp + (size_t)M * c), vec[c - i - 1]);
-              ax.part[(size_t)cc * M + r] = make_double2((double)ar + (double)arl, (double)ai + (double)ail);
-            }
-          } else {
-            const int k = it - tasks;  // 0..j: t1 over y_k; j+1..2j: t2 over u_(k-j-1)
-            const double2 *cp = k <= j ? &YB(0, k) : &PV(0, p + k - j - 1);
-            double2 acc = make_double2(0.0, 0.0);
-            for (int c = i + 1 + lane; c < N; c += 32) mac_ca(acc, ldc(cp + c), dfd(vec[c - i - 1]));
-            acc.x = bsum(acc.x);
-            acc.y = bsum(acc.y);
-            if (lane == 0) {
-              if (k <= j)
-                ax.t1[k] = acc;
-              else
-                ax.t2[k - j - 1] = acc;
-            }
-          }
-        }
-        for (int c = i + 1 + gt; c < N; c += gthr) PV(c, i) = dfd(vec[c - i - 1]);  // u_i
-      }
-      cluster.sync();
-      // ---- x_i = taup (w - V t1 - Xp t2); then column i+1 of the current matrix ----
-      const bool next_in_panel = j + 1 < jb;
-      if (tid <= j) {
-        sm[tid] = ldc(&ax.t1[tid]);
-        if (tid < j) sm[kPanel + tid] = ldc(&ax.t2[tid]);
-        if (next_in_panel) {
-          sm[2 * kPanel + tid] = ldc(&YB(i + 1, tid));      // y_k(i+1)
-          sm[3 * kPanel + tid] = ldc(&PV(i + 1, p + tid));  // u_k(i+1)
-        }
-      }
-      __syncthreads();
-      {
-        const int ncc = (N - i - 1 + kChunk - 1) / kChunk;
-        double acc = 0.0;
-        for (int r = i + 1 + gt; r < M; r += gthr) {
-          double2 w = make_double2(0.0, 0.0);
-          for (int q = 0; q < ncc; ++q) {  // fixed order
-            const double2 t = ldc(&ax.part[(size_t)q * M + r]);
-            w.x += t.x;
-            w.y += t.y;
-          }
-          for (int k = 0; k <= j; ++k) msub(w, dfl(&AE(r, p + k)), sm[k]);
-          for (int k = 0; k < j; ++k) msub(w, ldc(&XB(r, k)), sm[kPanel + k]);
-          const double2 x = cmul(tau2, w);
-          XB(r, j) = x;
-          if (next_in_panel) {
-            double2 a = dfl(&AE(r, i + 1));
-            for (int k = 0; k <= j; ++k) {
-              msub_cb(a, dfl(&AE(r, p + k)), sm[2 * kPanel + k]);
-              msub_cb(a, k < j ? ldc(&XB(r, k)) : x, sm[3 * kPanel + k]);
-            }
-            AE(r, i + 1) = dfs(a);
-            if (r >= i + 2) acc = fma(a.x, a.x, fma(a.y, a.y, acc));
-          }
-        }
-        if (next_in_panel) {
-          acc = block_sum(acc, red);
-          if (tid == 0) ax.nrmL[crank] = acc;
-        }
-      }
-      cluster.sync();
-    }
-    const int q = p + jb;
-    if (q >= N) break;
-    // ---- panel end: A0(q:M, q:N) -= V Y^H + Xp U^H (inner dimension 2 jb) ----
-    // 64 x 64 tiles over the cluster's CTAs, double-float on the FP32 pipe: each
-    // thread starts from its 8 elements of A0 and subtracts the 2 jb products
-    {
-      const int K2 = 2 * jb;
-      const int ntr = (M - q + kTile - 1) / kTile, ntc = (N - q + kTile - 1) / kTile;
-      float4 *Ls = reinterpret_cast<float4 *>(stg), *Rs = Ls + kKc * kTile;
-      const int tx = tid & 15, ty = tid >> 4;  // rows ty, ty + 32; columns tx + 16 b
-      for (int t = crank; t < ntr * ntc; t += C) {
-        const int r0 = q + (t % ntr) * kTile, c0 = q + (t / ntr) * kTile;
-        float4 acc[2][4];
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int r = r0 + ty + 32 * a, c = c0 + tx + 16 * b;
-            acc[a][b] = (r < M && c < N) ? __ldcg(&AE(r, c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-        for (int kc = 0; kc < K2; kc += kKc) {
-          __syncthreads();
-          for (int e = tid; e < kKc * kTile; e += nthr) {
-            const int rr = e % kTile, kk = e / kTile, k = kc + kk;
-            const int r = r0 + rr, c = c0 + rr;
-            float4 l = make_float4(0.f, 0.f, 0.f, 0.f), g = l;
-            if (k < K2) {
-              if (r < M) l = k < jb ? __ldcg(&AE(r, p + k)) : dfs(ldc(&XB(r, k - jb)));
-              if (c < N) g = dfs(k < jb ? ldc(&YB(c, k)) : ldc(&PV(c, p + k - jb)));
-            }
-            Ls[kk * kTile + rr] = l;
-            Rs[kk * kTile + rr] = g;
-          }
-          __syncthreads();
-          for (int kk = 0; kk < kKc; ++kk) {
-            const float4 l0 = Ls[kk * kTile + ty], l1 = Ls[kk * kTile + ty + 32];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-              const float4 g = Rs[kk * kTile + tx + 16 * b];
-              df_cmsub_cb(acc[0][b], l0, g);  // acc -= l conj(g)
-              df_cmsub_cb(acc[1][b], l1, g);
-            }
-          }
-        }
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int r = r0 + ty + 32 * a, c = c0 + tx + 16 * b;
-            if (r < M && c < N) AE(r, c) = df_norm4(acc[a][b]);
-          }
-      }
-    }
-    cluster.sync();
-    {  // norm partials of column q below the diagonal
-      double acc = 0.0;
-      for (int r = q + 1 + gt; r < M; r += gthr) {
-        const double2 a = dfl(&AE(r, q));
-        acc = fma(a.x, a.x, fma(a.y, a.y, acc));
-      }
-      acc = block_sum(acc, red);
-      if (tid == 0) ax.nrmL[crank] = acc;
-    }
-    cluster.sync();
-  }
-#undef AE
-#undef YB
-#undef XB
-#undef PV
-}
 
 // ---------------------------------------------------------------------------
 // 2. bisection: sigma_i of B for i < kk (one team of kTeam lanes each), Golub-Kahan Sturm counts
@@ -1640,7 +909,7 @@ __global__ void k_bd_transpose(Slot *slots, const int *path) {
 // ---------------------------------------------------------------------------
 // host orchestration: bidiagonal route for the slots flagged kPathBidiag / kPathBidiagT
 // ---------------------------------------------------------------------------
-size_t bidiag_aux_elems(int n) { return bd_aux_elems(n, n); }
+size_t bidiag_aux_elems(int n) { return gebrd_aux_elems(n, n); }
 
 size_t bidiag_ws_doubles(int n, int chi) {
   const int K = std::min(chi, n);
@@ -1664,82 +933,16 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
     k_bd_transpose<<<dim3(g, g, nb), 256, 0, st>>>(slots_d, path_d);
     TEBD_LAUNCHED(h);
   }
-  {
-    cudaLaunchConfig_t cfg = {};
-    const size_t smem = sizeof(double2) * ((size_t)nmax + 4 * kPanel) + sizeof(double) * kStageDoubles;
-    const bool dfp = b.dfp;
-    auto kern = dfp ? k_gebrd_df : k_gebrd;
-    if ((rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                         "bidiagonalisation shared memory")))
-      return rc;
-    cfg.blockDim = dim3(kBW * 32, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    // Cluster size: the kernel is bound by the SMs' FP64 pipes, so the batch's time
-    // goes as waves / C; clusters must fit in one GPC, so the co-resident count
-    // (occupancy query) decides how many waves a size needs.  Ties keep the
-    // smaller size (fewer barriers' worth of idle SMs in a partial wave).
-    // sizes up to 8, at least 4 (the autotuner measured 4 CTAs fastest for
-    // 64..320-column batches of 32 bonds, where ceil(n / 128) had allowed 1..3)
-    const int cmax = std::min(8, std::max(4, (nmax + 127) / 128));
-    int nbd = 0;  // bonds on this route (the others' clusters exit at once)
-    for (int s = 0; s < nb; ++s) nbd += b.path_h[s] != kPathQRJ;
-    const TuneParams tp = tune_lookup(h, dfp ? 1 : 0, nmax, nbd);
-    int C = 1;
-    bool tuned_ok = false;
-    double best = 1e300;
-    for (int c = 1; c <= cmax; ++c) {
-      cfg.gridDim = dim3(c, nb, 1);
-      attr[0].val.clusterDim.x = c;
-      int ncl = 0;
-      if (cudaOccupancyMaxActiveClusters(&ncl, (const void *)kern, &cfg) != cudaSuccess || ncl < 1) {
-        cudaGetLastError();
-        continue;
-      }
-      tuned_ok |= c == tp.cluster;
-      const double cost = (double)((nbd + ncl - 1) / ncl) / c;
-      if (cost < best * (1.0 - 1e-9)) {
-        best = cost;
-        C = c;
-      }
-    }
-    if (tp.cluster > cmax && tp.cluster <= 8) {  // beyond the default's range: every CTA
-      cfg.gridDim = dim3(tp.cluster, nb, 1);      // still gets its share of the rows (or none)
-      attr[0].val.clusterDim.x = tp.cluster;
-      int ncl = 0;
-      tuned_ok = cudaOccupancyMaxActiveClusters(&ncl, (const void *)kern, &cfg) == cudaSuccess && ncl >= 1;
-      if (!tuned_ok) cudaGetLastError();
-    }
-    if (tp.cluster > 0) {  // the autotuner's size, when the launch can use it
-      if (tuned_ok)
-        C = tp.cluster;
-      else
-        tune_reject(h);
-    }
-    cfg.gridDim = dim3(C, nb, 1);
-    attr[0].val.clusterDim.x = C;
-    if (dfp) {
-      k_bd_to_df<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
-      TEBD_LAUNCHED(h);
-    }
-    if (h->profiling) cudaEventRecord(h->ev[4], st);
-    rc = check_cuda(h, cudaLaunchKernelEx(&cfg, kern, slots_d, path_d),
-                    "bidiagonalisation launch");
-    if (rc) return rc;
-    if (h->profiling) cudaEventRecord(h->ev[5], st);
-    if (dfp) {  // the reflectors stay double-float for k_bd_apply_df; Pv follows
-      k_bd_pv_to_df<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
-      TEBD_LAUNCHED(h);
-    }
+  if (h->profiling) cudaEventRecord(h->ev[4], st);
+  if ((rc = launch_gebrd(h, b))) return rc;
+  if (h->profiling) cudaEventRecord(h->ev[5], st);
+  if (b.dfp) {  // the reflectors as double-float for k_bd_apply_df
+    k_bd_to_df<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
     TEBD_LAUNCHED(h);
-    ++h->stats.gebrd_launches;
+    k_bd_pv_to_df<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
+    TEBD_LAUNCHED(h);
   }
+  ++h->stats.gebrd_launches;
   {
     const size_t smem = (sizeof(double) + sizeof(float2) + sizeof(float)) * (size_t)(2 * nmax);
     // team size: multisection while the batch's values (nb x kk at most) leave the
@@ -1849,7 +1052,7 @@ int run_bidiag(tebd_handle *h, int nb, int nmax) {
 // (kk = the batch's largest N): aux, tau, taup (complex) and bdws (doubles).
 void bidiag_block_ws(int M, int N, int kk, size_t *aux_elems, size_t *bdws_doubles) {
   const int K = std::min(kk, N);
-  *aux_elems = bd_aux_elems(M, N);
+  *aux_elems = gebrd_aux_elems(M, N);
   *bdws_doubles = bd_scratch(N, kk) + 6 * (size_t)(2 * N) * K + 2 * (size_t)M * K + 4;
 }
 

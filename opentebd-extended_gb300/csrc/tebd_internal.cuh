@@ -250,6 +250,9 @@ struct BidiagBatch {
   int right_only = 0;  // 1: right singular vectors only (double-float form; S.X keeps no left vectors)
 };
 int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b);
+// the bidiagonalisation of the batch's slots (gebrd.cu) and its workspace in S.aux (complex elements)
+int launch_gebrd(tebd_handle *h, const BidiagBatch &b);
+size_t gebrd_aux_elems(int M, int N);
 // Autotuner table (tune.cu): the shape for route (0 FP64 bidiagonal, 1
 // double-float bidiagonal, 2 randomized-route Cholesky leaf, 3 its blocking),
 // largest dimension n and bonds nb; zeros where no entry exists.  tune_reject: the launch could not
