@@ -527,7 +527,7 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
   if (h->profiling) cudaEventRecord(h->ev[2], h->stream);
   int rc;
   if (h->mode == TEBD_MODE_DENSE) {
-    if ((rc = launch_dense_prepare(h, nb, false))) return rc;
+    if ((rc = launch_dense_prepare(h, nb, true))) return rc;
     int nmax = 0;
     std::vector<Compact> cps;
     if ((rc = dense_compact_sizes(h, nb, &nmax, &cps))) return rc;

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(96) k_compact(const double *__restrict__ lam, 
     c.m = d * cnt[0];
     c.n = d * cnt[2];
     c.k = c.n;
+    c.bad = 0;
     const double *l1 = lam + (size_t)link * chi;
     double lo = 0.0, hi = 0.0;
     for (int a = 0; a < chi; ++a)
@@ -550,14 +551,15 @@ __global__ void __launch_bounds__(256) k_restore_gamma2(double2 *gam, const doub
 // ---------------------------------------------------------------------------
 static inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
-int launch_dense_prepare(tebd_handle *h, int nb, bool /*real_gate: converted on the host*/) {
+int launch_dense_prepare(tebd_handle *h, int nb, bool gate) {
   const int chi = h->chi, d = h->d, n = h->n;
   cudaStream_t st = h->stream;
   JacobiProblem<double> *jp = reinterpret_cast<JacobiProblem<double> *>(h->jprob_d);
+  h->cps.clear();
   k_compact<<<nb, 96, 0, st>>>(h->lam, h->links_d, h->slots_d, jp, chi, d);
   TEBD_LAUNCHED(h);
   int tc = -1;  // tensor-core Theta (theta_tc.cu); -1: formed on the CUDA cores below
-  if (h->theta_form != 0 && h->mode == TEBD_MODE_DENSE && (tc = launch_theta_tc(h, nb)) > 0) return tc;
+  if (h->mode == TEBD_MODE_DENSE && (tc = launch_theta_tc(h, nb)) > 0) return tc;
   if (tc == 0) {
   } else if (h->opts.svd_mode == TEBD_SVD_DF || h->opts.svd_mode == TEBD_SVD_RSVD)
     k_theta_form_df<<<dim3(cdiv(n, TT_M), cdiv(n, TT_N), nb), 256, 0, st>>>(h->gam, h->lam, h->links_d,
@@ -567,11 +569,13 @@ int launch_dense_prepare(tebd_handle *h, int nb, bool /*real_gate: converted on 
                                                                          h->slots_d, chi, d);
   TEBD_LAUNCHED(h);
   const bool gdf = h->opts.svd_mode == TEBD_SVD_DF || h->opts.svd_mode == TEBD_SVD_RSVD;
-  int rc = check_cuda(h, set_gate_smem(d, gdf), "gate shared memory");
+  int rc = gate ? check_cuda(h, set_gate_smem(d, gdf), "gate shared memory") : TEBD_OK;
   if (rc) return rc;
-  (gdf ? k_gate_apply<true> : k_gate_apply<false>)<<<dim3(cdiv((size_t)chi * chi, kGatePairs), nb), 128,
-                                                     gate_smem_bytes(d), st>>>(h->slots_d, chi, d);
-  TEBD_LAUNCHED(h);
+  if (gate) {
+    (gdf ? k_gate_apply<true> : k_gate_apply<false>)<<<dim3(cdiv((size_t)chi * chi, kGatePairs), nb), 128,
+                                                       gate_smem_bytes(d), st>>>(h->slots_d, chi, d);
+    TEBD_LAUNCHED(h);
+  }
   k_norm_partial<<<dim3(kNormParts, nb), 256, 0, st>>>(h->slots_d, h->nrm_part);
   TEBD_LAUNCHED(h);
   k_norm_final<<<cdiv(nb, 128), 128, 0, st>>>(h->nrm_part, h->nrm, jp, nb, h->status_d);
@@ -627,15 +631,22 @@ int launch_dense_finish(tebd_handle *h, int nb) {
 
 namespace tebd {
 
-// Largest compacted column count of the batch (sizes the Jacobi rounds).
-int dense_compact_sizes(tebd_handle *h, int nb, int *nmax, std::vector<Compact> *out) {
+int read_compaction(tebd_handle *h, int nb) {
+  if (!h->cps.empty()) return TEBD_OK;
   std::vector<Compact> cp(nb);
-  int rc = check_cuda(h, cudaMemcpyAsync(cp.data(), h->cp_d, sizeof(Compact) * nb,
-                                         cudaMemcpyDeviceToHost, h->stream),
+  int rc = check_cuda(h, cudaMemcpyAsync(cp.data(), h->cp_d, sizeof(Compact) * nb, cudaMemcpyDeviceToHost, h->stream),
                       "read compaction");
   if (rc) return rc;
-  rc = check_cuda(h, cudaStreamSynchronize(h->stream), "read compaction");
+  if ((rc = check_cuda(h, cudaStreamSynchronize(h->stream), "read compaction"))) return rc;
+  h->cps.swap(cp);
+  return TEBD_OK;
+}
+
+// Largest compacted column count of the batch (sizes the Jacobi rounds).
+int dense_compact_sizes(tebd_handle *h, int nb, int *nmax, std::vector<Compact> *out) {
+  int rc = read_compaction(h, nb);
   if (rc) return rc;
+  const std::vector<Compact> &cp = h->cps;
   int mx = 0;
   for (int s = 0; s < nb; ++s) {
     if (cp[s].n > mx) mx = cp[s].n;

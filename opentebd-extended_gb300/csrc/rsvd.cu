@@ -465,7 +465,7 @@ void rsvd_free(tebd_handle *h) {
 
 // 7 digit planes of an n x n operand for every slot
 static size_t rs_digit_bytes(int n, int ns) {
-  return sizeof(unsigned short) * kOzMaxS * (size_t)ns * tc_pad(n, kTcBM) * tc_pad(2 * n, kOzBK);
+  return sizeof(unsigned short) * kOzCallS * (size_t)ns * tc_pad(n, kTcBM) * tc_pad(2 * n, kOzBK);
 }
 
 static int rsvd_alloc(tebd_handle *h, int sc) {
@@ -589,7 +589,7 @@ int run_rsvd(tebd_handle *h, int nb, const std::vector<Compact> &cps, std::vecto
   const RsCarve &c = R->carve;
   const long long pstr = (long long)(per / sizeof(double2));
   const int dstride = (int)(sizeof(RsDims) / sizeof(int));
-  const int sk = h->rs_slices, fin = kOzMaxS;
+  const int sk = h->rs_slices, fin = kOzCallS;
   // out (rows x cols, ld rows, workspace offset oo) = op(A) op(B); A and B are
   // workspace offsets unless a base pointer is given
   auto prod = [&](size_t ao, int lda, int at, const double2 *abase, long long astr, size_t bo, int ldb,
@@ -880,7 +880,7 @@ using namespace tebd;
 extern "C" int tebd_set_rsvd(tebd_handle *h, int oversample, int power_iters, double tol, int slices) {
   if (!h) return TEBD_ERR_ARG;
   if (oversample < 0 || power_iters < 0 || power_iters > 4 || !(tol > 0.0 && tol < 1.0) || slices < 3 ||
-      slices > kOzMaxS)
+      slices > kOzCallS)
     return set_error(h, TEBD_ERR_ARG, "rsvd: oversample >= 0, 0 <= power_iters <= 4, 0 < tol < 1, 3 <= slices <= 7");
   h->rs_oversample = oversample;
   h->rs_power = power_iters;

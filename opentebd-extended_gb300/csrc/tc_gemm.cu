@@ -483,7 +483,7 @@ extern "C" int tebd_zgemm_tc(int nprob, int m, int n, int k, const double *A, lo
                              const double *B, long long stride_b, int ldb, double *C, long long stride_c,
                              int ldc, int form, void *stream) {
   if (nprob < 1 || m < 1 || n < 1 || k < 1 || !A || !B || !C || lda < m || ldb < k || ldc < m ||
-      (form != kTc1xTF32 && form != kTc3xTF32 && !zprod_oz(form)))
+      (form != kTc1xTF32 && form != kTc3xTF32 && !(zprod_oz(form) && form <= 100 + kOzCallS)))
     return TEBD_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ZProd z = {};

@@ -90,7 +90,8 @@ inline int tc_planes(int form) { return form == kTc3xTF32 ? 2 : 1; }
 // ---------------------------------------------------------------------------
 constexpr int kOzBN = 128;     // real output columns per CTA
 constexpr int kOzBK = 32;      // bf16 per 64-byte row (K block)
-constexpr int kOzMaxS = 7;
+constexpr int kOzMaxS = 8;     // planes of the kernels; 8 serve Theta's default form (56 bits below the row maxima)
+constexpr int kOzCallS = 7;    // planes that the entry points let a caller ask for, and the randomized route's most
 
 struct OzBatch {
   const unsigned short *a_dig;  // bf16 digits [S][nprob][m_pad][k_pad]
@@ -154,6 +155,8 @@ struct ZProd {
   // optional events recorded around the product kernel alone (profiling)
   cudaEvent_t ev0, ev1;
 };
+// (8 planes: the sums of group 7, up to 2^24.4 in the worst case, may round in their
+// last bit, 2^-63 of the row maxima)
 inline bool zprod_oz(int form) { return form > 100 && form <= 100 + kOzMaxS; }
 size_t zprod_ws_bytes(const ZProd &z);
 // tensor-core multiply-adds the product kernel issues, as flops (2 per

@@ -475,7 +475,8 @@ cudaError_t oz_gemm_launch(const OzBatch &b, int *err_d, cudaStream_t st) {
     case 4: return go(k_tc_oz<4>);
     case 5: return go(k_tc_oz<5>);
     case 6: return go(k_tc_oz<6>);
-    default: return go(k_tc_oz<7>);
+    case 7: return go(k_tc_oz<7>);
+    default: return go(k_tc_oz<8>);
   }
 }
 

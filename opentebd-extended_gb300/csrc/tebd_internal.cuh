@@ -93,6 +93,7 @@ struct Compact {
   int m, n;        // d*r0 rows, d*r2 columns
   int k;           // singular triplets computed (numerical rank for the QR path, else n)
   float span;      // smallest / largest nonzero Lambda1 (the bond's own Schmidt values)
+  int bad;         // a NaN or Inf among the factors of a Theta formed from digits
 };
 
 struct Slot {
@@ -158,6 +159,7 @@ struct tebd_handle {
   tebd::Compact *cp_d;            // nslots compaction records
   int *path_d;                    // nslots SVD route per slot (kPathQRJ / kPathBidiag)
   std::vector<int> path_h;        // host copy of the current batch's routes
+  std::vector<tebd::Compact> cps; // host copy of the current batch's compaction records (empty: not read yet)
   int *idx_d;                     // nslots * 5 * chi index maps
   double *nrm_part;       // nslots * kNormParts partial sums of |Theta|^2
   double *nrm;            // nslots Frobenius norms
@@ -226,8 +228,9 @@ void set_noh_error(const std::string &msg);  // for tebd_last_error(NULL)
 int check_cuda(tebd_handle *h, cudaError_t e, const char *what);
 
 // kernels launched from capi.cu (defined in the .cu files)
-int launch_dense_prepare(tebd_handle *h, int nb, bool real_gate);
+int launch_dense_prepare(tebd_handle *h, int nb, bool gate);  // Theta of the batch's bonds, with their gates or as it is
 int run_jacobi(tebd_handle *h, int nb, int svd_mode, int nmax);
+int read_compaction(tebd_handle *h, int nb);  // fills h->cps once per batch (synchronises)
 int dense_compact_sizes(tebd_handle *h, int nb, int *nmax, std::vector<Compact> *out);
 int launch_dense_finish(tebd_handle *h, int nb);
 int launch_eye(tebd_handle *h, int nb);

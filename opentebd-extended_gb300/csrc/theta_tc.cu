@@ -17,6 +17,8 @@
 
 namespace tebd {
 
+constexpr double kThetaTcMin = 1 << 21;  // m n r1 from which Theta is formed on the tensor cores
+
 int tc_reserve(tebd_handle *h, size_t bytes) {
   if (!h->tc_err) {
     int rc = check_cuda(h, cudaMalloc(&h->tc_err, sizeof(int)), "alloc tensor-core flag");
@@ -96,10 +98,47 @@ int tc_check(tebd_handle *h) {
 
 namespace {
 
+// Power-of-two balance of the inner index for the default form: with a_g the largest
+// |A(:, g)| and b_g the largest |B(g, :)|, A's column g is multiplied by 2^s and B's row by
+// 2^-s so that both come near sqrt(a_g b_g).  The digits are cut off relative to the
+// largest entry of a row of A and of a column of B; unbalanced, an inner index with
+// small Lambda1 (Gamma1 ~ 1 / Lambda1 in a chain that is not left-canonical) costs every
+// other one of them its low digits (energies of such a chain, span 6e-6: 7e-14 off
+// instead of 2e-16; FP64 sums: 1.5e-15).  One warp per (bond, g); s goes to the slot's vn.
+__global__ void __launch_bounds__(256) k_theta_balance(const double2 *__restrict__ gam, const double *__restrict__ lam,
+                                                       const int *__restrict__ links, const Slot *slots, int chi,
+                                                       int d) {
+  const int s = blockIdx.y;
+  const Compact cp = *slots[s].cp;
+  const int gk = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (gk >= cp.r1) return;
+  const int link = links[s], g = slots[s].idx1[gk];
+  const size_t csz = (size_t)chi * d * chi;
+  const double2 *G1 = gam + (size_t)(link - 1) * csz, *G2 = gam + (size_t)link * csz;
+  const double *l0 = lam + (size_t)(link - 1) * chi, *l2 = lam + (size_t)(link + 1) * chi;
+  const double l1 = lam[(size_t)link * chi + g];
+  int ea = 0, eb = 0;  // largest exponent fields
+  auto field = [](double x) { return (__double2hiint(x) >> 20) & 0x7ff; };
+  for (int e = lane; e < d * cp.r0; e += 32) {
+    const int i = e / cp.r0, a = slots[s].idx0[e - i * cp.r0];
+    const double2 v = G1[a + (size_t)chi * i + (size_t)chi * d * g];
+    ea = max(ea, max(field(v.x * l0[a]), field(v.y * l0[a])));
+  }
+  for (int e = lane; e < d * cp.r2; e += 32) {
+    const int j = e / cp.r2, b = slots[s].idx2[e - j * cp.r2];
+    const double2 v = G2[g + (size_t)chi * j + (size_t)chi * d * b];
+    const double w = l1 * l2[b];
+    eb = max(eb, max(field(v.x * w), field(v.y * w)));
+  }
+  ea = __reduce_max_sync(0xffffffffu, ea);
+  eb = __reduce_max_sync(0xffffffffu, eb);
+  if (lane == 0) reinterpret_cast<int *>(slots[s].vn)[gk] = ea && eb ? max(-500, min(500, (eb - ea) / 2)) : 0;
+}
+
 __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restrict__ gam,
                                                         const double *__restrict__ lam,
                                                         const int *__restrict__ links, const Slot *slots, int chi,
-                                                        int d, int m_max, int r1_max, int n_max) {
+                                                        int d, int m_max, int r1_max, int n_max, int *status) {
   const int s = blockIdx.y;
   const Compact cp = *slots[s].cp;
   const int link = links[s];
@@ -111,7 +150,13 @@ __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restric
   const double *l2 = lam + (size_t)(link + 1) * chi;
   const int *idx0 = slots[s].idx0, *idx1 = slots[s].idx1, *idx2 = slots[s].idx2;
   double2 *A = slots[s].aux;
+  auto mark = [&](int q) {
+    atomicOr(status, 1);
+    atomicOr(&slots[q].cp->bad, 1);
+  };
   double2 *B = A + (size_t)m_max * r1_max;
+  const int *bal = reinterpret_cast<const int *>(slots[s].vn);  // with `status`: the default form
+  auto pow2 = [](int k) { return __longlong_as_double((long long)(k + 1023) << 52); };
   const size_t na = (size_t)m_max * r1_max, total = na + (size_t)r1_max * n_max;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
     double2 v = make_double2(0.0, 0.0);
@@ -120,6 +165,8 @@ __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restric
       if (r < cp.m && gk < cp.r1) {
         const int i = r / cp.r0, a = idx0[r - i * cp.r0], g = idx1[gk];
         v = cscale(G1[a + (size_t)chi * i + (size_t)chi * d * g], l0[a]);
+        if (status) v = cscale(v, pow2(bal[gk]));
+        if (status && !(isfinite(v.x) && isfinite(v.y))) mark(s);  // the digits of NaN and Inf are zeros
       }
       A[e] = v;
     } else {
@@ -128,6 +175,8 @@ __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restric
       if (gk < cp.r1 && c < cp.n) {
         const int j = c / cp.r2, b = idx2[c - j * cp.r2], g = idx1[gk];
         v = cscale(G2[g + (size_t)chi * j + (size_t)chi * d * b], l1[g] * l2[b]);
+        if (status) v = cscale(v, pow2(-bal[gk]));
+        if (status && !(isfinite(v.x) && isfinite(v.y))) mark(s);
       }
       B[f] = v;
     }
@@ -138,13 +187,18 @@ __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restric
 
 // Theta of the batch on the tensor cores; returns -1 (nothing launched) when a
 // dimension of the batch is zero, so that the caller forms it on the CUDA cores.
+// The default form (0) takes this path for large products: 8 planes hold 56 bits below
+// each row's and column's largest magnitude, so that the error of a sum of r1 products,
+// about 2^-56 sqrt(r1) of the largest, is below FP64's own (640 x 128 x 640: 3e-17
+// against 1e-16 of the row and column maxima).  The CUDA cores' kernel is bound by the
+// FP64 pipe: 32 bonds of 640 x 640 (chi = 128) took 11.5 ms, 1.1 ms now, packs included.
 int launch_theta_tc(tebd_handle *h, int nb) {
-  std::vector<Compact> cp(nb);
-  int rc = check_cuda(h, cudaMemcpyAsync(cp.data(), h->cp_d, sizeof(Compact) * nb, cudaMemcpyDeviceToHost,
-                                         h->stream),
-                      "read compaction");
-  if (rc) return rc;
-  if ((rc = check_cuda(h, cudaStreamSynchronize(h->stream), "read compaction"))) return rc;
+  int rc;
+  const int form = h->theta_form ? h->theta_form : 100 + kOzMaxS;
+  // the largest product that the batch can have: do not read the records for less
+  if (!h->theta_form && (double)h->n * h->n * h->chi < kThetaTcMin) return -1;
+  if ((rc = read_compaction(h, nb))) return rc;
+  const std::vector<Compact> &cp = h->cps;
   int m_max = 0, n_max = 0, r1_max = 0;
   for (const Compact &c : cp) {
     m_max = std::max(m_max, c.m);
@@ -153,13 +207,19 @@ int launch_theta_tc(tebd_handle *h, int nb) {
   }
   // small products (early, low-rank updates) stay on the CUDA cores: packing and
   // the extra synchronisation cost more than the tiled FP64 kernel there
-  if (m_max == 0 || n_max == 0 || r1_max == 0 || (double)m_max * n_max * r1_max < (double)(1 << 21)) return -1;
+  if (m_max == 0 || n_max == 0 || r1_max == 0 || (double)m_max * n_max * r1_max < kThetaTcMin) return -1;
   const Slot &s0 = h->slots[0];
   const long long aux_stride = nb > 1 ? (long long)(h->slots[1].aux - s0.aux) : 0;
   const size_t total = (size_t)m_max * r1_max + (size_t)r1_max * n_max;
   unsigned gx = (unsigned)std::min<size_t>((total + 255) / 256, 2048);
+  if (!h->theta_form) {
+    k_theta_balance<<<dim3((r1_max + 7) / 8, nb), 256, 0, h->stream>>>(h->gam, h->lam, h->links_d, h->slots_d, h->chi,
+                                                                      h->d);
+    TEBD_LAUNCHED(h);
+  }
   k_theta_operands<<<dim3(gx, nb), 256, 0, h->stream>>>(h->gam, h->lam, h->links_d, h->slots_d, h->chi, h->d,
-                                                         m_max, r1_max, n_max);
+                                                         m_max, r1_max, n_max,
+                                                         h->theta_form ? nullptr : h->status_d);
   TEBD_LAUNCHED(h);
   ZProd z = {};
   z.a = s0.aux;
@@ -172,7 +232,7 @@ int launch_theta_tc(tebd_handle *h, int nb) {
   z.m = m_max;
   z.n = n_max;
   z.k = r1_max;
-  z.form = h->theta_form;
+  z.form = form;
   z.rs = 1;
   z.cs = 0;  // column stride = the bond's own m
   z.m_d = &h->cp_d[0].m;
@@ -194,7 +254,7 @@ using namespace tebd;
 
 extern "C" int tebd_set_theta_form(tebd_handle *h, int form) {
   if (!h) return TEBD_ERR_ARG;
-  if (!(form == 0 || form == kTc3xTF32 || (form >= 103 && form <= 100 + kOzMaxS)))
+  if (!(form == 0 || form == kTc3xTF32 || (form >= 103 && form <= 100 + kOzCallS)))
     return set_error(h, TEBD_ERR_ARG, "theta form must be 0, 3 (3xTF32) or 103..107 (bf16 digit planes)");
   if (h->mode != TEBD_MODE_DENSE && form != 0 && !zprod_oz(form))
     return set_error(h, TEBD_ERR_STATE, "NC handles take theta form 0 or 103..107 (3xTF32 is for dense handles)");
