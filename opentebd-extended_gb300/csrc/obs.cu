@@ -10,8 +10,8 @@
 //   tebd_chain_entropy     ChainEntropy for every link                       :1583-1602
 // Sums run in a fixed order (deterministic), not in the reference's loop order,
 // so results agree with it to rounding.  Two-site density matrices reuse the
-// update's batched Theta formation (k_compact + k_theta_form with an identity
-// gate) on the handle's SVD slots, so observables and updates of one handle are
+// update's batched Theta formation (k_compact + k_theta_form, no gate)
+// on the handle's SVD slots, so observables and updates of one handle are
 // serialised on its stream.
 #include <math.h>
 #include <string.h>
@@ -36,76 +36,145 @@ __device__ __forceinline__ void cacc(double2 &acc, double2 x, double2 y, double 
   acc.y = fma(w, im, acc.y);
 }
 
-// rho_s(i,j) = sum_{a,b} l0(a)^2 l1(b)^2 G(a,i,b) conj(G(a,j,b)); one CTA per site,
-// d^2 entries x (blockDim / d^2) chunks of (a,b), chunk sums added in chunk order.
-__global__ void __launch_bounds__(kObsThreads) k_obs_rho1(const double2 *gam, const double *lam,
-                                                          double2 *rho, int chi, int d) {
-  __shared__ double2 part[kObsThreads];
-  const int s = blockIdx.x;
-  const double2 *G = gam + (size_t)s * chi * d * chi;
+// rho_s(i,j) = sum_{a,b} l0(a)^2 l1(b)^2 G(a,i,b) conj(G(a,j,b)), i <= j (the rest is its
+// conjugate).  A CTA takes a part of the columns b of one site, its threads the rows a
+// (neighbouring in memory), every G entry read once; the CTA's sums go to part[site][CTA],
+// added in that order by k_obs_rho1_sum.  One CTA per site with the d^2 entries split
+// over its threads was bound by the latency of its reads (chi = 512: 24 ms for 16 sites;
+// now 0.86 ms; chi = 128, 64 sites: 1.56 -> 0.34 ms).
+template <int kD>
+__global__ void __launch_bounds__(kObsThreads) k_obs_rho1(const double2 *gam, const double *lam, double2 *part,
+                                                          int chi, int cols) {
+  constexpr int kPairs = kD * (kD + 1) / 2;
+  const int s = blockIdx.y, b0 = blockIdx.x * cols, b1 = min(chi, b0 + cols);
+  const double2 *G = gam + (size_t)s * chi * kD * chi;
   const double *l0 = lam + (size_t)s * chi, *l1 = lam + (size_t)(s + 1) * chi;
-  const int d2 = d * d, nch = kObsThreads / d2;
-  const int t = threadIdx.x, ij = t % d2, ch = t / d2;
-  double2 acc = make_double2(0.0, 0.0);
-  if (ch < nch) {
-    const int i = ij % d, j = ij / d;  // column-major position i + d j
-    for (size_t e = ch; e < (size_t)chi * chi; e += nch) {
-      const int a = (int)(e % chi), b = (int)(e / chi);
-      const double w = l0[a] * l0[a] * l1[b] * l1[b];
-      if (w == 0.0) continue;
-      cacc(acc, G[a + (size_t)chi * (i + (size_t)d * b)], G[a + (size_t)chi * (j + (size_t)d * b)], w);
-    }
+  double2 acc[kPairs];
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) acc[q] = make_double2(0.0, 0.0);
+  for (size_t e = threadIdx.x; e < (size_t)chi * (b1 - b0); e += kObsThreads) {
+    const int a = (int)(e % chi), b = b0 + (int)(e / chi);
+    const double w = l0[a] * l0[a] * l1[b] * l1[b];
+    if (w == 0.0) continue;
+    double2 g[kD];
+#pragma unroll
+    for (int i = 0; i < kD; ++i) g[i] = G[a + (size_t)chi * (i + (size_t)kD * b)];
+    int q = 0;
+#pragma unroll
+    for (int i = 0; i < kD; ++i)
+#pragma unroll
+      for (int j = i; j < kD; ++j) cacc(acc[q++], g[i], g[j], w);
   }
-  part[t] = acc;
+  __shared__ double2 red[kObsThreads / 32][kPairs];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) {
+    double2 v = acc[q];
+    for (int o = 16; o > 0; o >>= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+    if (lane == 0) red[warp][q] = v;
+  }
   __syncthreads();
-  if (t < d2) {
-    double2 r = make_double2(0.0, 0.0);
-    for (int c = 0; c < nch; ++c) {
-      r.x += part[t + c * d2].x;
-      r.y += part[t + c * d2].y;
+  if (threadIdx.x < kPairs) {
+    double2 v = make_double2(0.0, 0.0);
+    for (int w = 0; w < kObsThreads / 32; ++w) {
+      v.x += red[w][threadIdx.x].x;
+      v.y += red[w][threadIdx.x].y;
     }
-    rho[(size_t)s * d2 + t] = r;
+    part[((size_t)s * gridDim.x + blockIdx.x) * kPairs + threadIdx.x] = v;
   }
+}
+
+__global__ void k_obs_rho1_sum(const double2 *part, double2 *rho, int d, int nparts) {
+  const int s = blockIdx.x, t = threadIdx.x, pairs = d * (d + 1) / 2;
+  if (t >= d * d) return;
+  const int i = min(t % d, t / d), j = max(t % d, t / d);
+  const int q = i * d - i * (i - 1) / 2 + (j - i);
+  double2 v = make_double2(0.0, 0.0);
+  for (int c = 0; c < nparts; ++c) {
+    const double2 p = part[((size_t)s * nparts + c) * pairs + q];
+    v.x += p.x;
+    v.y += p.y;
+  }
+  if (t % d > t / d) v.y = -v.y;  // rho(i,j), i > j: the conjugate of rho(j,i)
+  rho[(size_t)s * d * d + t] = v;
 }
 
 // rho2[(i,j),(l,k)] = sum_{a,b} Theta(a,i,j,b) conj(Theta(a,l,k,b)) from the slot's
 // compacted Theta X (row i*r0 + a', column j*r2 + b', ld m = d*r0); row index
-// i*d + j, column l*d + k (the gate's order), column-major d^2 x d^2.  One CTA
-// per (row, bond).
-__global__ void __launch_bounds__(kObsThreads) k_obs_rho2(const Slot *slots, double2 *rho2, int d) {
-  __shared__ double2 part[kObsThreads];
-  const int s = blockIdx.y, row = blockIdx.x;
+// i*d + j, column l*d + k (the gate's order), column-major d^2 x d^2.  A CTA takes a
+// part of the (a', b') pairs of one bond, staged kRhoE at a time with their d^2 entries,
+// its threads the (row, column) pairs with row <= column; sums to part[bond][CTA], added
+// in order by k_obs_rho2_sum.  (One CTA per row, two global reads per multiply-add,
+// took 4.2 ms for 32 bonds of 640 x 640; now 3.1 ms, nearly the FP64 pipe's 2.6.)
+constexpr int kRhoE = 16;
+__global__ void __launch_bounds__(kObsThreads) k_obs_rho2(const Slot *slots, double2 *part, int d) {
+  extern __shared__ double2 th[];  // kRhoE x d^2
+  const int s = blockIdx.y;
   const Slot S = slots[s];
   const Compact cp = *S.cp;
-  const int r0 = cp.r0, r2 = cp.r2, m = cp.m;
-  const int d2 = d * d, nch = kObsThreads / d2;
-  const int t = threadIdx.x, col = t % d2, ch = t / d2;
-  const int i = row / d, j = row % d, l = col / d, k = col % d;
-  double2 acc = make_double2(0.0, 0.0);
-  if (ch < nch)
-    for (size_t e = ch; e < (size_t)r0 * r2; e += nch) {
-      const int a = (int)(e % r0), b = (int)(e / r0);
-      cacc(acc, S.X[(i * r0 + a) + (size_t)m * (j * r2 + b)], S.X[(l * r0 + a) + (size_t)m * (k * r2 + b)],
-           1.0);
+  const int r0 = cp.r0, r2 = cp.r2, m = cp.m, d2 = d * d, pairs = d2 * (d2 + 1) / 2;
+  const int total = r0 * r2, per = (total + gridDim.x - 1) / gridDim.x;
+  const int e0 = blockIdx.x * per, e1 = min(total, e0 + per);
+  double2 *out = part + ((size_t)s * gridDim.x + blockIdx.x) * pairs;
+  // pairs of one pass: as many as the threads hold accumulators for, two each
+  for (int p0 = 0; p0 < pairs; p0 += 2 * kObsThreads) {
+    int row[2], col[2];
+    double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      int q = p0 + u * kObsThreads + threadIdx.x, r = 0;
+      if (q >= pairs) q = pairs - 1;
+      while (q >= d2 - r) {
+        q -= d2 - r;
+        ++r;
+      }
+      row[u] = r;
+      col[u] = r + q;
     }
-  part[t] = acc;
-  __syncthreads();
-  if (t < d2) {
-    double2 r = make_double2(0.0, 0.0);
-    for (int c = 0; c < nch; ++c) {
-      r.x += part[t + c * d2].x;
-      r.y += part[t + c * d2].y;
+    const bool two = p0 + kObsThreads < pairs;
+    for (int e = e0; e < e1; e += kRhoE) {
+      const int ne = min(kRhoE, e1 - e);
+      __syncthreads();
+      for (int t = threadIdx.x; t < kRhoE * d2; t += kObsThreads) {
+        const int x = t % kRhoE, ij = t / kRhoE;
+        double2 v = make_double2(0.0, 0.0);
+        if (x < ne) {
+          const int a = (e + x) % r0, b = (e + x) / r0;
+          v = S.X[((ij / d) * r0 + a) + (size_t)m * ((ij % d) * r2 + b)];
+        }
+        th[x * d2 + ij] = v;
+      }
+      __syncthreads();
+      for (int x = 0; x < ne; ++x) {
+        cacc(acc[0], th[x * d2 + row[0]], th[x * d2 + col[0]], 1.0);
+        if (two) cacc(acc[1], th[x * d2 + row[1]], th[x * d2 + col[1]], 1.0);
+      }
     }
-    rho2[(size_t)s * d2 * d2 + row + (size_t)d2 * t] = r;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (p0 + u * kObsThreads + threadIdx.x < pairs) out[p0 + u * kObsThreads + threadIdx.x] = acc[u];
   }
 }
 
-__global__ void k_obs_identity_gates(double2 *gates, int d2, int nb) {
-  const size_t total = (size_t)nb * d2 * d2;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const size_t q = e % ((size_t)d2 * d2);
-    gates[e] = make_double2((q % d2) == (q / d2) ? 1.0 : 0.0, 0.0);
+__global__ void __launch_bounds__(kObsThreads) k_obs_rho2_sum(const Slot *slots, const double2 *part, double2 *rho2,
+                                                              int d, int nparts) {
+  const int s = blockIdx.y, d2 = d * d, pairs = d2 * (d2 + 1) / 2;
+  const int t = blockIdx.x * kObsThreads + threadIdx.x;
+  if (t >= d2 * d2) return;
+  const int row = t % d2, col = t / d2, r = min(row, col), c = max(row, col);
+  const int q = r * d2 - r * (r - 1) / 2 + (c - r);
+  double2 v = make_double2(0.0, 0.0);
+  for (int k = 0; k < nparts; ++k) {
+    const double2 p = part[((size_t)s * nparts + k) * pairs + q];
+    v.x += p.x;
+    v.y += p.y;
   }
+  if (row > col) v.y = -v.y;
+  if (slots[s].cp->bad) v = make_double2(nan(""), nan(""));
+  rho2[(size_t)s * d2 * d2 + t] = v;
 }
 
 // S(link) = -sum_{lambda != 0} lambda^2 ln|lambda^2| / ln(d), one warp per link
@@ -122,80 +191,115 @@ __global__ void k_obs_entropy(const double *lam, double *ent, int chi, int nlink
   if (lane == 0) ent[link] = a * inv_logd;
 }
 
-// C (M x N, ld ldc) = sum_k opA(m,k) B(k,n), FP64 complex, 64 x 64 tiles.
-//   opA(m,k) = conjA ? conj(A[k + lda m]) * sa[m] : A[m + lda k]
-//   B(k,n)   = B[k + ldb n] * (sb ? sb[n / sdiv] : 1)
-constexpr int kGT = 64, kGK = 16;
-__global__ void __launch_bounds__(256) k_obs_gemm(int M, int N, int K, const double2 *A, int lda, bool conjA,
-                                                  const double *sa, const double2 *B, int ldb, const double *sb,
-                                                  int sdiv, double2 *C, int ldc) {
+// One product of the overlap's chains: C(m, n) at C[m + ldc n] = sum_k A(m, k) B(k, n),
+// A(m, k) = a[m am + k ak] (conjugated if conj_a) times sa[(m or k) / div], B(k, n) =
+// b[k bk + n bn] times sb[(k or n) / div] where these are given, in FP64.
+struct ObsGemm {
+  int M, N, K, am, ak, bk, bn, ldc;
+  const double2 *a, *b;
+  double2 *c;
+  bool conj_a, sa_k, sb_k;  // scale index: k, else m (n)
+  const double *sa, *sb;
+  int sa_div, sb_div;
+};
+struct ObsGemms {
+  ObsGemm g[2];
+};
+// 16 x 16 tiles: the products are as small as chi x chi x (d chi), and a site's two
+// products wait for the previous site's, so a chain needs every SM on one product
+// (64 x 64 tiles left 4 CTAs on the second product: 3.2 ms per site at d = 5, chi = 128,
+// 204 ms for 64 sites; now 19 ms, 10 of them the FP64 pipe's).
+constexpr int kGT = 16, kGK = 16, kGThreads = 64;
+__global__ void __launch_bounds__(kGThreads) k_obs_gemm(const ObsGemms both) {
   __shared__ double2 As[kGK][kGT + 1], Bs[kGK][kGT + 1];
+  const ObsGemm &p = both.g[blockIdx.z];
   const int m0 = blockIdx.x * kGT, n0 = blockIdx.y * kGT;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  double2 acc[4][4];
+  if (m0 >= p.M || n0 >= p.N) return;  // uniform
+  const int t = threadIdx.x, tx = t & 7, ty = t >> 3;  // rows ty + 8 u, columns tx + 8 v
+  double2 acc[2][2];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = make_double2(0.0, 0.0);
-  for (int k0 = 0; k0 < K; k0 += kGK) {
-    for (int e = t; e < kGK * kGT; e += 256) {
-      int mm, kk;
-      if (conjA) {
-        kk = e % kGK;
-        mm = e / kGK;
-      } else {
-        mm = e % kGT;
-        kk = e / kGT;
+    for (int v = 0; v < 2; ++v) acc[u][v] = make_double2(0.0, 0.0);
+  for (int k0 = 0; k0 < p.K; k0 += kGK) {
+    __syncthreads();
+    for (int e = t; e < kGK * kGT; e += kGThreads) {
+      int x = e % kGT, k = e / kGT;  // the index that is contiguous in memory runs fastest
+      if (p.ak == 1) {
+        k = e % kGK;
+        x = e / kGK;
       }
-      const int gm = m0 + mm, gk = k0 + kk;
-      double2 a = make_double2(0.0, 0.0);
-      if (gm < M && gk < K) {
-        if (conjA) {
-          a = A[gk + (size_t)lda * gm];
-          const double w = sa ? sa[gm] : 1.0;
-          a = make_double2(a.x * w, -a.y * w);
-        } else {
-          a = A[gm + (size_t)lda * gk];
+      double2 v = make_double2(0.0, 0.0);
+      if (m0 + x < p.M && k0 + k < p.K) {
+        v = p.a[(size_t)(m0 + x) * p.am + (size_t)(k0 + k) * p.ak];
+        if (p.sa) {
+          const double w = p.sa[(p.sa_k ? k0 + k : m0 + x) / p.sa_div];
+          v = make_double2(v.x * w, v.y * w);
+        }
+        if (p.conj_a) v.y = -v.y;
+      }
+      As[k][x] = v;
+      x = e % kGT;
+      k = e / kGT;
+      if (p.bk == 1) {
+        k = e % kGK;
+        x = e / kGK;
+      }
+      v = make_double2(0.0, 0.0);
+      if (n0 + x < p.N && k0 + k < p.K) {
+        v = p.b[(size_t)(k0 + k) * p.bk + (size_t)(n0 + x) * p.bn];
+        if (p.sb) {
+          const double w = p.sb[(p.sb_k ? k0 + k : n0 + x) / p.sb_div];
+          v = make_double2(v.x * w, v.y * w);
         }
       }
-      As[kk][mm] = a;
-      const int nn = e / kGK, kb = e % kGK;  // B tile: k fastest
-      const int gn = n0 + nn, gkb = k0 + kb;
-      double2 b = make_double2(0.0, 0.0);
-      if (gn < N && gkb < K) {
-        b = B[gkb + (size_t)ldb * gn];
-        if (sb) {
-          const double w = sb[gn / sdiv];
-          b = make_double2(b.x * w, b.y * w);
-        }
-      }
-      Bs[kb][nn] = b;
+      Bs[k][x] = v;
     }
     __syncthreads();
 #pragma unroll 4
     for (int kk = 0; kk < kGK; ++kk) {
-      double2 av[4], bv[4];
+      double2 av[2], bv[2];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) av[u] = As[kk][ty + 16 * u];
+      for (int u = 0; u < 2; ++u) av[u] = As[kk][ty + 8 * u];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) bv[v] = Bs[kk][tx + 16 * v];
+      for (int v = 0; v < 2; ++v) bv[v] = Bs[kk][tx + 8 * v];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
+        for (int v = 0; v < 2; ++v) {
           acc[u][v].x = fma(av[u].x, bv[v].x, fma(-av[u].y, bv[v].y, acc[u][v].x));
           acc[u][v].y = fma(av[u].x, bv[v].y, fma(av[u].y, bv[v].x, acc[u][v].y));
         }
     }
-    __syncthreads();
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int gm = m0 + ty + 16 * u, gn = n0 + tx + 16 * v;
-      if (gm < M && gn < N) C[gm + (size_t)ldc * gn] = acc[u][v];
+    for (int v = 0; v < 2; ++v) {
+      const int m = m0 + ty + 8 * u, n = n0 + tx + 8 * v;
+      if (m < p.M && n < p.N) p.c[m + (size_t)p.ldc * n] = acc[u][v];
     }
+}
+
+// sum over all entries of E F (one CTA, fixed order)
+__global__ void __launch_bounds__(kObsThreads) k_obs_close(const double2 *E, const double2 *F, size_t n, double2 *out) {
+  __shared__ double2 part[kObsThreads];
+  double2 acc = make_double2(0.0, 0.0);
+  for (size_t e = threadIdx.x; e < n; e += kObsThreads) {
+    const double2 x = E[e], y = F[e];
+    acc.x = fma(x.x, y.x, fma(-x.y, y.y, acc.x));
+    acc.y = fma(x.x, y.y, fma(x.y, y.x, acc.y));
+  }
+  part[threadIdx.x] = acc;
+  __syncthreads();
+  for (int o = kObsThreads / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      part[threadIdx.x].x += part[threadIdx.x + o].x;
+      part[threadIdx.x].y += part[threadIdx.x + o].y;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *out = part[0];
 }
 
 __global__ void k_obs_unit(double2 *E, int chi, double *e1) {  // E = e1 e1^T, e1 = unit vector
@@ -211,8 +315,11 @@ __global__ void k_obs_unit(double2 *E, int chi, double *e1) {  // E = e1 e1^T, e
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// Workspace: rho1 (L d^2) or rho2 (nslots d^4) results, transfer matrices E, E'
-// (chi^2 each), T (chi x d chi), a unit vector (chi doubles), entropies (L+1).
+// Workspace: rho1 (L d^2) or rho2 (nslots d^4) results with the CTAs' partial sums, or,
+// for each of the two chains of an overlap, transfer matrices E, E' (chi^2 each) and T
+// (chi x d chi) with a unit vector (chi doubles), or the entropies (L+1).
+constexpr int kRho1Parts = 32;  // CTAs per site, per bond
+constexpr int kRho2Parts = 10;
 static int obs_ws(tebd_handle *h, size_t bytes) {
   if (h->obs_bytes >= bytes) return TEBD_OK;
   cudaFree(h->obs_buf);
@@ -226,11 +333,11 @@ static int obs_ws(tebd_handle *h, size_t bytes) {
 static int obs_begin(tebd_handle *h) {
   int rc = check_cuda(h, cudaSetDevice(h->device), "cudaSetDevice");
   if (rc) return rc;
-  size_t n = (size_t)h->chi;
-  size_t need = sizeof(double2) * std::max({(size_t)h->L * h->d * h->d,
-                                            (size_t)h->nslots * h->d * h->d * h->d * h->d,
-                                            3 * n * n + n * h->d * n}) +
-                sizeof(double) * (n + h->L + 1) + 1024;
+  const size_t n = (size_t)h->chi, d2 = (size_t)h->d * h->d;
+  const size_t need = sizeof(double2) * std::max({(size_t)h->L * (d2 + kRho1Parts * d2),
+                                                  (size_t)h->nslots * (d2 * d2 + kRho2Parts * d2 * (d2 + 1) / 2),
+                                                  2 * (2 * n * n + n * h->d * n) + 1}) +
+                      sizeof(double) * (n + h->L + 1) + 1024;
   return obs_ws(h, need);
 }
 
@@ -265,10 +372,12 @@ static int obs_rho2(tebd_handle *h, const std::vector<int> &links, std::vector<d
       return rc;
     if ((rc = check_cuda(h, cudaMemsetAsync(h->status_d, 0, sizeof(int) * 4, h->stream), "reset status")))
       return rc;
-    k_obs_identity_gates<<<64, 256, 0, h->stream>>>(h->gates_d, d2, nb);
-    TEBD_LAUNCHED(h);
     if ((rc = launch_dense_prepare(h, nb, false))) return rc;
-    k_obs_rho2<<<dim3(d2, nb), kObsThreads, 0, h->stream>>>(h->slots_d, rho2_d, d);
+    double2 *part = rho2_d + (size_t)h->nslots * d4;
+    const int nparts = std::max(1, std::min(kRho2Parts, 304 / nb));  // two CTAs per SM
+    k_obs_rho2<<<dim3(nparts, nb), kObsThreads, sizeof(double2) * kRhoE * d2, h->stream>>>(h->slots_d, part, d);
+    TEBD_LAUNCHED(h);
+    k_obs_rho2_sum<<<dim3(cdiv(d4, kObsThreads), nb), kObsThreads, 0, h->stream>>>(h->slots_d, part, rho2_d, d, nparts);
     TEBD_LAUNCHED(h);
     std::vector<double2> tmp((size_t)nb * d4);
     if ((rc = check_cuda(h, cudaMemcpyAsync(tmp.data(), rho2_d, sizeof(double2) * tmp.size(),
@@ -276,6 +385,7 @@ static int obs_rho2(tebd_handle *h, const std::vector<int> &links, std::vector<d
                          "read two-site density matrices")))
       return rc;
     if ((rc = obs_finish(h, "two-site density matrices"))) return rc;
+    if ((rc = tc_check(h))) return rc;
     for (int s = 0; s < nb; ++s)
       memcpy(out.data() + (size_t)idx[s] * d4, tmp.data() + (size_t)s * d4, sizeof(double2) * d4);
   }
@@ -304,7 +414,21 @@ extern "C" int tebd_single_site_rho(tebd_handle *h, double *rho) {
   if ((rc = obs_begin(h))) return rc;
   const size_t d2 = (size_t)h->d * h->d;
   double2 *rho_d = reinterpret_cast<double2 *>(h->obs_buf);
-  k_obs_rho1<<<h->L, kObsThreads, 0, h->stream>>>(h->gam, h->lam, rho_d, h->chi, h->d);
+  double2 *part = rho_d + d2 * h->L;
+  const int cols = (int)cdiv(h->chi, kRho1Parts), nparts = (int)cdiv(h->chi, cols);
+  auto rho1 = [&](auto kern) { kern<<<dim3(nparts, h->L), kObsThreads, 0, h->stream>>>(h->gam, h->lam, part, h->chi, cols); };
+  switch (h->d) {
+    case 1: rho1(k_obs_rho1<1>); break;
+    case 2: rho1(k_obs_rho1<2>); break;
+    case 3: rho1(k_obs_rho1<3>); break;
+    case 4: rho1(k_obs_rho1<4>); break;
+    case 5: rho1(k_obs_rho1<5>); break;
+    case 6: rho1(k_obs_rho1<6>); break;
+    case 7: rho1(k_obs_rho1<7>); break;
+    default: rho1(k_obs_rho1<8>); break;
+  }
+  TEBD_LAUNCHED(h);
+  k_obs_rho1_sum<<<h->L, 64, 0, h->stream>>>(part, rho_d, h->d, nparts);
   TEBD_LAUNCHED(h);
   if ((rc = check_cuda(h, cudaMemcpyAsync(rho, rho_d, sizeof(double2) * d2 * h->L, cudaMemcpyDeviceToHost,
                                           h->stream),
@@ -405,31 +529,48 @@ extern "C" int tebd_inner_product(tebd_handle *left, tebd_handle *right, double 
   if ((rc = obs_begin(h))) return rc;
   if (right != left && (rc = check_cuda(h, cudaStreamSynchronize(right->stream), "sync right chain"))) return rc;
   const int chi = h->chi, d = h->d, L = h->L;
-  const size_t cc = (size_t)chi * chi;
-  double2 *E = reinterpret_cast<double2 *>(h->obs_buf), *E2 = E + cc, *T = E2 + cc;
-  double *e1 = reinterpret_cast<double *>(T + cc * d + cc);
+  const size_t cc = (size_t)chi * chi, gsz = cc * d;
+  double2 *ws = reinterpret_cast<double2 *>(h->obs_buf);
+  // [0]: from the left, sites 1..half; [1]: from the right, sites L..half+1.  Both
+  // chains take a site per step in the same launches; their products' ends meet in
+  // sum_{x,y} E(x,y) F(x,y).
+  double2 *E[2] = {ws, ws + cc}, *E2[2] = {ws + 2 * cc, ws + 3 * cc};
+  double2 *T[2] = {ws + 4 * cc, ws + 4 * cc + gsz};
+  double2 *res = ws + 4 * cc + 2 * gsz;
+  double *e1 = reinterpret_cast<double *>(res + 1);
   cudaStream_t st = h->stream;
-  k_obs_unit<<<64, 256, 0, st>>>(E, chi, e1);
-  TEBD_LAUNCHED(h);
-  const size_t gsz = (size_t)chi * d * chi;
-  for (int s = 0; s < L; ++s) {
-    // the reference contracts the first site from left index 1 and the last site
-    // into right index 1 (edge Lambdas e_1), without the edge Lambdas themselves
-    const double *lr = s == L - 1 ? e1 : right->lam + (size_t)(s + 1) * chi;
-    const double *ll = s == L - 1 ? e1 : left->lam + (size_t)(s + 1) * chi;
-    // T = E (Gamma_R Lambda_R): chi x (d chi), column c = i + d beta
-    k_obs_gemm<<<dim3(cdiv(chi, kGT), cdiv((size_t)d * chi, kGT)), 256, 0, st>>>(
-        chi, d * chi, chi, E, chi, false, nullptr, right->gam + s * gsz, chi, lr, d, T, chi);
+  for (int q = 0; q < 2; ++q) {
+    k_obs_unit<<<64, 256, 0, st>>>(E[q], chi, e1);
+    TEBD_LAUNCHED(h);
+  }
+  // the reference contracts the first site from left index 1 and the last site
+  // into right index 1 (edge Lambdas e_1), without the edge Lambdas themselves
+  auto lr = [&](int s) { return s == L - 1 ? e1 : right->lam + (size_t)(s + 1) * chi; };
+  auto ll = [&](int s) { return s == L - 1 ? e1 : left->lam + (size_t)(s + 1) * chi; };
+  const int half = (L + 1) / 2;
+  for (int step = 0; step < half; ++step) {
+    const int nz = L - 1 - step >= half ? 2 : 1, s0 = step, s1 = L - 1 - step;
+    const double2 *gl0 = left->gam + s0 * gsz, *gr0 = right->gam + s0 * gsz;
+    const double2 *gl1 = left->gam + s1 * gsz, *gr1 = right->gam + s1 * gsz;
+    ObsGemms g = {};
+    // T = E (Gamma_R Lambda_R): chi x (d chi), column i + d beta
+    g.g[0] = {chi, d * chi, chi, 1, chi, 1, chi, chi, E[0], gr0, T[0], false, false, false, nullptr, lr(s0), 1, d};
+    // T(alpha' + chi i, beta) = sum_beta' Gamma_R(alpha', i, beta') Lambda_R(beta') F(beta, beta')
+    g.g[1] = {d * chi, chi, chi, 1, d * chi, chi, 1, d * chi, gr1, E[1], T[1], false, true, false, lr(s1), nullptr, 1, 1};
+    k_obs_gemm<<<dim3(cdiv(nz == 2 ? (size_t)d * chi : chi, kGT), cdiv((size_t)d * chi, kGT), nz), kGThreads, 0, st>>>(g);
     TEBD_LAUNCHED(h);
     // E' = (Gamma_L Lambda_L)^H T over (gamma, i): chi x chi
-    k_obs_gemm<<<dim3(cdiv(chi, kGT), cdiv(chi, kGT)), 256, 0, st>>>(chi, chi, d * chi, left->gam + s * gsz,
-                                                                    d * chi, true, ll, T, d * chi, nullptr, 1,
-                                                                    E2, chi);
+    g.g[0] = {chi, chi, d * chi, d * chi, 1, 1, d * chi, chi, gl0, T[0], E2[0], true, false, false, ll(s0), nullptr, 1, 1};
+    // F'(alpha, alpha') = sum_(i, beta) conj(Gamma_L(alpha, i, beta) Lambda_L(beta)) T(alpha', i, beta)
+    g.g[1] = {chi, chi, d * chi, 1, chi, chi, 1, chi, gl1, T[1], E2[1], true, true, false, ll(s1), nullptr, d, 1};
+    k_obs_gemm<<<dim3(cdiv(chi, kGT), cdiv(chi, kGT), nz), kGThreads, 0, st>>>(g);
     TEBD_LAUNCHED(h);
-    std::swap(E, E2);
+    for (int q = 0; q < nz; ++q) std::swap(E[q], E2[q]);
   }
+  k_obs_close<<<1, kObsThreads, 0, st>>>(E[0], E[1], cc, res);
+  TEBD_LAUNCHED(h);
   double2 v;
-  if ((rc = check_cuda(h, cudaMemcpyAsync(&v, E, sizeof(double2), cudaMemcpyDeviceToHost, st), "read overlap")))
+  if ((rc = check_cuda(h, cudaMemcpyAsync(&v, res, sizeof(double2), cudaMemcpyDeviceToHost, st), "read overlap")))
     return rc;
   if ((rc = obs_finish(h, "inner product"))) return rc;
   value[0] = v.x;
