@@ -15,56 +15,28 @@
 //      width 2 eps.
 //   3. Singular vectors of B: inverse iteration on the Golub-Kahan matrix shifted
 //      by sigma_i (tridiagonal LU with partial pivoting, 3 solves from a fixed
-//      pseudo-random start), eigenvector z = (v0,u0,v1,u1,...)/sqrt2; then the
-//      u's and the v's are each re-orthogonalised (classical Gram-Schmidt applied
-//      twice) in descending sigma order, which restores orthogonality inside
-//      clusters of nearby values.
-//   4. U = Q [Ub; 0], V = P Vb by applying the reflectors in reverse, one warp per
-//      kept column; X(:,i) = U(:,i) sigma_i, V(:,i), the same layout the sort and
-//      restore kernels read from the Jacobi routes.
-// Steps 2 to 4 are FP64, step 1 64-bit fixed point.  Cost: 32/3 n^3 (bidiagonalisation) + 16 (m+n) n chi'
+//      start), eigenvector z = (v0,u0,v1,u1,...)/sqrt2; then (bdorth.cu)
+//      the u's and the v's are each re-orthogonalised in descending sigma order.
+//   4. (bdapply.cu) U = Q [Ub; 0], V = P Vb by applying the reflectors in reverse, four at
+//      a time; X(:,i) = U(:,i) sigma_i, V(:,i), the same layout the sort and restore
+//      kernels read from the Jacobi routes.
+// The values and the solves are FP64, everything else 64-bit fixed point, whose products the
+// integer pipe does 5 times faster.  Cost: 32/3 n^3 (bidiagonalisation) + 16 (m+n) n chi'
 // (back-transformation) instead of the Jacobi route's many O(n k^2) sweeps.
-#include <cooperative_groups.h>
 #include <math.h>
 
 #include <algorithm>
-#include <vector>
 
+#include "bidiag.cuh"
 #include "df.cuh"
-#include "tebd_internal.cuh"
 
 namespace tebd {
 
 namespace {
 
-__device__ __forceinline__ double bsum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
-__device__ __forceinline__ bool on_route(int p) { return p == kPathBidiag || p == kPathBidiagT; }
-
-// The matrix that is bidiagonalised, M x N with M >= N, in place in S.X (ld M):
-// Theta itself (m x n) or, on the transposed route, Theta^H (n x m).
-__device__ __forceinline__ void bd_dims(const Compact &cp, int p, int &M, int &N) {
-  M = p == kPathBidiagT ? cp.n : cp.m;
-  N = p == kPathBidiagT ? cp.m : cp.n;
-}
-
-// bdws layout of one bond (doubles): d (n), e (n), sigma (kk), then from an even
-// offset the inverse-iteration scratch U0, U1, U2, PV, Y (2n x K each), the
-// eigenvectors Z (2n x K) and the left vectors Yu (m x K complex, 16-byte aligned)
-__host__ __device__ __forceinline__ size_t bd_scratch(int n, int kk) {
-  return ((size_t)2 * n + kk + 1) & ~(size_t)1;
-}
-
 }  // namespace
-
-// warp sum of a double-float, as a double (each lane's pair is exact in FP64)
-__device__ __forceinline__ double df_warp_sum(float h, float l) { return bsum((double)h + (double)l); }
 
 // ---------------------------------------------------------------------------
 // 2. bisection: sigma_i of B for i < kk (one team of kTeam lanes each), Golub-Kahan Sturm counts
@@ -277,7 +249,7 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
   double *U0 = base, *U1 = base + (size_t)N * K, *U2 = base + 2 * (size_t)N * K,
          *PV = base + 3 * (size_t)N * K, *Y = base + 4 * (size_t)N * K, *Z = base + 5 * (size_t)N * K;
 #define AT(A, j) A[(size_t)(j) * K + i]
-  const double lam = sig[i];
+  double lam = sig[i];
   if (lam <= 0.0) {  // an exactly zero value: FormLambda1 drops it, its vectors are zero
     for (int j = 0; j < N; ++j) AT(Z, j) = 0.0;
     return;
@@ -288,6 +260,14 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
   double tnorm = 0.0;
   for (int j = 0; j < N - 1; ++j) tnorm = fmax(tnorm, fabs(off(j)));
   const double ptol = fmax(2.220446049250313e-16 * tnorm, 1e-300);
+  // The shift lies 64 ulps of ||T|| above the value, so that the members of a cluster (a
+  // degenerate value spreads over tens of ulps by the rounding of B) are all about as far
+  // from it and three solves leave each a like share of the cluster's vectors.  With
+  // the value itself as the shift one member takes all: the set's condition is 1e6 to
+  // 1e13, and its left and right vectors, each re-orthogonalised, no longer belong together
+  // (U diag(s) V^H off by up to 1e-8 ||B|| for 128 equal values; now 5e-15).  A single
+  // value 1e-11 ||T|| or more from the next is resolved to rounding by three solves.
+  lam += 64.0 * ptol;
   auto guard = [&](double p) -> double { return fabs(p) >= ptol ? p : (p < 0.0 ? -ptol : ptol); };
   // LU with partial pivoting of T - lam I (diagonal -lam, off-diagonals off(j))
   double d0 = -lam, d1 = N > 1 ? off(0) : 0.0;
@@ -315,14 +295,20 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
     }
   }
   AT(U0, N - 1) = 1.0 / guard(d0);  // U0 holds the reciprocal pivots
-  // start vector: fixed pseudo-random (splitmix-style hash of (i, j)), max-norm 1/2
-  for (int j = 0; j < N; ++j) {
-    unsigned long long x = (unsigned long long)(i + 1) * 0x9E3779B97F4A7C15ull +
-                           (unsigned long long)j * 0xBF58476D1CE4E5B9ull;
-    x ^= x >> 31;
-    x *= 0x94D049BB133111EBull;
-    x ^= x >> 29;
-    AT(Z, j) = (double)(x >> 11) * (1.0 / 9007199254740992.0) - 0.5;
+  // start vector: row i of the cosine transform with fixed pseudo-random signs on the v's,
+  // zero on the u's.  The rows are orthogonal, so that the starts of a cluster's members
+  // are as independent inside its eigenspace as they can be; of independent random
+  // vectors one in ten is close to a combination of the others.
+  for (int j = 0; j < n; ++j) {
+    unsigned x = (unsigned)(j + 1) * 0x9E3779B9u;  // a published integer hash (Wellons' lowbias32)
+    x ^= x >> 16;
+    x *= 0x7feb352du;
+    x ^= x >> 15;
+    x *= 0x846ca68bu;
+    x ^= x >> 16;
+    const float a = (float)(((long long)(2 * j + 1) * i) % (4 * n)) / (float)(2 * n);
+    AT(Z, 2 * j) = (double)(x & 1 ? cospif(a) : -cospif(a));
+    AT(Z, 2 * j + 1) = 0.0;
   }
   double scale = 1.0;  // the right-hand side is Z * scale
   for (int it = 0; it < 3; ++it) {
@@ -375,362 +361,12 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
 #undef AT
 }
 
-// 3b. split z into v (even rows) and u (odd rows) and re-orthogonalise each set in
-// order of descending sigma by classical Gram-Schmidt, with a second pass only
-// when the first removed more than 1 - 1/sqrt(2) of the vector's norm (the
-// "twice is enough" test of Daniel, Gragg, Kaufman and Stewart).  A cluster of
-// kOrthCluster CTAs per (bond, set) splits the rows; partial dot products and
-// norms meet in the (free by now) inverse-iteration scratch, double-buffered.
-// Z is row-major (element (j, i) at j*K + i): the dot products run one thread per
-// earlier vector over a quarter of the CTA's rows (coalesced across threads), the
-// subtraction one warp per row.
-constexpr int kOrthThreads = 512;
-constexpr int kOrthCluster = 2;
-__global__ void __launch_bounds__(kOrthThreads) k_bd_orth(Slot *slots, const int *path, int kk, int cap) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int C = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  const int s = blockIdx.y, part = blockIdx.x / C;  // part 0: v = z[2j], 1: u = z[2j+1]
-  const int route = path[s];
-  if (!on_route(route)) return;  // uniform per cluster
-  const Slot S = slots[s];
-  int m, n;
-  bd_dims(*S.cp, route, m, n);
-  const int N = 2 * n, K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
-  double *Z = S.bdws + bd_scratch(n, kk) + 5 * (size_t)N * K;
-  double *xch = S.bdws + bd_scratch(n, kk) + (size_t)part * N * K;  // 2 x C x (K + 1)
-  const int j0 = (int)((long long)n * crank / C), j1 = (int)((long long)n * (crank + 1) / C);
-  extern __shared__ double dots[];  // K dot products, then 4 x K partial sums
-  double *psum = dots + K;
-  __shared__ double red[kOrthThreads / 32];
-  __shared__ double nrm_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarp = kOrthThreads / 32;
-  const int qt = tid & 127, jc = tid >> 7;  // 128 vector slots x 4 row quarters
-  int post = 0;                             // postings so far (buffer = post & 1)
-#define ZE(j, i) Z[(size_t)(2 * (j) + part) * K + (i)]
-#define XC(buf, r, q) xch[((size_t)(buf) * C + (r)) * (K + 1) + (q)]
-  // CTA sum of the squared norm of z_i over this CTA's rows
-  auto norm_part = [&](int i) -> double {
-    double a = 0.0;
-    for (int j = j0 + tid; j < j1; j += kOrthThreads) a = fma(ZE(j, i), ZE(j, i), a);
-    a = bsum(a);
-    __syncthreads();
-    if (lane == 0) red[warp] = a;
-    __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < nwarp; ++w) t += red[w];
-    return t;
-  };
-  // post this CTA's dot products of z_i with z_q (q < i) and, optionally, a norm
-  auto post_dots = [&](int i, bool with_norm) {
-    const int buf = post & 1;
-    for (int q = qt; q < i; q += 128) {
-      double a0 = 0.0, a1 = 0.0;
-      int j = j0 + jc;
-      for (; j + 4 < j1; j += 8) {
-        a0 = fma(ZE(j, q), ZE(j, i), a0);
-        a1 = fma(ZE(j + 4, q), ZE(j + 4, i), a1);
-      }
-      for (; j < j1; j += 4) a0 = fma(ZE(j, q), ZE(j, i), a0);
-      psum[jc * K + q] = a0 + a1;
-    }
-    const double nr = with_norm ? norm_part(i) : 0.0;  // (its barriers also order psum)
-    __syncthreads();
-    for (int q = tid; q < i; q += kOrthThreads)
-      XC(buf, crank, q) = (psum[q] + psum[K + q]) + (psum[2 * K + q] + psum[3 * K + q]);
-    if (with_norm && tid == 0) XC(buf, crank, K) = nr;
-  };
-  // gather the posted dots (q < i) into shared memory and return the posted norm
-  auto gather = [&](int i, bool dots_too) -> double {
-    const int buf = post & 1;
-    if (dots_too)
-      for (int q = tid; q < i; q += kOrthThreads) {
-        double t = 0.0;
-        for (int r = 0; r < C; ++r) t += __ldcg(&XC(buf, r, q));
-        dots[q] = t;
-      }
-    if (tid == 0) {
-      double t = 0.0;
-      for (int r = 0; r < C; ++r) t += __ldcg(&XC(buf, r, K));
-      nrm_s = t;
-    }
-    __syncthreads();
-    ++post;
-    return nrm_s;
-  };
-  auto subtract = [&](int i) {
-    for (int j = j0 + warp; j < j1; j += nwarp) {
-      double a = 0.0;
-      for (int q = lane; q < i; q += 32) a = fma(dots[q], ZE(j, q), a);
-      a = bsum(a);
-      if (lane == 0) ZE(j, i) -= a;
-    }
-    __syncthreads();
-  };
-  auto post_norm = [&](int i) {
-    const double nr = norm_part(i);
-    if (tid == 0) XC(post & 1, crank, K) = nr;
-  };
-  for (int i = 0; i < K; ++i) {
-    post_dots(i, true);
-    cluster.sync();
-    const double nrm0 = gather(i, true);
-    double nrm = nrm0;
-    if (i > 0) {
-      subtract(i);
-      post_norm(i);
-      cluster.sync();
-      nrm = gather(i, false);
-      if (nrm < 0.5 * nrm0) {  // second pass
-        post_dots(i, false);
-        cluster.sync();
-        gather(i, true);
-        subtract(i);
-        post_norm(i);
-        cluster.sync();
-        nrm = gather(i, false);
-      }
-    }
-    const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
-    for (int j = j0 + tid; j < j1; j += kOrthThreads) ZE(j, i) *= inv;
-    __syncthreads();
-  }
-#undef ZE
-#undef XC
-}
-
-// Precision form of step 3's re-orthogonalisation: the same schedule on Z held
-// as double-float (float2 per real, converted in place by k_bd_z_df before and
-// back after), so the dot products and the subtractions run on the FP32 pipe;
-// the cross-lane and cross-CTA sums and the norms stay FP64.
-__global__ void k_bd_z_df(Slot *slots, const int *path, int kk, int cap, int to_df) {
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;
-  const Slot S = slots[s];
-  int m, n;
-  bd_dims(*S.cp, route, m, n);
-  const int N = 2 * n, K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
-  double *Z = S.bdws + bd_scratch(n, kk) + 5 * (size_t)N * K;
-  float2 *Zf = reinterpret_cast<float2 *>(Z);
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)N * K;
-       e += (size_t)gridDim.x * blockDim.x) {
-    if (to_df) {
-      const double x = Z[e];
-      const float h = (float)x;
-      Zf[e] = make_float2(h, (float)(x - (double)h));
-    } else {
-      const float2 v = Zf[e];
-      Z[e] = (double)v.x + (double)v.y;
-    }
-  }
-}
-
-__device__ __forceinline__ void df_fma2(float &h, float &l, float2 a, float2 b) { df_mac(h, l, a.x, a.y, b.x, b.y); }
-
-__global__ void __launch_bounds__(kOrthThreads) k_bd_orth_df(Slot *slots, const int *path, int kk, int cap) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int C = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  const int s = blockIdx.y, part = blockIdx.x / C;  // part 0: v = z[2j], 1: u = z[2j+1]
-  const int route = path[s];
-  if (!on_route(route)) return;  // uniform per cluster
-  const Slot S = slots[s];
-  int m, n;
-  bd_dims(*S.cp, route, m, n);
-  const int N = 2 * n, K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
-  float2 *Z = reinterpret_cast<float2 *>(S.bdws + bd_scratch(n, kk) + 5 * (size_t)N * K);
-  double *xch = S.bdws + bd_scratch(n, kk) + (size_t)part * N * K;  // 2 x C x (K + 1)
-  const int j0 = (int)((long long)n * crank / C), j1 = (int)((long long)n * (crank + 1) / C);
-  extern __shared__ double dots[];  // K dot products, then 4 x K partial sums
-  double *psum = dots + K;
-  float2 *dotf = reinterpret_cast<float2 *>(psum);  // the dots as double-float for the subtraction
-  __shared__ double red[kOrthThreads / 32];
-  __shared__ double nrm_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarp = kOrthThreads / 32;
-  const int qt = tid & 127, jc = tid >> 7;
-  int post = 0;
-#define ZE(j, i) Z[(size_t)(2 * (j) + part) * K + (i)]
-#define XC(buf, r, q) xch[((size_t)(buf) * C + (r)) * (K + 1) + (q)]
-  auto norm_part = [&](int i) -> double {
-    float h = 0.f, l = 0.f;
-    for (int j = j0 + tid; j < j1; j += kOrthThreads) df_fma2(h, l, ZE(j, i), ZE(j, i));
-    const double a = bsum((double)h + (double)l);
-    __syncthreads();
-    if (lane == 0) red[warp] = a;
-    __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < nwarp; ++w) t += red[w];
-    return t;
-  };
-  auto post_dots = [&](int i, bool with_norm) {
-    const int buf = post & 1;
-    for (int q = qt; q < i; q += 128) {
-      float h = 0.f, l = 0.f;
-      for (int j = j0 + jc; j < j1; j += 4) df_fma2(h, l, ZE(j, q), ZE(j, i));
-      psum[jc * K + q] = (double)h + (double)l;
-    }
-    const double nr = with_norm ? norm_part(i) : 0.0;  // (its barriers also order psum)
-    __syncthreads();
-    for (int q = tid; q < i; q += kOrthThreads)
-      XC(buf, crank, q) = (psum[q] + psum[K + q]) + (psum[2 * K + q] + psum[3 * K + q]);
-    if (with_norm && tid == 0) XC(buf, crank, K) = nr;
-  };
-  auto gather = [&](int i, bool dots_too) -> double {
-    const int buf = post & 1;
-    if (dots_too)
-      for (int q = tid; q < i; q += kOrthThreads) {
-        double t = 0.0;
-        for (int r = 0; r < C; ++r) t += __ldcg(&XC(buf, r, q));
-        dots[q] = t;
-      }
-    if (tid == 0) {
-      double t = 0.0;
-      for (int r = 0; r < C; ++r) t += __ldcg(&XC(buf, r, K));
-      nrm_s = t;
-    }
-    __syncthreads();
-    ++post;
-    return nrm_s;
-  };
-  auto subtract = [&](int i) {
-    for (int q = tid; q < i; q += kOrthThreads) {  // the dots as double-float (psum is free here)
-      const double x = dots[q];
-      const float hq = (float)x;
-      dotf[q] = make_float2(hq, (float)(x - (double)hq));
-    }
-    __syncthreads();
-    // one thread per row: row j of Z is contiguous in q, the dots are broadcast
-    // from shared memory, and no cross-lane reduction is needed
-    for (int j = j0 + tid; j < j1; j += kOrthThreads) {
-      float h = 0.f, l = 0.f;
-      for (int q = 0; q < i; ++q) df_fma2(h, l, dotf[q], ZE(j, q));
-      const float2 z = ZE(j, i);
-      const double r = ((double)z.x + (double)z.y) - ((double)h + (double)l);
-      const float rh = (float)r;
-      ZE(j, i) = make_float2(rh, (float)(r - (double)rh));
-    }
-    __syncthreads();
-  };
-  auto post_norm = [&](int i) {
-    const double nr = norm_part(i);
-    if (tid == 0) XC(post & 1, crank, K) = nr;
-  };
-  for (int i = 0; i < K; ++i) {
-    post_dots(i, true);
-    cluster.sync();
-    const double nrm0 = gather(i, true);
-    double nrm = nrm0;
-    if (i > 0) {
-      subtract(i);
-      post_norm(i);
-      cluster.sync();
-      nrm = gather(i, false);
-      if (nrm < 0.5 * nrm0) {  // second pass
-        post_dots(i, false);
-        cluster.sync();
-        gather(i, true);
-        subtract(i);
-        post_norm(i);
-        cluster.sync();
-        nrm = gather(i, false);
-      }
-    }
-    const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
-    for (int j = j0 + tid; j < j1; j += kOrthThreads) {
-      const float2 z = ZE(j, i);
-      const double r = ((double)z.x + (double)z.y) * inv;
-      const float rh = (float)r;
-      ZE(j, i) = make_float2(rh, (float)(r - (double)rh));
-    }
-    __syncthreads();
-  }
-#undef ZE
-#undef XC
-}
-
-// ---------------------------------------------------------------------------
-// 4. left vectors Q [Ub; 0] (M x K) and right vectors P Vb (N x K) of the
-//    bidiagonalised matrix, one warp per kept column.
-//    Theta route:   left -> Yu (scratch), right -> S.V (ld n).
-//    Theta^H route: left -> Yu (= V of Theta), right -> Ru (= U of Theta, scratch
-//    in the inverse-iteration LU area, free by now).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_bd_apply(Slot *slots, const int *path, int kk, int cap) {
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;
-  const Slot S = slots[s];
-  int m, n;
-  bd_dims(*S.cp, route, m, n);
-  const int N = 2 * n, K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * 8 + warp;
-  if (col >= 2 * K) return;
-  double *base = S.bdws + bd_scratch(n, kk);
-  const double *Z = base + 5 * (size_t)N * K;
-  double2 *Yu = reinterpret_cast<double2 *>(base + 6 * (size_t)N * K);
-  double2 *Ru = route == kPathBidiagT ? reinterpret_cast<double2 *>(base) : S.V;
-  const double2 *Pv = S.aux;
-  if (col < K) {  // left: Y = H(0) ... H(n-1) [u; 0]
-    const int i = col;
-    double2 *Y = Yu + (size_t)m * i;
-    for (int r = lane; r < m; r += 32)
-      Y[r] = make_double2(r < n ? Z[(size_t)(2 * r + 1) * K + i] : 0.0, 0.0);
-    __syncwarp();
-    for (int j = n - 1; j >= 0; --j) {
-      const double2 tq = S.tau[j];
-      double wr = 0.0, wi = 0.0;
-      for (int r = j + lane; r < m; r += 32) {
-        const double2 y = Y[r];
-        const double2 v = r == j ? make_double2(1.0, 0.0) : S.X[r + (size_t)m * j];
-        wr = fma(v.x, y.x, fma(v.y, y.y, wr));
-        wi = fma(v.x, y.y, fma(-v.y, y.x, wi));
-      }
-      wr = bsum(wr);
-      wi = bsum(wi);
-      const double fr = tq.x * wr - tq.y * wi, fi = tq.x * wi + tq.y * wr;
-      for (int r = j + lane; r < m; r += 32) {
-        const double2 v = r == j ? make_double2(1.0, 0.0) : S.X[r + (size_t)m * j];
-        double2 y = Y[r];
-        y.x -= v.x * fr - v.y * fi;
-        y.y -= v.x * fi + v.y * fr;
-        Y[r] = y;
-      }
-      __syncwarp();
-    }
-  } else {  // right: Y = G(0) ... G(n-2) v
-    const int i = col - K;
-    double2 *Y = Ru + (size_t)n * i;
-    for (int r = lane; r < n; r += 32) Y[r] = make_double2(Z[(size_t)(2 * r) * K + i], 0.0);
-    __syncwarp();
-    for (int j = n - 2; j >= 0; --j) {
-      const double2 tp = S.taup[j];
-      double wr = 0.0, wi = 0.0;
-      for (int r = j + 1 + lane; r < n; r += 32) {
-        const double2 y = Y[r];
-        const double2 u = Pv[r + (size_t)n * j];
-        wr = fma(u.x, y.x, fma(u.y, y.y, wr));
-        wi = fma(u.x, y.y, fma(-u.y, y.x, wi));
-      }
-      wr = bsum(wr);
-      wi = bsum(wi);
-      const double fr = tp.x * wr - tp.y * wi, fi = tp.x * wi + tp.y * wr;
-      for (int r = j + 1 + lane; r < n; r += 32) {
-        const double2 u = Pv[r + (size_t)n * j];
-        double2 y = Y[r];
-        y.x -= u.x * fr - u.y * fi;
-        y.y -= u.x * fi + u.y * fr;
-        Y[r] = y;
-      }
-      __syncwarp();
-    }
-  }
-}
+// 3b. the v's (even rows) and u's (odd rows) re-orthogonalised: bdorth.cu
+// 4. left vectors Q [Ub; 0] (M x K) and right vectors P Vb (N x K): bdapply.cu
 
 // X(:, i) = U(:, i) sigma_i (Theta's m rows, ld m) and, on the transposed route,
 // V(:, i) = the left vectors of Theta^H (n rows, ld n).
-__global__ void k_bd_store(Slot *slots, const int *path, int kk, int cap) {
+__global__ void k_bd_store(Slot *slots, const int *path, int kk, int cap, int right_only) {
   const int s = blockIdx.y;
   const int route = path[s];
   if (!on_route(route)) return;
@@ -741,9 +377,9 @@ __global__ void k_bd_store(Slot *slots, const int *path, int kk, int cap) {
   double *base = S.bdws + bd_scratch(N, kk);
   const double *sig = S.bdws + 2 * N;
   const double2 *Yu = reinterpret_cast<const double2 *>(base + 12 * (size_t)N * K);
-  const double2 *U = route == kPathBidiagT ? reinterpret_cast<const double2 *>(base) : Yu;
+  const double2 *U = route == kPathBidiagT ? reinterpret_cast<const double2 *>(base + 10 * (size_t)N * K) : Yu;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)m * K; e += stride) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; !right_only && e < (size_t)m * K; e += stride) {
     const int i = (int)(e / m);
     const double2 y = U[e];
     S.X[e] = make_double2(y.x * sig[i], y.y * sig[i]);
@@ -757,116 +393,6 @@ __global__ void k_bd_store(Slot *slots, const int *path, int kk, int cap) {
   } else if (blockIdx.x == 0 && threadIdx.x == 0) {
     S.cp->k = K;
   }
-}
-
-// Precision form of step 4: the same reflector products in double-float, reading
-// the left reflectors from the double-float matrix the bidiagonalisation left in
-// S.X and the right ones from Pv converted in place (k_bd_pv_to_df); the vectors
-// Yu / Ru are double-float too and k_bd_store_df converts them.
-__global__ void __launch_bounds__(256) k_bd_apply_df(Slot *slots, const int *path, int kk, int cap,
-                                                     int right_only) {
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;
-  const Slot S = slots[s];
-  int m, n;
-  bd_dims(*S.cp, route, m, n);
-  const int N = 2 * n, K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * 8 + warp + (right_only ? K : 0);  // right only: columns K .. 2K-1
-  if (col >= 2 * K) return;
-  double *base = S.bdws + bd_scratch(n, kk);
-  const double *Z = base + 5 * (size_t)N * K;
-  float4 *Yu = reinterpret_cast<float4 *>(base + 6 * (size_t)N * K);
-  float4 *Ru = route == kPathBidiagT ? reinterpret_cast<float4 *>(base) : reinterpret_cast<float4 *>(S.V);
-  const float4 *Xf = reinterpret_cast<const float4 *>(S.X);
-  const float4 *Pf = reinterpret_cast<const float4 *>(S.aux);
-  const float4 one = make_float4(1.f, 0.f, 0.f, 0.f);
-  const bool left = col < K;
-  const int i = left ? col : col - K;
-  const int len = left ? m : n;
-  float4 *Y = left ? Yu + (size_t)m * i : Ru + (size_t)n * i;
-  for (int r = lane; r < len; r += 32)
-    Y[r] = dfs(make_double2(left ? (r < n ? Z[(size_t)(2 * r + 1) * K + i] : 0.0) : Z[(size_t)(2 * r) * K + i], 0.0));
-  __syncwarp();
-  for (int j = left ? n - 1 : n - 2; j >= 0; --j) {
-    // reflector j: left v (rows j.., v(j) = 1) or right u (rows j+1.., u(j+1) = 1)
-    const int r0 = left ? j : j + 1;
-    const float4 *vc = left ? Xf + (size_t)m * j : Pf + (size_t)n * j;
-    const double2 t = left ? S.tau[j] : S.taup[j];
-    float wrh = 0.f, wrl = 0.f, wih = 0.f, wil = 0.f;  // w = sum conj(v) y
-    for (int r = r0 + lane; r < len; r += 32)
-      df_cmac_ca(wrh, wrl, wih, wil, (left && r == j) ? one : __ldcg(vc + r), Y[r]);
-    const double wr = df_warp_sum(wrh, wrl), wi = df_warp_sum(wih, wil);
-    const float4 f = dfs(make_double2(t.x * wr - t.y * wi, t.x * wi + t.y * wr));  // tau w
-    const float4 nf = make_float4(-f.x, -f.y, -f.z, -f.w);
-    for (int r = r0 + lane; r < len; r += 32) {  // y -= v f
-      const float4 v = (left && r == j) ? one : __ldcg(vc + r);
-      float4 y = Y[r];
-      df_mac(y.x, y.y, v.x, v.y, nf.x, nf.y);
-      df_mac(y.x, y.y, v.z, v.w, f.z, f.w);
-      df_mac(y.z, y.w, v.x, v.y, nf.z, nf.w);
-      df_mac(y.z, y.w, v.z, v.w, nf.x, nf.y);
-      Y[r] = df_norm4(y);
-    }
-    __syncwarp();
-  }
-}
-
-__global__ void k_bd_pv_to_df(Slot *slots, const int *path) {  // Pv in place, N x N
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;
-  const Slot S = slots[s];
-  int M, N;
-  bd_dims(*S.cp, route, M, N);
-  float4 *F = reinterpret_cast<float4 *>(S.aux);
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)N * N; e += (size_t)gridDim.x * blockDim.x)
-    F[e] = dfs(S.aux[e]);
-}
-
-__global__ void k_bd_store_df(Slot *slots, const int *path, int kk, int cap, int right_only) {
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;
-  const Slot S = slots[s];
-  int M, N;
-  bd_dims(*S.cp, route, M, N);
-  const int m = S.cp->m, n = S.cp->n, K = cap ? min(min(kk, N), S.cp->k) : min(kk, N);
-  double *base = S.bdws + bd_scratch(N, kk);
-  const double *sig = S.bdws + 2 * N;
-  const float4 *Yu = reinterpret_cast<const float4 *>(base + 12 * (size_t)N * K);
-  const float4 *U = route == kPathBidiagT ? reinterpret_cast<const float4 *>(base) : Yu;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; !right_only && e < (size_t)m * K; e += stride) {
-    const int i = (int)(e / m);
-    const double2 y = dfd(U[e]);
-    S.X[e] = make_double2(y.x * sig[i], y.y * sig[i]);
-  }
-  const float4 *Vs = route == kPathBidiagT ? Yu : reinterpret_cast<const float4 *>(S.V);
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)n * K; e += stride)
-    S.V[e] = dfd(Vs[e]);  // in place on the tall route (same element, same size)
-  if (cap) {  // columns past the capped count read as zero singular values
-    for (size_t e = (size_t)m * K + blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)m * n; e += stride)
-      S.X[e] = make_double2(0.0, 0.0);
-  } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-    S.cp->k = K;
-  }
-}
-
-// Precision form: the M x N matrix of the route as double-float in place before
-// the bidiagonalisation (float4 per complex element); its reflectors stay in that
-// form for k_bd_apply_df.
-__global__ void k_bd_to_df(Slot *slots, const int *path) {
-  const int s = blockIdx.y;
-  const int route = path[s];
-  if (!on_route(route)) return;
-  const Slot S = slots[s];
-  int M, N;
-  bd_dims(*S.cp, route, M, N);
-  float4 *F = reinterpret_cast<float4 *>(S.X);
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)M * N; e += (size_t)gridDim.x * blockDim.x)
-    F[e] = dfs(S.X[e]);
 }
 
 // Transposed route, before the bidiagonalisation: X (m x n, ld m) -> V (copy),
@@ -913,7 +439,7 @@ size_t bidiag_aux_elems(int n) { return gebrd_aux_elems(n, n); }
 
 size_t bidiag_ws_doubles(int n, int chi) {
   const int K = std::min(chi, n);
-  return bd_scratch(n, chi) + 6 * (size_t)(2 * n) * K + 2 * (size_t)n * K;
+  return bd_scratch(n, chi) + 6 * (size_t)(2 * n) * K + 2 * (size_t)n * K + bd_orth_ws_doubles(K);
 }
 
 int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
@@ -936,12 +462,6 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
   if (h->profiling) cudaEventRecord(h->ev[4], st);
   if ((rc = launch_gebrd(h, b))) return rc;
   if (h->profiling) cudaEventRecord(h->ev[5], st);
-  if (b.dfp) {  // the reflectors as double-float for k_bd_apply_df
-    k_bd_to_df<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
-    TEBD_LAUNCHED(h);
-    k_bd_pv_to_df<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
-    TEBD_LAUNCHED(h);
-  }
   ++h->stats.gebrd_launches;
   {
     const size_t smem = (sizeof(double) + sizeof(float2) + sizeof(float)) * (size_t)(2 * nmax);
@@ -966,63 +486,10 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
   }  // vectors
   k_bd_invit<<<dim3(cdiv(kk, 32), nb), 32, 0, st>>>(slots_d, path_d, kk, cap);
   TEBD_LAUNCHED(h);
-  {
-    const size_t smem = sizeof(double) * 5 * (size_t)(kk > 1 ? kk : 1);
-    auto okern = b.dfp ? k_bd_orth_df : k_bd_orth;
-    if ((rc = check_cuda(h, cudaFuncSetAttribute(okern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                         "orthogonalisation shared memory")))
-      return rc;
-    if (b.dfp) {
-      k_bd_z_df<<<dim3(64, nb), 256, 0, st>>>(slots_d, path_d, kk, cap, 1);
-      TEBD_LAUNCHED(h);
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kOrthThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int oc = kOrthCluster;  // or the autotuner's size, when the launch can co-schedule it
-    const TuneParams tpo = tune_lookup(h, b.dfp ? 1 : 0, nmax, nb);
-    if (tpo.orth_cluster > 0) {
-      cfg.gridDim = dim3((b.right_only ? 1 : 2) * tpo.orth_cluster, nb, 1);
-      attr[0].val.clusterDim.x = tpo.orth_cluster;
-      int ncl = 0;
-      if (tpo.orth_cluster <= 8 &&
-          cudaOccupancyMaxActiveClusters(&ncl, (const void *)okern, &cfg) == cudaSuccess && ncl >= 1) {
-        oc = tpo.orth_cluster;
-      } else {
-        cudaGetLastError();
-        tune_reject(h);
-      }
-    }
-    cfg.gridDim = dim3((b.right_only ? 1 : 2) * oc, nb, 1);  // part 0 (right), then 1 (left)
-    attr[0].val.clusterDim.x = oc;
-    if ((rc = check_cuda(h, cudaLaunchKernelEx(&cfg, okern, slots_d, path_d, kk, cap),
-                         "orthogonalisation launch")))
-      return rc;
-    if (b.dfp) {
-      TEBD_LAUNCHED(h);
-      k_bd_z_df<<<dim3(64, nb), 256, 0, st>>>(slots_d, path_d, kk, cap, 0);
-    }
-  }
+  if ((rc = launch_bd_orth(h, b))) return rc;
+  if ((rc = launch_bd_apply(h, b))) return rc;
+  k_bd_store<<<dim3(256, nb), 256, 0, st>>>(slots_d, path_d, kk, cap, b.right_only);
   TEBD_LAUNCHED(h);
-  if (b.dfp) {
-    k_bd_apply_df<<<dim3(cdiv((b.right_only ? 1 : 2) * (size_t)kk, 8), nb), 256, 0, st>>>(slots_d, path_d, kk, cap,
-                                                                                         b.right_only);
-    TEBD_LAUNCHED(h);
-    k_bd_store_df<<<dim3(256, nb), 256, 0, st>>>(slots_d, path_d, kk, cap, b.right_only);
-    TEBD_LAUNCHED(h);
-  } else {
-    k_bd_apply<<<dim3(cdiv(2 * (size_t)kk, 8), nb), 256, 0, st>>>(slots_d, path_d, kk, cap);
-    TEBD_LAUNCHED(h);
-    k_bd_store<<<dim3(256, nb), 256, 0, st>>>(slots_d, path_d, kk, cap);
-    TEBD_LAUNCHED(h);
-  }
   if (h->profiling) {
     cudaEventRecord(h->ev[1], st);
     if ((rc = check_cuda(h, cudaStreamSynchronize(st), "bidiag"))) return rc;
@@ -1053,7 +520,7 @@ int run_bidiag(tebd_handle *h, int nb, int nmax) {
 void bidiag_block_ws(int M, int N, int kk, size_t *aux_elems, size_t *bdws_doubles) {
   const int K = std::min(kk, N);
   *aux_elems = gebrd_aux_elems(M, N);
-  *bdws_doubles = bd_scratch(N, kk) + 6 * (size_t)(2 * N) * K + 2 * (size_t)M * K + 4;
+  *bdws_doubles = bd_scratch(N, kk) + 6 * (size_t)(2 * N) * K + 2 * (size_t)M * K + bd_orth_ws_doubles(K) + 4;
 }
 
 }  // namespace tebd

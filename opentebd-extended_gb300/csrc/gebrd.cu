@@ -29,6 +29,8 @@
 // rows alone (and the 16 dot products, all of them, for itself), all of the raw vector,
 // so the reflector's scale factor can follow later and a column needs two cluster
 // barriers: the current column (then row) and its squared norm are posted before each.
+// The reflectors are left in fixed point (units of 2^-62) for the back-transformation:
+// v_i from its 1 on in column i of S.X, u_i in column i of the N x N array at S.aux.
 //
 // Measured (GB300, 2070 MHz), a batch of 32 matrices of 640 x 640: 148 ms with FP64
 // dot products and FP64 tensor-core updates, 40 ms now; 10 of 270 x 270: 23.2 -> 5.5
@@ -43,6 +45,7 @@
 
 #include <algorithm>
 
+#include "fixed.cuh"
 #include "tebd_internal.cuh"
 
 namespace tebd {
@@ -62,42 +65,11 @@ __host__ __device__ __forceinline__ int own_count(int n, int C) { return up(up(n
 
 __device__ __forceinline__ double2 ldc(const double2 *p) { return __ldcg(p); }
 
-// A fixed-point number x in memory: x + 8 as hi 2^32 + lo with lo signed, so that hi and
-// lo >> 4 are x rounded to 28 bits below hi.  A complex one is (re lo, re hi, im lo, im hi).
-__device__ __forceinline__ int2 enc(long long x) {
-  const long long y = x + 8;
-  return make_int2((int)y, (int)((y + 0x80000000ll) >> 32));
-}
-__device__ __forceinline__ long long dec(int lo, int hi) { return (((long long)hi << 32) + lo) - 8; }
-__device__ __forceinline__ int4 enc2(long long re, long long im) {
-  const int2 a = enc(re), b = enc(im);
-  return make_int4(a.x, a.y, b.x, b.y);
-}
-// a vector entry for the products: (re hi, re lo >> 4, im hi, im lo >> 4)
-__device__ __forceinline__ int4 vec_entry(long long re, long long im) {
-  const int4 e = enc2(re, im);
-  return make_int4(e.y, e.x >> 4, e.w, e.z >> 4);
-}
 __device__ __forceinline__ double wsum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-
-// x 2^sh rounded to an integer, |x| 2^sh < 2^63, in integer instructions (the FP64
-// pipe, at 16 cycles per warp instruction, is what the kernel must spare)
-__device__ __forceinline__ long long to_fix(double x, int sh) {
-  const long long b = __double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7ff);
-  const long long m = (b & 0xfffffffffffffll) | 0x10000000000000ll;
-  const int s = e - 1075 + sh;
-  long long r = s >= 0 ? m << min(s, 10) : (s > -54 ? (m + (1ll << (-s - 1))) >> (-s) : 0ll);
-  if (e == 0) r = 0;
-  return b < 0 ? -r : r;
-}
-
-// 2^k as a double, -1022 <= k <= 1023
-__device__ __forceinline__ double pow2(int k) { return __longlong_as_double((long long)(k + 1023) << 52); }
 
 // ZLARFG's scalars from alpha and ||x||^2: beta (real), tau, and 1/(alpha - beta).  One
 // FP64 instruction holds a warp's scheduler for 64 cycles, so the root and the two
@@ -192,7 +164,8 @@ __host__ __device__ __forceinline__ size_t ws_elems(int M, int N) {
 // The problem, in shared memory: held in registers it would push the loops' own values
 // into local memory.
 struct Ctx {
-  double2 *X, *Pv, *tau, *taup;
+  double2 *X, *tau, *taup;
+  int4 *Pv;
   double *d, *e;
   int4 *A;             // fixed-point matrix
   int4 *Li, *Ri;       // [V X], [Y U]: V, U in units of 2^-62, X, Y in units of 2^(eA - 58)
@@ -244,53 +217,6 @@ __device__ __forceinline__ int first_own(int x, int C, int rank) {
   const int o = b <= rank ? 0 : (b - rank + C - 1) / C;
   return o * 8 + ((o * C + rank) == b ? (x & 7) : 0);
 }
-
-__device__ __forceinline__ void mw(long long &acc, int a, int b) { acc += (long long)a * b; }  // one IMAD.WIDE
-
-// A sum in halves: h of the high x high products, x of the cross terms
-struct Acc {
-  long long hr = 0, hi = 0, xr = 0, xi = 0;
-  // += a v: `a` as stored, v a vector entry, nh, nl the negatives of v.z, v.w
-  __device__ __forceinline__ void add(const int4 &a, const int4 &v, int nh, int nl) {
-    const int arl = a.x >> 4, ail = a.z >> 4;
-    mw(hr, a.y, v.x);
-    mw(hr, a.w, nh);
-    mw(hi, a.y, v.z);
-    mw(hi, a.w, v.x);
-    mw(xr, a.y, v.y);
-    mw(xr, arl, v.x);
-    mw(xr, a.w, nl);
-    mw(xr, ail, nh);
-    mw(xi, a.y, v.w);
-    mw(xi, arl, v.z);
-    mw(xi, a.w, v.y);
-    mw(xi, ail, v.x);
-  }
-  // += conj(a) v: nh, nl the negatives of v.x, v.y
-  __device__ __forceinline__ void add_conj(const int4 &a, const int4 &v, int nh, int nl) {
-    const int arl = a.x >> 4, ail = a.z >> 4;
-    mw(hr, a.y, v.x);
-    mw(hr, a.w, v.z);
-    mw(hi, a.y, v.z);
-    mw(hi, a.w, nh);
-    mw(xr, a.y, v.y);
-    mw(xr, arl, v.x);
-    mw(xr, a.w, v.w);
-    mw(xr, ail, v.z);
-    mw(xi, a.y, v.w);
-    mw(xi, arl, v.z);
-    mw(xi, a.w, nl);
-    mw(xi, ail, nh);
-  }
-  // in units of 2^(64 - kUp) times the factors' own (h has 2^64, x 2^36)
-  template <int kUp>
-  __device__ __forceinline__ longlong2 value() const {
-    constexpr int dn = 28 - kUp;
-    constexpr long long half = 1ll << (dn - 1);
-    return make_longlong2((long long)((unsigned long long)hr << kUp) + ((xr + half) >> dn),
-                          (long long)((unsigned long long)hi << kUp) + ((xi + half) >> dn));
-  }
-};
 
 // D^H x for two columns of D (leading dimension ldd; entries [ka, kb), multiples of 32)
 // by one warp, lanes over k, x in shared memory.  Lane 8 q returns value q: the real and
@@ -701,15 +627,16 @@ __device__ __noinline__ void put_reflector(bool left, int i, int j, double2 mine
   const double2 sc = scal(left ? 0 : 1).sc;
   const double2 *raw = left ? x.col : x.row;
   int4 *P = left ? x.Li + (size_t)x.Mp * j : x.Ri + (size_t)x.Np * (8 + j);
-  double2 *out = left ? x.X + (size_t)x.M * i : x.Pv + (size_t)x.N * i;
+  int4 *out = left ? reinterpret_cast<int4 *>(x.X) + (size_t)x.M * i : x.Pv + (size_t)x.N * i;
   const int o0 = first_own(one, C, rank) + tid;
   for (int o = o0; o < own; o += kThreads) {
     const int r = glob(o, C, rank);
     if (r >= lim) continue;
     const double2 v = r == one ? make_double2(1.0, 0.0) : cmul(o == o0 ? mine : ldc(&raw[r]), sc);
-    P[r] = enc2(to_fix(v.x, 62), to_fix(v.y, 62));
-    if (!left || r > i) out[r] = v;
+    P[r] = out[r] = enc2(to_fix(v.x, 62), to_fix(v.y, 62));
   }
+  // the back-transformation takes four reflectors together, from the first one's start
+  if (x.rank == 0 && tid < (i & 3)) out[one - 1 - tid] = make_int4(8, 0, 8, 0);
 }
 
 // raw column q of the matrix (panel start) for the own rows; returns this thread's first entry
@@ -768,7 +695,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gebrd(Slot *slots, const int *p
       p += n;
       return q;
     };
-    c.Pv = take((size_t)c.N * c.N);
+    c.Pv = reinterpret_cast<int4 *>(take((size_t)c.N * c.N));
     c.A = reinterpret_cast<int4 *>(take((size_t)c.Mp * c.Np));
     c.Li = reinterpret_cast<int4 *>(take(16 * (size_t)c.Mp));
     c.Ri = reinterpret_cast<int4 *>(take(16 * (size_t)c.Np));
