@@ -41,109 +41,82 @@ inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 // ---------------------------------------------------------------------------
 // 2. bisection: sigma_i of B for i < kk (one team of kTeam lanes each), Golub-Kahan Sturm counts
 // ---------------------------------------------------------------------------
-// Sturm count of the Golub-Kahan matrix: eigenvalues below x; sq = squared
-// off-diagonals (2n-1 of them).  Two independent recurrences interleave.
-__device__ __forceinline__ void gk_count2(const double *sq, int n1, double x0, double x1, double pivmin,
-                                          int &c0, int &c1) {
-  double q0 = -x0, q1 = -x1;
-  c0 = q0 < 0.0;
-  c1 = q1 < 0.0;
-  for (int j = 0; j < n1; ++j) {
-    const double o2 = sq[j];
-    if (fabs(q0) < pivmin) q0 = -pivmin;
-    if (fabs(q1) < pivmin) q1 = -pivmin;
-    q0 = -x0 - o2 / q0;
-    q1 = -x1 - o2 / q1;
-    c0 += q0 < 0.0;
-    c1 += q1 < 0.0;
-  }
-}
+// Sturm counts of the Golub-Kahan matrix (eigenvalues below x) from the characteristic
+// polynomials of its leading blocks, p_{j+2} = -x p_{j+1} - o_j^2 p_j: the count is the number
+// of sign changes, a zero counting as either sign.  No divisions: an FP64 step is two
+// instructions (130 cycles of a scheduler) where the quotient form's takes 645, and one
+// FP32 step 10 cycles against 45.  Each computed p_{j+2} satisfies the recurrence with x and
+// o_j^2 changed by a few ulps, so that the counts are those of a matrix that close, as
+// the quotient form's.  Everything is scaled by the Gershgorin bound (entries in [0, 1]),
+// and the pair is rescaled by powers of two every kRescale steps; squared off-diagonals
+// below kTiny2 (kTiny2F) are raised to it, far below what a count resolves, so that the
+// pair cannot vanish in between.
+constexpr int kRescale = 8, kRescaleF = 4;
+constexpr double kTiny2 = 1e-70;
+constexpr float kTiny2F = 1e-14f;
 
-__device__ __forceinline__ int gk_count(const double *sq, int n1, double x, double pivmin) {
-  double q = -x;
-  int c = q < 0.0;
-  for (int j = 0; j < n1; ++j) {
-    if (fabs(q) < pivmin) q = -pivmin;
-    q = -x - sq[j] / q;
-    c += q < 0.0;
-  }
-  return c;
-}
-
-// the same count in FP32 on off-diagonals scaled by 1/hi (values in [0, 1])
-__device__ __forceinline__ int gk_count_f32(const float *sqf, int n1, float x) {
-  float q = -x;
-  int c = q < 0.0f;
-  for (int j = 0; j < n1; ++j) {
-    if (fabsf(q) < 1e-30f) q = -1e-30f;
-    q = -x - __fdividef(sqf[j], q);
-    c += q < 0.0f;
-  }
-  return c;
-}
-
-// The count in double-float on off-diagonals scaled by 1/hi (FP32 pipe): each step
-// q = -x - o^2/q with Dekker's double-length division (quotient of the leading
-// parts, remainder from an exact product, one correction).  Sign decisions are
-// good to ~2^-44 ||T||; the FP64 stage checks the bracket it produces.
-__device__ __forceinline__ int gk_count_df(const float2 *sqd, int n1, float xh, float xl) {
-  float qh = -xh, ql = -xl;
-  int c = qh < 0.0f;
-  for (int j = 0; j < n1; ++j) {
-    if (fabsf(qh) < 1e-30f) {
-      qh = -1e-30f;
-      ql = 0.0f;
+__device__ __forceinline__ int gk_count(const double *sq, int n1, double x) {
+  double p0 = 1.0, p1 = -x;
+  int c = 1;  // x > 0
+  for (int j = 0; j < n1; j += kRescale) {
+#pragma unroll
+    for (int u = 0; u < kRescale; ++u)
+      if (j + u < n1) {
+        const double p2 = fma(-x, p1, -sq[j + u] * p0);
+        c += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+        p0 = p1;
+        p1 = p2;
+      }
+    const int e = (max(__double2hiint(p0) & 0x7fffffff, __double2hiint(p1) & 0x7fffffff) >> 20) - 1023;
+    if (e != 0) {  // both by 2^-e (what underflows is far below the other)
+      const int h0 = __double2hiint(p0), h1 = __double2hiint(p1), sh = e << 20;
+      p0 = (h0 & 0x7ff00000) > max(sh, 0) ? __hiloint2double(h0 - sh, __double2loint(p0)) : copysign(0.0, p0);
+      p1 = (h1 & 0x7ff00000) > max(sh, 0) ? __hiloint2double(h1 - sh, __double2loint(p1)) : copysign(0.0, p1);
     }
-    const float2 a = sqd[j];
-    const float q1 = __fdiv_rn(a.x, qh);
-    const float ph = __fmul_rn(q1, qh);
-    const float pe = fmaf(q1, qh, -ph);
-    // remainder a - q1 q (exact leading difference, then the small terms)
-    const float rh = __fadd_rn(a.x, -ph);
-    const float rr = __fadd_rn(__fadd_rn(rh, -pe), __fadd_rn(a.y, -__fmul_rn(q1, ql)));
-    const float q2 = __fdiv_rn(rr, qh);
-    // t = q1 + q2 (fast two-sum), then q = -x - t
-    const float th = __fadd_rn(q1, q2);
-    const float tl = __fadd_rn(q2, -__fadd_rn(th, -q1));
-    const float sh = __fadd_rn(-xh, -th);
-    const float bp = __fadd_rn(sh, xh);
-    const float err = __fadd_rn(__fadd_rn(-xh, -__fadd_rn(sh, -bp)), __fadd_rn(-th, -bp));
-    const float sl = __fadd_rn(err, __fadd_rn(-xl, -tl));
-    qh = __fadd_rn(sh, sl);
-    ql = __fadd_rn(sl, -__fadd_rn(qh, -sh));
-    c += qh < 0.0f;
   }
   return c;
 }
 
-// sigma_i of B for i < min(kk, n), descending.  One thread per value, one warp
-// per block so that the FP64 work spreads over the SMs:
-//   1. FP32 bisection on the scaled problem to width 2^-22 ||T||; FP32 Sturm counts
-//      are exact for a T perturbed by a few float ulps, so the bracket widened by
-//      2^-18 ||T|| holds sigma_i; two FP64 counts check it (reset to [0, ||T||]
-//      otherwise).
-//   2. Double-float bisection (FP32 pipe) to width 2^-42 ||T||; the bracket widened
-//      by 2^-40 ||T|| is checked with two FP64 counts (reset to [0, ||T||]
-//      otherwise).
-//   3. FP64 bisection to width 2 eps sigma + eps ||T||: the absolute accuracy
-//      LAPACK's bidiagonal SVD reaches on Theta as a whole.
-//   Each value is found by a team of kTeam lanes that evaluate kTeam points of
-//   the bracket at once (multisection): the counts are monotone in x, so the
-//   leading run of "count <= target" in the team's ballot picks one of kTeam + 1
-//   subintervals (8 lanes: about 3.2 bits per step instead of bisection's 1).
-//   With few values in the batch (a dense sweep: 32 bonds x chi) the kernel is
-//   bound by the latency of the sequential Sturm recurrences and the extra lanes
-//   are free; with many (number-conserving blocks: every value of every block)
-//   the counts fill the GPU on their own and teams of 1 lane (bisection) do the
-//   least work.  The host picks kTeam per launch.
+__device__ __forceinline__ int gk_count_f32(const float *sqf, int n1, float x) {
+  float p0 = 1.0f, p1 = -x;
+  int c = 1;
+  for (int j = 0; j < n1; j += kRescaleF) {
+#pragma unroll
+    for (int u = 0; u < kRescaleF; ++u)
+      if (j + u < n1) {
+        const float p2 = fmaf(-x, p1, -sqf[j + u] * p0);
+        c += (unsigned)(__float_as_int(p2) ^ __float_as_int(p1)) >> 31;
+        p0 = p1;
+        p1 = p2;
+      }
+    const int e = max(__float_as_int(p0) & 0x7fffffff, __float_as_int(p1) & 0x7fffffff) >> 23;
+    const float s = __int_as_float(max(1, min(253, 254 - e)) << 23);  // about 2^-(e - 127)
+    p0 *= s;
+    p1 *= s;
+  }
+  return c;
+}
+
+// sigma_i of B for i < min(kk, n), descending.
+//   1. FP32 bisection on the scaled problem to width 2^-22 ||T||; FP32 counts are exact
+//      for a T perturbed by a few float ulps, so the bracket widened by 2^-18 ||T|| holds
+//      sigma_i; two FP64 counts check it (reset to [0, ||T||] otherwise).
+//   2. FP64 bisection to width 2 eps sigma + eps ||T||: the absolute accuracy LAPACK's
+//      bidiagonal SVD reaches on Theta as a whole.
+// Each value is found by a team of kTeam lanes that evaluate kTeam points of the bracket
+// at once (multisection): the counts are monotone in x, so the leading run of "count <=
+// target" in the team's ballot picks one of kTeam + 1 subintervals (16 lanes: 4.1 bits per
+// step instead of bisection's 1).  While the values leave schedulers idle, the
+// sequential recurrences bound the kernel and extra lanes are free; once there is a warp
+// per scheduler, teams of 1 lane (bisection) do the least work.  The host picks kTeam
+// per launch.  Measured: 128 values of 32 bonds, n = 640: 7.8 -> 2.4 ms; 90 of 10, n =
+// 270: 2.26 -> 0.60 ms.
 constexpr int kSigmaThreads = 32;
 template <int kTeam>
 __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const int *path, int kk) {
   constexpr int kSigmaValues = kSigmaThreads / kTeam;  // values per block
-  // step caps (safety only; the width tests end the loops): log2(kTeam + 1) bits
-  // per step for the 22 bits of the FP32 stage and the ~26 of the double-float one
+  // step cap (safety only; the width test ends the loop): log2(kTeam + 1) bits per step
   constexpr int kIt32 = kTeam == 1 ? 26 : kTeam == 2 ? 17 : kTeam == 4 ? 12 : 10;
-  constexpr int kItDf = kTeam == 1 ? 34 : kTeam == 2 ? 22 : kTeam == 4 ? 16 : 12;
   const int s = blockIdx.y;
   const int route = path[s];
   if (!on_route(route)) return;
@@ -153,9 +126,8 @@ __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const i
   const int K = min(kk, n);
   if ((int)(blockIdx.x * kSigmaValues) >= K) return;  // uniform per block
   const int n1 = 2 * n - 1;
-  extern __shared__ double sq[];  // n1 squared off-diagonals, n1 scaled double-float, n1 scaled FP32
-  float2 *sqd = reinterpret_cast<float2 *>(sq + n1);
-  float *sqf = reinterpret_cast<float *>(sqd + n1);
+  extern __shared__ double sq[];  // n1 scaled squared off-diagonals, then in FP32
+  float *sqf = reinterpret_cast<float *>(sq + n1);
   const double *dd = S.bdws, *ee = S.bdws + n;
   double hl = 0.0;
   for (int j = threadIdx.x; j < n; j += blockDim.x)
@@ -166,11 +138,9 @@ __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const i
   const double inv_hi = 1.0 / hi;
   for (int j = threadIdx.x; j < n1; j += blockDim.x) {
     const double o = (j & 1) ? ee[j >> 1] : dd[j >> 1];
-    sq[j] = o * o;
     const double os = (o * inv_hi) * (o * inv_hi);
-    const float oh = (float)os;
-    sqd[j] = make_float2(oh, (float)(os - (double)oh));
-    sqf[j] = oh;
+    sq[j] = os < kTiny2 ? kTiny2 : os;
+    sqf[j] = fmaxf((float)os, kTiny2F);
   }
   __syncthreads();
   const int team = threadIdx.x / kTeam, t = threadIdx.x % kTeam;
@@ -178,13 +148,12 @@ __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const i
   const int i = blockIdx.x * kSigmaValues + team;
   if (i >= K) return;  // the whole team leaves together
   const int target = 2 * n - 1 - i;  // count(< x) <= target  <=>  x <= sigma_i
-  const double pivmin = 1e-290 * fmax(1.0, hi * hi);
   // leading run of true votes of the team (bit t: point t has count <= target)
   auto lead = [&](bool ok) -> int {
-    const unsigned b = (__ballot_sync(tmask, ok) >> (kTeam * team)) & ((1u << kTeam) - 1u);
-    return __ffs(~b) - 1;
+    const unsigned b = (__ballot_sync(tmask, ok) & tmask) >> (kTeam * team);
+    return b == (kTeam == 32 ? 0xffffffffu : (1u << kTeam) - 1u) ? kTeam : __ffs(~b) - 1;
   };
-  // 1. FP32 bracket of width 2^-22 on the scaled problem
+  // 1. FP32 bracket of width 2^-22
   float lf = 0.0f, hf = 1.0f;
   for (int it = 0; it < kIt32 && hf - lf > 2.384185791015625e-07f; ++it) {
     const float w = (hf - lf) * (1.0f / (kTeam + 1));
@@ -193,47 +162,52 @@ __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const i
     hf = k < kTeam ? lf + w * (float)(k + 1) : hf;
     lf = nl;
   }
-  // 2. double-float stage to 2^-42 from the FP32 bracket widened by 2^-18
-  double ls = fmax(0.0, (double)lf - 3.814697265625e-06), hs = fmin(1.0, (double)hf + 3.814697265625e-06);
-  for (int it = 0; it < kItDf && hs - ls > 2.2737367544323206e-13; ++it) {
-    const double w = (hs - ls) * (1.0 / (kTeam + 1));
-    const double x = ls + w * (double)(t + 1);
-    const float xh = (float)x;
-    const int k = lead(gk_count_df(sqd, n1, xh, (float)(x - (double)xh)) <= target);
-    const double nl = k > 0 ? ls + w * (double)k : ls;
-    hs = k < kTeam ? ls + w * (double)(k + 1) : hs;
-    ls = nl;
+  // widened by 2^-18, and checked
+  double lo = fmax(0.0, (double)lf - 3.814697265625e-06), h = fmin(1.0, (double)hf + 3.814697265625e-06);
+  bool good;
+  if (kTeam == 1) {
+    good = (lo <= 0.0 || gk_count(sq, n1, lo) <= target) && gk_count(sq, n1, h) > target;
+  } else {
+    const int c = gk_count(sq, n1, t == 0 ? fmax(lo, 1e-300) : h);
+    good = __all_sync(tmask, t > 1 || (t == 0 ? c <= target : c > target));
   }
-  double lo = fmax(0.0, ls - 9.094947017729282e-13) * hi;  // widened by 2^-40
-  double h = fmin(1.0, hs + 9.094947017729282e-13) * hi;
-  {
-    int c0, c1;
-    gk_count2(sq, n1, lo, h, pivmin, c0, c1);
-    if (!(c0 <= target && c1 > target)) {
-      lo = 0.0;
-      h = hi;
-    }
+  if (!good) {
+    lo = 0.0;
+    h = 1.0;
   }
-  // 3. FP64 multisection to 2 eps sigma + eps ||T||
-  for (int it = 0; it < 60; ++it) {
-    if (h - lo <= 4.440892098500626e-16 * h + 2.220446049250313e-16 * hi || h < 1e-30 * hi) break;
+  // 2. FP64 multisection to 2 eps sigma + eps ||T||
+  for (int it = 0; it < 80; ++it) {
+    if (h - lo <= 4.440892098500626e-16 * h + 2.220446049250313e-16 || h < 1e-30) break;
     const double w = (h - lo) * (1.0 / (kTeam + 1));
-    const int k = lead(gk_count(sq, n1, lo + w * (double)(t + 1), pivmin) <= target);
+    const int k = lead(gk_count(sq, n1, lo + w * (double)(t + 1)) <= target);
     const double nl = k > 0 ? lo + w * (double)k : lo;
     h = k < kTeam ? lo + w * (double)(k + 1) : h;
     lo = nl;
   }
   const double sg = 0.5 * (lo + h);
-  if (t == 0) S.bdws[2 * n + i] = sg < 1e-30 * hi ? 0.0 : sg;
+  if (t == 0) S.bdws[2 * n + i] = sg < 1e-30 ? 0.0 : sg * hi;
 }
 
 // ---------------------------------------------------------------------------
 // 3a. inverse iteration on (T_GK - sigma_i I), one thread per value.
 // Scratch per value (transposed so that threads of a warp touch adjacent words):
 //   U0 (reciprocal pivots), U1, U2 (upper factor of the pivoted LU), PV (multipliers),
-//   Y (swap flags), then the vector Z itself.
+//   Y (swap flags, ints), then the vector Z itself.
 // ---------------------------------------------------------------------------
-__global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
+// An FP64 instruction holds its scheduler for 65 cycles here and a batch has about a warp
+// per scheduler, so the loops keep to the few that the solves need (comparisons, row
+// swaps and power-of-two scaling on the integer pipe) and load kAhead steps' entries
+// before they are used.  Measured: 128 values of 32 bonds, n = 640: 6.4 -> 2.5 ms; 90 of
+// 10, n = 270: 1.77 -> 0.92 ms.
+constexpr int kAhead = 8;
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ double times_pow2(double x, int e) {  // x 2^e; 0 where it underflows
+  const int h = __double2hiint(x), f = ((h >> 20) & 0x7ff) + e;
+  return f <= 0 || (h & 0x7ff00000) == 0 ? 0.0 : __hiloint2double(h + (e << 20), __double2loint(x));
+}
+__global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
   const int s = blockIdx.y;
   const int route = path[s];
   if (!on_route(route)) return;
@@ -242,24 +216,31 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
   bd_dims(*S.cp, route, m, n);
   const int N = 2 * n;
   const int K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K) return;
+  if ((int)(blockIdx.x * blockDim.x) >= K) return;  // uniform
+  const int i = min((int)(blockIdx.x * blockDim.x + threadIdx.x), K - 1);
+  const bool mine = (int)(blockIdx.x * blockDim.x + threadIdx.x) < K;
   const double *dd = S.bdws, *ee = S.bdws + n, *sig = S.bdws + 2 * n;
   double *base = S.bdws + bd_scratch(n, kk);
-  double *U0 = base, *U1 = base + (size_t)N * K, *U2 = base + 2 * (size_t)N * K,
-         *PV = base + 3 * (size_t)N * K, *Y = base + 4 * (size_t)N * K, *Z = base + 5 * (size_t)N * K;
+  double *U0 = base, *U1 = base + (size_t)N * K, *U2 = base + 2 * (size_t)N * K, *PV = base + 3 * (size_t)N * K,
+         *Z = base + 5 * (size_t)N * K;
+  int *Y = reinterpret_cast<int *>(base + 4 * (size_t)N * K);  // 1: rows j and j + 1 swapped
 #define AT(A, j) A[(size_t)(j) * K + i]
+  extern __shared__ double off[];  // T(j, j+1), j < N - 1
+  for (int j = threadIdx.x; j < N - 1; j += 32) off[j] = (j & 1) ? ee[j >> 1] : dd[j >> 1];
+  __syncwarp();
+  // pivots below eps ||T|| are raised to it (sign kept), as LAPACK's DLAGTS does,
+  // so the solve stays finite when sigma_i is an eigenvalue to working precision
+  unsigned long long tb = 0;
+  for (int j = threadIdx.x; j < N - 1; j += 32) tb = max(tb, abs_bits(off[j]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) tb = max(tb, __shfl_xor_sync(0xffffffffu, tb, o));
+  if (!mine) return;
   double lam = sig[i];
   if (lam <= 0.0) {  // an exactly zero value: FormLambda1 drops it, its vectors are zero
     for (int j = 0; j < N; ++j) AT(Z, j) = 0.0;
     return;
   }
-  auto off = [&](int j) -> double { return (j & 1) ? ee[j >> 1] : dd[j >> 1]; };  // T(j, j+1)
-  // pivots below eps ||T|| are raised to it (sign kept), as LAPACK's DLAGTS does,
-  // so the solve stays finite when sigma_i is an eigenvalue to working precision
-  double tnorm = 0.0;
-  for (int j = 0; j < N - 1; ++j) tnorm = fmax(tnorm, fabs(off(j)));
-  const double ptol = fmax(2.220446049250313e-16 * tnorm, 1e-300);
+  const double ptol = fmax(2.220446049250313e-16 * __longlong_as_double((long long)tb), 1e-300);
   // The shift lies 64 ulps of ||T|| above the value, so that the members of a cluster (a
   // degenerate value spreads over tens of ulps by the rounding of B) are all about as far
   // from it and three solves leave each a like share of the cluster's vectors.  With
@@ -268,31 +249,22 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
   // (U diag(s) V^H off by up to 1e-8 ||B|| for 128 equal values; now 5e-15).  A single
   // value 1e-11 ||T|| or more from the next is resolved to rounding by three solves.
   lam += 64.0 * ptol;
-  auto guard = [&](double p) -> double { return fabs(p) >= ptol ? p : (p < 0.0 ? -ptol : ptol); };
-  // LU with partial pivoting of T - lam I (diagonal -lam, off-diagonals off(j))
-  double d0 = -lam, d1 = N > 1 ? off(0) : 0.0;
+  const unsigned long long pbits = abs_bits(ptol);
+  auto guard = [&](double p) -> double { return abs_bits(p) >= pbits ? p : copysign(ptol, p); };
+  // LU with partial pivoting of T - lam I (diagonal -lam, off-diagonals off[j])
+  double d0 = -lam, d1 = N > 1 ? off[0] : 0.0;
   for (int j = 0; j < N - 1; ++j) {
-    const double sub = off(j);
-    const double nd0 = -lam, nd1 = j + 1 < N - 1 ? off(j + 1) : 0.0;
-    if (fabs(d0) >= fabs(sub)) {  // keep row j as the pivot row
-      const double piv = guard(d0), rp = 1.0 / piv, mult = sub * rp;
-      AT(U0, j) = rp;
-      AT(U1, j) = d1;
-      AT(U2, j) = 0.0;
-      AT(PV, j) = mult;
-      AT(Y, j) = 0.0;  // no swap
-      d0 = nd0 - mult * d1;
-      d1 = nd1;
-    } else {  // row j+1 becomes the pivot row
-      const double mult = d0 / sub;
-      AT(U0, j) = 1.0 / sub;
-      AT(U1, j) = nd0;
-      AT(U2, j) = nd1;
-      AT(PV, j) = mult;
-      AT(Y, j) = 1.0;  // swapped
-      d0 = d1 - mult * nd0;
-      d1 = -mult * nd1;
-    }
+    const double sb = off[j], nd0 = -lam, nd1 = j + 1 < N - 1 ? off[j + 1] : 0.0;
+    const bool keep = abs_bits(d0) >= abs_bits(sb);  // row j stays the pivot row
+    const double rp = 1.0 / (keep ? guard(d0) : sb), mult = (keep ? sb : d0) * rp;
+    const double up = keep ? d1 : nd0;
+    AT(U0, j) = rp;
+    AT(U1, j) = up;
+    AT(U2, j) = keep ? 0.0 : nd1;
+    AT(PV, j) = mult;
+    AT(Y, j) = keep ? 0 : 1;
+    d0 = fma(-mult, up, keep ? nd0 : d1);
+    d1 = keep ? nd1 : -mult * nd1;
   }
   AT(U0, N - 1) = 1.0 / guard(d0);  // U0 holds the reciprocal pivots
   // start vector: row i of the cosine transform with fixed pseudo-random signs on the v's,
@@ -310,54 +282,88 @@ __global__ void k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
     AT(Z, 2 * j) = (double)(x & 1 ? cospif(a) : -cospif(a));
     AT(Z, 2 * j + 1) = 0.0;
   }
-  double scale = 1.0;  // the right-hand side is Z * scale
+  int scale = 0;  // the right-hand side is Z 2^scale
   for (int it = 0; it < 3; ++it) {
     // forward: the row operations (with swaps) applied to the right-hand side
-    double carry = AT(Z, 0) * scale;
-    for (int j = 0; j < N - 1; ++j) {
-      const double next = AT(Z, j + 1) * scale;
-      if (AT(Y, j) == 0.0) {
-        AT(Z, j) = carry;
-        carry = next - AT(PV, j) * carry;
-      } else {
-        AT(Z, j) = next;
-        carry = carry - AT(PV, j) * next;
-      }
+    double carry = times_pow2(AT(Z, 0), scale);
+    for (int j = 0; j < N - 1; j += kAhead) {
+      double z[kAhead], pv[kAhead];
+      int sw[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (j + u < N - 1) {
+          z[u] = AT(Z, j + u + 1);
+          pv[u] = AT(PV, j + u);
+          sw[u] = AT(Y, j + u);
+        }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (j + u < N - 1) {
+          const double next = times_pow2(z[u], scale);
+          AT(Z, j + u) = sw[u] ? next : carry;
+          carry = fma(-pv[u], sw[u] ? next : carry, sw[u] ? carry : next);
+        }
     }
     AT(Z, N - 1) = carry;
     // back substitution with the upper factor (diagonal U0, super-diagonals U1, U2);
     // a partial result that grows past 2^500 is rescaled, with the values already
-    // produced, so that nothing overflows
-    double x1 = 0.0, x2 = 0.0, amax = 0.0;
-    for (int j = N - 1; j >= 0; --j) {
-      double sacc = AT(Z, j);
-      if (j + 1 < N) sacc -= AT(U1, j) * x1;
-      if (j + 2 < N) sacc -= AT(U2, j) * x2;
-      double x = sacc * AT(U0, j);
-      if (fabs(x) > 3.273390607896142e150) {
-        const double r = 3.054936363499605e-151;  // 2^-500
-        for (int q = j + 1; q < N; ++q) AT(Z, q) *= r;
-        x *= r;
-        x1 *= r;
-        x2 *= r;
-        amax *= r;
-        // the remaining right-hand side entries scale with the solution
-        for (int q = 0; q < j; ++q) AT(Z, q) *= r;
-      }
-      AT(Z, j) = x;
-      amax = fmax(amax, fabs(x));
-      x2 = x1;
-      x1 = x;
+    // produced and the right-hand side, so that nothing overflows
+    double x1 = 0.0, x2 = 0.0;
+    int top = 0;  // largest exponent field
+    for (int j = N - 1; j >= 0; j -= kAhead) {
+      double z[kAhead], u0[kAhead], u1[kAhead], u2[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (j - u >= 0) {
+          z[u] = AT(Z, j - u);
+          u0[u] = AT(U0, j - u);
+          u1[u] = j - u + 1 < N ? AT(U1, j - u) : 0.0;
+          u2[u] = j - u + 2 < N ? AT(U2, j - u) : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (j - u >= 0) {
+          double x = fma(-u2[u], x2, fma(-u1[u], x1, z[u])) * u0[u];
+          int f = (__double2hiint(x) >> 20) & 0x7ff;
+          if (f > 1023 + 500) {
+            for (int q = j - u + 1; q < N; ++q) AT(Z, q) = times_pow2(AT(Z, q), -500);
+            for (int q = 0; q < j - u; ++q) AT(Z, q) = times_pow2(AT(Z, q), -500);
+#pragma unroll
+            for (int v = 0; v < kAhead; ++v)
+              if (v > u) z[v] = times_pow2(z[v], -500);
+            x = times_pow2(x, -500);
+            x1 = times_pow2(x1, -500);
+            f -= 500;
+            top -= 500;
+          }
+          AT(Z, j - u) = x;
+          top = max(top, f);
+          x2 = x1;
+          x1 = x;
+        }
     }
-    scale = amax > 0.0 ? 1.0 / amax : 0.0;
+    scale = 1023 - top;
   }
   double nrm = 0.0;
-  for (int j = 0; j < N; ++j) {
-    const double v = AT(Z, j) * scale;
-    nrm = fma(v, v, nrm);
+  for (int j = 0; j < N; j += kAhead) {
+    double z[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) z[u] = j + u < N ? AT(Z, j + u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      z[u] = times_pow2(z[u], scale);
+      nrm = fma(z[u], z[u], nrm);
+    }
   }
-  const double inv = nrm > 0.0 ? scale / sqrt(nrm) : 0.0;
-  for (int j = 0; j < N; ++j) AT(Z, j) *= inv;
+  const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
+  for (int j = 0; j < N; j += kAhead) {
+    double z[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) z[u] = j + u < N ? AT(Z, j + u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (j + u < N) AT(Z, j + u) = times_pow2(z[u], scale) * inv;
+  }
 #undef AT
 }
 
@@ -464,18 +470,22 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
   if (h->profiling) cudaEventRecord(h->ev[5], st);
   ++h->stats.gebrd_launches;
   {
-    const size_t smem = (sizeof(double) + sizeof(float2) + sizeof(float)) * (size_t)(2 * nmax);
-    // team size: multisection while the batch's values (nb x kk at most) leave the
-    // GPU's resident threads idle, plain bisection once they fill them
+    const size_t smem = (sizeof(double) + sizeof(float)) * (size_t)(2 * nmax);
+    // team size: multisection while the batch's values (nb x kk at most) leave warp
+    // schedulers idle, plain bisection once there is a warp for each
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const double values = (double)nb * kk, slots_resident = 2048.0 * std::max(sms, 1);
-    int team = values * 8 <= slots_resident ? 8 : values * 4 <= slots_resident ? 4
-               : values * 2 <= slots_resident ? 2 : 1;
+    const double values = (double)nb * kk, lanes = 4.0 * 32.0 * std::max(sms, 1);
+    int team = 1;
+    while (team < 16 && values * 2 * team <= lanes) team *= 2;
     const TuneParams tp = tune_lookup(h, b.dfp ? 1 : 0, nmax, nb);
     if (tp.team == 1 || tp.team == 2 || tp.team == 4 || tp.team == 8) team = tp.team;
-    auto kern = team == 8 ? k_bd_sigma<8> : team == 4 ? k_bd_sigma<4> : team == 2 ? k_bd_sigma<2> : k_bd_sigma<1>;
+    auto kern = team == 16  ? k_bd_sigma<16>
+                : team == 8 ? k_bd_sigma<8>
+                : team == 4 ? k_bd_sigma<4>
+                : team == 2 ? k_bd_sigma<2>
+                            : k_bd_sigma<1>;
     if ((rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                          "bisection shared memory")))
       return rc;
@@ -484,7 +494,13 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
   TEBD_LAUNCHED(h);
   if (b.phase == 1) return check_cuda(h, cudaGetLastError(), "bidiag launch");
   }  // vectors
-  k_bd_invit<<<dim3(cdiv(kk, 32), nb), 32, 0, st>>>(slots_d, path_d, kk, cap);
+  {
+    const size_t smem = sizeof(double) * (size_t)(2 * nmax);
+    if ((rc = check_cuda(h, cudaFuncSetAttribute(k_bd_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                         "inverse iteration shared memory")))
+      return rc;
+    k_bd_invit<<<dim3(cdiv(kk, 32), nb), 32, smem, st>>>(slots_d, path_d, kk, cap);
+  }
   TEBD_LAUNCHED(h);
   if ((rc = launch_bd_orth(h, b))) return rc;
   if ((rc = launch_bd_apply(h, b))) return rc;
