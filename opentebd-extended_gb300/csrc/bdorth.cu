@@ -65,7 +65,9 @@ __host__ __device__ __forceinline__ int splits(int rows) {  // parts of the earl
 // subtraction's partial sums
 __host__ __device__ __forceinline__ size_t orth_smem(int n, int K, int C) {
   const size_t rows = rows_of(n, C);
-  return sizeof(long long) * kPan * (rows + (size_t)K + splits((int)rows) * rows);
+  // splits(r) r is at most max(r, 512), but not monotone in r: the batch's smaller problems
+  // may need more than its largest
+  return sizeof(long long) * kPan * (rows + (size_t)K + (rows > 32 * kWarps ? rows : 32 * kWarps));
 }
 constexpr int kMostK = 2048;  // coefficients of more vectors stay in global memory
 

@@ -258,8 +258,9 @@ __device__ __forceinline__ void row_sum(Acc &acc, const int4 *base, size_t ldk, 
 // [part][column], the dot products of the panel's V, X with v, and quarters of the
 // panel's correction of the current row, [Y U] rvec.  (The phases' functions are not
 // inlined: each keeps its registers for its own loop.)
-__device__ __forceinline__ int left_parts(int nk, int nz) {  // enough tasks for two rounds, at least 128 k each
-  return max(1, min((2 * kWorkers + nz - 1) / max(1, nz), nk / 128));
+__device__ __forceinline__ int left_parts(int nk, int nz) {  // enough tasks for two rounds, at least 128 k each,
+  const Ctx &x = ctx();                                       // as many as the sums have room for
+  return max(1, min(min((2 * kWorkers + nz - 1) / max(1, nz), nk / 128), (x.zp_at - x.zc_at) / x.ownC));
 }
 __device__ __noinline__ void left_products(int i, bool panel, int warp, int lane) {
   const Ctx &x = ctx();

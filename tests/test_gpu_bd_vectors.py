@@ -51,3 +51,24 @@ def test_clusters(pkg, n, kind, svd_mode):
     want = theta / np.linalg.norm(theta)
     back = (u * l1) @ v
     assert np.linalg.norm(back / np.linalg.norm(back) - want) <= 10 * n * n * 2.2e-16
+
+
+@pytest.mark.parametrize("sizes", [(170, 128, 96, 33), (300, 256, 129, 64), (40, 170, 7, 2), (520, 300, 40, 256)])
+def test_one_batch_of_several_sizes(pkg, sizes):
+    """Three bonds of different Theta in one batch: the launch is sized by the largest."""
+    rng = np.random.default_rng(sum(sizes))
+    chi = max(sizes)
+    gam = [np.asfortranarray(rng.standard_normal((chi, 1, chi)) + 1j * rng.standard_normal((chi, 1, chi)))
+           for _ in range(6)]
+    lam = [np.ones(chi) for _ in range(7)]
+    for q, r in enumerate(sizes):  # Theta of bond 2 q + 1 is sizes[q] x sizes[q + 1]
+        lam[2 * q] = np.where(np.arange(chi) < r, np.exp(-2.0 * np.arange(chi) / chi), 0.0)
+        lam[2 * q] /= np.linalg.norm(lam[2 * q])
+    with pkg.Chain(6, 1, chi, svd_mode=3) as c:
+        c.set_state(gam, lam)
+        c.apply_bonds([1, 3, 5], [np.eye(1, dtype=complex)] * 3)
+        for b in range(3):
+            l0, l2, l1 = lam[2 * b], lam[2 * b + 2], c.get_lambda(2 * b + 2)
+            want = (l0[:, None] * gam[2 * b][:, 0, :]) @ (gam[2 * b + 1][:, 0, :] * l2)
+            back = (l0[:, None] * c.get_gamma(2 * b + 1)[:, 0, :] * l1) @ (c.get_gamma(2 * b + 2)[:, 0, :] * l2)
+            assert np.linalg.norm(back / np.linalg.norm(back) - want / np.linalg.norm(want)) <= 1e-12
