@@ -596,36 +596,42 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
       // bidiagonalising from 64 columns).  Mixing the routes in one batch would
       // serialise them (the QR batch, then the bidiagonal one).  A batch that took
       // the randomized route holds saturated bonds.
-      bool full_batch = nrs > 0;
+      //
+      // Below 64 columns the same holds for a saturated bond (32 columns, rank 32: 5.1 ms by
+      // the QR route, 1.1 by the bidiagonal one), and a batch's other small bonds ride
+      // along, as long as a bond's values span no more than kBidiagSpan: the Jacobi
+      // sweeps resolve the vectors of the smallest values to their own size, the
+      // bidiagonal route only to the largest one's.  These bonds still report all their
+      // values (kPathAll).
+      const int mode = h->opts.svd_mode;
+      const bool choose = mode != TEBD_SVD_BIDIAG && mode != TEBD_SVD_QRJ;
+      bool full_batch = nrs > 0, any_full = full_batch;
       for (int s = 0; s < nb; ++s) {
         const int mn = std::min(cps[s].m, cps[s].n);
-        if (mn >= kBidiagMinDim && std::max(cps[s].m, cps[s].n) <= kBidiagMaxDim &&
-            (cps[s].r1 >= h->chi || mn > kQrjMaxDim))
-          full_batch = true;
+        if (std::max(cps[s].m, cps[s].n) > kBidiagMaxDim) continue;
+        const bool full = cps[s].r1 >= h->chi;
+        if (mn >= kBidiagMinDim && (full || mn > kQrjMaxDim)) full_batch = true;
+        if (full && mn >= kBidiagSmallDim && cps[s].span >= kBidiagSpan) any_full = true;
       }
+      any_full |= full_batch;
       for (int s = 0; s < nb; ++s) {
-        if (nrs && h->path_h[s] != kPathQRJ) {  // randomized route, or its fallback to the full SVD
-          if (h->path_h[s] != kPathRsvd) {
-            const int mn = std::min(cps[s].m, cps[s].n), mx = std::max(cps[s].m, cps[s].n);
-            ++nbd;
-            nbd_max = std::max(nbd_max, mx);
-            h->stats.gebrd_flops += 16.0 * mx * (double)mn * mn - 16.0 / 3.0 * (double)mn * mn * mn;
-          }
-          continue;
-        }
         const int mn = std::min(cps[s].m, cps[s].n), mx = std::max(cps[s].m, cps[s].n);
-        const bool bd = mx > kBidiagMaxDim                   ? false
-                        : h->opts.svd_mode == TEBD_SVD_BIDIAG ? mn >= 2
-                        : h->opts.svd_mode == TEBD_SVD_QRJ    ? false
-                                                              : mn >= kBidiagMinDim && full_batch;
-        h->path_h[s] = !bd ? kPathQRJ : (cps[s].m >= cps[s].n ? kPathBidiag : kPathBidiagT);
-        if (bd) {
+        const bool done = nrs && h->path_h[s] == kPathRsvd;
+        if (done) continue;
+        const bool back = nrs && h->path_h[s] != kPathQRJ;  // the randomized route's fallback to the full SVD
+        const bool bd = back || (mx <= kBidiagMaxDim && mn >= 2 &&
+                                 (mode == TEBD_SVD_BIDIAG || (choose && mn >= kBidiagMinDim && full_batch)));
+        const bool small = !bd && choose && any_full && mx <= kBidiagMaxDim && mn >= 2 && cps[s].span >= kBidiagSpan;
+        h->path_h[s] = !(bd || small) ? kPathQRJ : cps[s].m >= cps[s].n ? kPathBidiag : kPathBidiagT;
+        if (small) h->path_h[s] |= kPathAll;
+        h->stats.bidiag_updates += bd;
+        if (bd || small) {
           ++nbd;
           nbd_max = std::max(nbd_max, mx);
           h->stats.gebrd_flops += 16.0 * mx * (double)mn * mn - 16.0 / 3.0 * (double)mn * mn * mn;
         }
+        if (small) h->stats.rank_sum += mn;
       }
-      h->stats.bidiag_updates += nbd;
       CK(cudaMemcpyAsync(h->path_d, h->path_h.data(), sizeof(int) * nb, cudaMemcpyHostToDevice,
                          h->stream),
          "upload SVD routes");
