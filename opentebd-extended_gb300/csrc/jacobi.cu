@@ -36,71 +36,83 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-template <typename T>
-struct JacobiBig;
-template <>
-struct JacobiBig<double> {
-  static __device__ __forceinline__ double v() { return 1e150; }
-};
-template <>
-struct JacobiBig<float> {
-  static __device__ __forceinline__ float v() { return 1e18f; }
-};
+// x 2^-e as a float, rounded towards zero; |x| 2^-e < 2^127; 0 below 2^-126
+__device__ __forceinline__ float scaled_float(double x, int e) {
+  const int hi = __double2hiint(x), f = ((hi >> 20) & 0x7ff) - 896 - e;
+  if (f <= 0) return 0.0f;
+  return __int_as_float((hi & 0x80000000) | (f << 23) | ((hi & 0xfffff) << 3) |
+                        (int)((unsigned)__double2loint(x) >> 29));
+}
+__device__ __forceinline__ double as_double(float x) {  // by integer instructions; 0 below 2^-126
+  const int b = __float_as_int(x), f = (b >> 23) & 0xff;
+  return f == 0 ? 0.0 : __hiloint2double((b & 0x80000000) | ((f + 896) << 20) | ((b & 0x7fffff) >> 3), b << 29);
+}
+// four sums over the lanes at once: of n values a lane keeps half at each exchange (6
+// additions instead of 20)
+__device__ __forceinline__ void warp_sum4(double &a, double &b, double &c, double &d, int lane) {
+  const bool u16 = lane & 16, u8 = lane & 8;
+  double x = (u16 ? c : a) + __shfl_xor_sync(0xffffffffu, u16 ? a : c, 16);
+  double y = (u16 ? d : b) + __shfl_xor_sync(0xffffffffu, u16 ? b : d, 16);
+  x = (u8 ? y : x) + __shfl_xor_sync(0xffffffffu, u8 ? x : y, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  a = __shfl_sync(0xffffffffu, x, 0);
+  b = __shfl_sync(0xffffffffu, x, 8);
+  c = __shfl_sync(0xffffffffu, x, 16);
+  d = __shfl_sync(0xffffffffu, x, 24);
+}
 
-// Rotate columns (A, B) of X and (VA, VB) of V by the unitary 2x2 that makes
-// them orthogonal.  Gram [[al, g e^{i phi}], [g e^{-i phi}, be]]:
-//   zeta = (be - al) / (2 g),  t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)),
-//   c = 1/sqrt(1+t^2), s = c t,
-//   a' = c a - s e^{-i phi} b,   b' = s e^{i phi} a + c b.
-template <typename T>
-__device__ __forceinline__ bool jacobi_pair(typename cplx<T>::type *__restrict__ A,
-                                            typename cplx<T>::type *__restrict__ B,
-                                            typename cplx<T>::type *__restrict__ VA,
-                                            typename cplx<T>::type *__restrict__ VB, int m,
-                                            int nv, int lane, T tol, double floor) {
-  using C2 = typename cplx<T>::type;
-  T al = 0, be = 0, gr = 0, gi = 0;
+// Rotate columns (A, B) of X and (VA, VB) of V by a unitary 2x2 that makes them
+// orthogonal.  Gram [[al, g], [conj g, be]], g = a^H b:
+//   zeta = (be - al) / (2 |g|),  t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)),
+//   tau = t g / |g|,  c = 1/sqrt(1+|tau|^2), s = c tau,
+//   a' = c a - conj(s) b,   b' = s a + c b.
+// The rotation is unitary for any tau, so tau is computed in FP32 (the pair keeps
+// 1e-7 of its product, which the next sweep takes) and only c and s in FP64, from that
+// tau: an FP64 square root or quotient takes its scheduler 400 to 700 cycles, and there
+// were seven of them per pair.  Measured on whole calls that are half Jacobi sweeps: 12
+// steps of a 32-site spin chain, rank 10 of 20, 35.8 -> 28.0 ms; single bonds of a
+// 13-site ring, chi = 45, 81.9 -> 62.0 ms.
+__device__ __forceinline__ bool jacobi_pair(double2 *__restrict__ A, double2 *__restrict__ B, double2 *__restrict__ VA,
+                                            double2 *__restrict__ VB, int m, int nv, int lane, double tol,
+                                            double floor) {
+  double al = 0, be = 0, gr = 0, gi = 0;
   for (int r = lane; r < m; r += 32) {
-    const C2 a = __ldcg(A + r), b = __ldcg(B + r);
+    const double2 a = __ldcg(A + r), b = __ldcg(B + r);
     al = fma(a.x, a.x, fma(a.y, a.y, al));
     be = fma(b.x, b.x, fma(b.y, b.y, be));
     gr = fma(a.x, b.x, fma(a.y, b.y, gr));
     gi = fma(a.x, b.y, fma(-a.y, b.x, gi));
   }
-  al = warp_sum(al);
-  be = warp_sum(be);
-  gr = warp_sum(gr);
-  gi = warp_sum(gi);
-  const T g = sqrt(gr * gr + gi * gi);
-  if (!(g > tol * sqrt(al) * sqrt(be)) || (double)al <= floor || (double)be <= floor) return false;
-  const T zeta = (be - al) / (T(2) * g);
-  T t;
-  if (fabs(zeta) > JacobiBig<T>::v())
-    t = T(0.5) / zeta;
-  else
-    t = copysign(T(1), zeta) / (fabs(zeta) + sqrt(T(1) + zeta * zeta));
-  const T c = T(1) / sqrt(T(1) + t * t);
-  const T s = c * t;
-  const T sr = s * (gr / g), si = s * (gi / g);
+  warp_sum4(al, be, gr, gi, lane);
+  const double larger = al > be ? al : be;
+  if (!(al > floor) || !(be > floor) || !(larger < INFINITY)) return false;
+  const int e = ((__double2hiint(larger) >> 20) & 0x7ff) - 1023;
+  const float fr = scaled_float(gr, e), fi = scaled_float(gi, e), big = fmaxf(fabsf(fr), fabsf(fi));
+  if (big == 0.0f) return false;
+  const float ratio = fminf(fabsf(fr), fabsf(fi)) / big, g = big * sqrtf(1.0f + ratio * ratio);
+  auto root = [&](double x) -> float {  // sqrt(x 2^-e), also where x 2^-e is out of FP32's range
+    int ex = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
+    ex -= (ex - e) & 1;
+    return sqrtf(scaled_float(x, ex)) * __int_as_float(max(0, (ex - e) / 2 + 127) << 23);
+  };
+  if (!(g > (float)tol * root(al) * root(be))) return false;
+  const float zeta = scaled_float(be - al, e + 1) / g;
+  const float t = fabsf(zeta) > 1e15f ? 0.5f / zeta : copysignf(1.0f, zeta) / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
+  const double tr = as_double(t * (fr / g)), ti = as_double(t * (fi / g));
+  // c = 1 / sqrt(q), q in [1, 2]: the FP32 value, then one step of third order
+  const double q = fma(tr, tr, fma(ti, ti, 1.0)), y = as_double(rsqrtf(scaled_float(q, 0)));
+  const double res = fma(-q * y, y, 1.0), c = fma(y * res, fma(0.375, res, 0.5), y);
+  const double sr = c * tr, si = c * ti;
   for (int r = lane; r < m; r += 32) {
-    const C2 a = __ldcg(A + r), b = __ldcg(B + r);
-    C2 na, nb;
-    na.x = fma(c, a.x, fma(-sr, b.x, -si * b.y));
-    na.y = fma(c, a.y, fma(-sr, b.y, si * b.x));
-    nb.x = fma(sr, a.x, fma(-si, a.y, c * b.x));
-    nb.y = fma(sr, a.y, fma(si, a.x, c * b.y));
-    A[r] = na;
-    B[r] = nb;
+    const double2 a = __ldcg(A + r), b = __ldcg(B + r);
+    A[r] = make_double2(fma(c, a.x, fma(-sr, b.x, -si * b.y)), fma(c, a.y, fma(-sr, b.y, si * b.x)));
+    B[r] = make_double2(fma(sr, a.x, fma(-si, a.y, c * b.x)), fma(sr, a.y, fma(si, a.x, c * b.y)));
   }
   for (int r = lane; r < nv; r += 32) {
-    const C2 a = __ldcg(VA + r), b = __ldcg(VB + r);
-    C2 na, nb;
-    na.x = fma(c, a.x, fma(-sr, b.x, -si * b.y));
-    na.y = fma(c, a.y, fma(-sr, b.y, si * b.x));
-    nb.x = fma(sr, a.x, fma(-si, a.y, c * b.x));
-    nb.y = fma(sr, a.y, fma(si, a.x, c * b.y));
-    VA[r] = na;
-    VB[r] = nb;
+    const double2 a = __ldcg(VA + r), b = __ldcg(VB + r);
+    VA[r] = make_double2(fma(c, a.x, fma(-sr, b.x, -si * b.y)), fma(c, a.y, fma(-sr, b.y, si * b.x)));
+    VB[r] = make_double2(fma(sr, a.x, fma(-si, a.y, c * b.x)), fma(sr, a.y, fma(si, a.x, c * b.y)));
   }
   return true;
 }
@@ -136,7 +148,7 @@ __global__ void __launch_bounds__(kJacobiWarps * 32)
   }
   bool rotated = false;
   if (i >= 0 && j < P.n)  // j == P.n is the phantom column of an odd n
-    rotated = jacobi_pair<T>(P.X + (size_t)P.ldx * i, P.X + (size_t)P.ldx * j,
+    rotated = jacobi_pair(P.X + (size_t)P.ldx * i, P.X + (size_t)P.ldx * j,
                              P.V + (size_t)P.ldv * i, P.V + (size_t)P.ldv * j, P.m, P.n, lane, tol,
                              P.floor);
   const int c = __syncthreads_count(rotated && lane == 0);
@@ -205,6 +217,7 @@ __global__ void __launch_bounds__(kPW * 32)
   const int C = (int)cluster.num_blocks();
   const JacobiProblem<T> P = probs[p];
   const int npad = P.n + (P.n & 1), R = npad - 1, half = npad / 2;
+  if (!(tol > 0)) tol = (P.n > 16 ? P.n : 16) * 2.220446049250313e-16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gw = crank * kPW + warp, nw = C * kPW;
   int sw = 0, converged = (P.n < 2);
@@ -228,11 +241,14 @@ __global__ void __launch_bounds__(kPW * 32)
           j = t;
         }
         if (j < P.n &&
-            jacobi_pair<T>(P.X + (size_t)P.ldx * i, P.X + (size_t)P.ldx * j, P.V + (size_t)P.ldv * i,
+            jacobi_pair(P.X + (size_t)P.ldx * i, P.X + (size_t)P.ldx * j, P.V + (size_t)P.ldv * i,
                            P.V + (size_t)P.ldv * j, P.m, P.n, lane, tol, P.floor))
           local += (lane == 0);
       }
-      cluster.sync();
+      if (C > 1)
+        cluster.sync();
+      else
+        __syncthreads();
       // the other parity's counter was last read before this sweep's first barrier
       if (r == 0 && crank == 0 && threadIdx.x == 0) rotc[2 * p + ((sw + 1) & 1)] = 0;
     }
@@ -258,10 +274,13 @@ __global__ void __launch_bounds__(kPW * 32)
   }
 }
 
-// Cluster size: enough warps for the pairs of one round, at most 8 CTAs.
-static int persistent_cluster_size(int nmax) {
-  const int half = (nmax + (nmax & 1)) / 2;
-  int c = (half + kPW - 1) / kPW;
+// Cluster size: the FP64 pipes bound a round, so the pairs go to as many SMs as the
+// batch leaves for a problem, down to four pairs per CTA; at most 8 CTAs.
+static int persistent_cluster_size(int nmax, int nprob) {
+  const int half = (nmax + 1) / 2;
+  const int need = (half + kPW - 1) / kPW, most = (half + 3) / 4, share = 152 / (nprob > 0 ? nprob : 1);
+  int c = most < share ? most : share;
+  if (c < need) c = need;
   return c < 1 ? 1 : (c > 8 ? 8 : c);
 }
 
@@ -271,7 +290,7 @@ static int jacobi_persistent(tebd_handle *h, const JacobiProblem<T> *probs_d, in
   cudaStream_t st = h->stream;
   int rc = check_cuda(h, cudaMemsetAsync(h->js.rot, 0, sizeof(int) * 2 * nprob, st), "reset counters");
   if (rc) return rc;
-  const int C = persistent_cluster_size(nmax);
+  const int C = persistent_cluster_size(nmax, nprob);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, nprob, 1);
   cfg.blockDim = dim3(kPW * 32, 1, 1);
@@ -307,42 +326,6 @@ static int jacobi_persistent(tebd_handle *h, const JacobiProblem<T> *probs_d, in
     if (!dn[p])
       return set_error(h, TEBD_ERR_SVD_NOCONV, "Jacobi SVD did not converge within the sweep cap");
   return TEBD_OK;
-}
-
-template <typename T>
-static int jacobi_sweeps(tebd_handle *h, const JacobiProblem<T> *probs_d, int nprob, int nmax,
-                         T tol, int max_sweeps, int *sweeps_used) {
-  cudaStream_t st = h->stream;
-  const int npad = nmax + (nmax & 1);
-  const int rounds = npad - 1;
-  const unsigned gx = (unsigned)((npad / 2 + kJacobiWarps - 1) / kJacobiWarps);
-  int *pending_h = reinterpret_cast<int *>(h->pinned);
-  for (int sw = 0; sw < max_sweeps; ++sw) {
-    if (h->profiling) cudaEventRecord(h->ev[0], st);
-    for (int r = 0; r < rounds; ++r) {
-      k_jacobi_round<T><<<dim3(gx, nprob), kJacobiWarps * 32, 0, st>>>(probs_d, h->js.done,
-                                                                       h->js.rot, r, tol);
-      TEBD_LAUNCHED(h);
-    }
-    h->stats.jacobi_launches += rounds;
-    if (h->profiling) cudaEventRecord(h->ev[1], st);
-    k_jacobi_sweep_end<T><<<1, 32, 0, st>>>(probs_d, nprob, h->js.rot, h->js.done, h->js.sweeps,
-                                             h->js.pending, h->js.counters);
-    TEBD_LAUNCHED(h);
-    int rc = check_cuda(h, cudaMemcpyAsync(pending_h, h->js.pending, sizeof(int),
-                                           cudaMemcpyDeviceToHost, st),
-                        "jacobi pending copy");
-    if (rc) return rc;
-    rc = check_cuda(h, cudaStreamSynchronize(st), "jacobi sweep");
-    if (rc) return rc;
-    if (h->profiling) {
-      float ms = 0.f;
-      if (cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]) == cudaSuccess) h->stats.jacobi_ms += ms;
-    }
-    *sweeps_used = sw + 1;
-    if (*pending_h == 0) return TEBD_OK;
-  }
-  return set_error(h, TEBD_ERR_SVD_NOCONV, "Jacobi SVD did not converge within the sweep cap");
 }
 
 // Dense batch: nmax = largest compacted column count of the batch (the rounds
