@@ -38,9 +38,9 @@ int check_cuda(tebd_handle *h, cudaError_t e, const char *what) {
 
 // pinned staging layout
 constexpr size_t kPinFlags = 0;        // 64 bytes: pending count, status flags
-constexpr size_t kPinTrunc = 64;       // nslots doubles
+constexpr size_t kPinTrunc = 64;       // nslots doubles, then nslots compaction records
 static size_t pin_gates_off(const tebd_handle *h) {
-  return (kPinTrunc + sizeof(double) * h->nslots + 255) & ~(size_t)255;
+  return (kPinTrunc + (sizeof(double) + sizeof(Compact)) * h->nslots + 255) & ~(size_t)255;
 }
 static size_t pin_links_off(const tebd_handle *h) {
   return pin_gates_off(h) + sizeof(double2) * (size_t)h->nslots * h->d * h->d * h->d * h->d;
@@ -525,7 +525,7 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
      "upload links");
   CK(cudaMemsetAsync(h->status_d, 0, sizeof(int) * 4, h->stream), "reset status");
   if (h->profiling) cudaEventRecord(h->ev[2], h->stream);
-  int rc;
+  int rc, nqr = 0;  // nqr: bonds on the QR route
   if (h->mode == TEBD_MODE_DENSE) {
     if ((rc = launch_dense_prepare(h, nb, true))) return rc;
     int nmax = 0;
@@ -635,9 +635,8 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
       CK(cudaMemcpyAsync(h->path_d, h->path_h.data(), sizeof(int) * nb, cudaMemcpyHostToDevice,
                          h->stream),
          "upload SVD routes");
-      int nqr = 0;
       for (int s = 0; s < nb; ++s) nqr += h->path_h[s] == kPathQRJ;
-      if (nqr > 0 && (rc = run_qrj(h, nb, nmax))) return rc;
+      if (nqr > 0 && (rc = run_qrj(h, nb))) return rc;
       if (nbd > 0 && (rc = run_bidiag(h, nb, nbd_max))) return rc;
     }
     if (h->unnormalized && (rc = launch_unit_norm(h, nb))) return rc;
@@ -654,8 +653,12 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
   f_pin[8] = 0;
   if (h->tc_err)  // a tensor-core product of the batch whose pipeline wait expired
     CK(cudaMemcpyAsync(f_pin + 8, h->tc_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "read tensor-core flag");
+  Compact *c_pin = (Compact *)(pin + kPinTrunc + sizeof(double) * h->nslots);
+  if (nqr > 0)
+    CK(cudaMemcpyAsync(c_pin, h->cp_d, sizeof(Compact) * nb, cudaMemcpyDeviceToHost, h->stream), "read ranks");
   if (h->profiling) cudaEventRecord(h->ev[3], h->stream);
   CK(cudaStreamSynchronize(h->stream), "bond batch");
+  if (nqr > 0) qrj_count(h, nb, c_pin);
   for (int s = 0; s < nb; ++s) truncerr[s] = t_pin[s];
   if (h->profiling) {
     float ms = 0.f;

@@ -241,7 +241,8 @@ int launch_unit_norm(tebd_handle *h, int nb);
 int run_jacobi_problems(tebd_handle *h, const JacobiProblem<double> *probs_d, int nprob, int nmax);
 int jacobi_persistent_double(tebd_handle *h, const JacobiProblem<double> *probs_d, int nprob,
                              int nmax, double tol, int max_sweeps);
-int run_qrj(tebd_handle *h, int nb, int nmax);
+int run_qrj(tebd_handle *h, int nb);
+void qrj_count(tebd_handle *h, int nb, const Compact *cp);  // ranks and flops of a finished batch
 int run_bidiag(tebd_handle *h, int nb, int nmax);
 // A batch of bidiagonal problems described by slot entries (X, V, aux, tau, taup,
 // bdws, cp) and routes; kk triplets per problem (min(kk, N) computed).
