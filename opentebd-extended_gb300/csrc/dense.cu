@@ -37,9 +37,16 @@ __global__ void __launch_bounds__(96) k_compact(const double *__restrict__ lam, 
   int *idx = w == 0 ? slots[s].idx0 : (w == 1 ? slots[s].idx1 : slots[s].idx2);
   int *inv = w == 0 ? slots[s].inv0 : (w == 2 ? slots[s].inv2 : nullptr);
   int count = 0;
+  long long lo = 0x7fffffffffffffffll, hi = 0;  // bits of the smallest and the largest |value|
   for (int base = 0; base < chi; base += 32) {
     const int a = base + lane;
-    const bool keep = a < chi && l[a] != 0.0;
+    const double v = a < chi ? l[a] : 0.0;
+    const bool keep = v != 0.0;
+    if (keep) {
+      const long long b = __double_as_longlong(v) & 0x7fffffffffffffffll;
+      lo = min(lo, b);
+      hi = max(hi, b);
+    }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     const int pos = count + __popc(m & ((1u << lane) - 1u));
     if (keep) idx[pos] = a;
@@ -47,6 +54,15 @@ __global__ void __launch_bounds__(96) k_compact(const double *__restrict__ lam, 
     count += __popc(m);
   }
   __shared__ int cnt[3];
+  __shared__ double ends[2];
+  if (w == 1) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane < 2) ends[lane] = __longlong_as_double(lane ? hi : lo);
+  }
   if (lane == 0) cnt[w] = count;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -58,15 +74,7 @@ __global__ void __launch_bounds__(96) k_compact(const double *__restrict__ lam, 
     c.n = d * cnt[2];
     c.k = c.n;
     c.bad = 0;
-    const double *l1 = lam + (size_t)link * chi;
-    double lo = 0.0, hi = 0.0;
-    for (int a = 0; a < chi; ++a)
-      if (l1[a] != 0.0) {
-        const double v = fabs(l1[a]);
-        lo = (lo == 0.0 || v < lo) ? v : lo;
-        hi = v > hi ? v : hi;
-      }
-    c.span = hi > 0.0 ? (float)(lo / hi) : 0.f;
+    c.span = ends[1] > 0.0 ? (float)(ends[0] / ends[1]) : 0.f;
     *slots[s].cp = c;
     jp[s].m = c.m;
     jp[s].n = c.n;
@@ -80,14 +88,18 @@ __global__ void __launch_bounds__(96) k_compact(const double *__restrict__ lam, 
 // A[r', g'] = l0[a] G1[a + chi*i + chi*d*g]   r' = i*r0 + a', a = idx0[a'], g = idx1[g']
 // B[g', c'] = l1[g] G2[g + chi*l + chi*d*b] l2[b]   c' = l + d*b', b = idx2[b']
 // C[r', c'] is stored at X[r' + m*(l*r2 + b')].
-// Tile 64x64 outputs, k-step 8, 256 threads, 4x4 complex outputs per thread.
+// A CTA of 256 threads makes a tile of 16 kQ x 16 kQ outputs, kQ x kQ per thread.  The FP64
+// pipe bounds it, so that the tile must not be larger than a small Theta (a 20 x 20 one
+// of rank 10 took one CTA of 64 x 64 63 us); a larger tile reads less.  The host picks
+// kQ by chi d: 1 up to 128, 2 up to 1024, 4 beyond.  Measured: 36 batches of 16
+// such bonds 63 -> 13 us each, 24 of 32 bonds with a 160 x 160 Theta of rank 36 230 -> 158.
 // ---------------------------------------------------------------------------
-constexpr int TT_M = 64, TT_N = 64, TT_K = 8;
-
+template <int kQ>
 __global__ void __launch_bounds__(256) k_theta_form(const double2 *__restrict__ gam,
                                                     const double *__restrict__ lam,
                                                     const int *__restrict__ links, Slot *slots,
                                                     int chi, int d) {
+  constexpr int TT_M = 16 * kQ, TT_N = 16 * kQ, TT_K = kQ == 1 ? 16 : 8;
   const int s = blockIdx.z;
   const Compact cp = *slots[s].cp;
   const int r0b = blockIdx.x * TT_M, c0b = blockIdx.y * TT_N;
@@ -107,11 +119,11 @@ __global__ void __launch_bounds__(256) k_theta_form(const double2 *__restrict__ 
   __shared__ double2 Bs[TT_K][TT_N + 1];
   const int tid = threadIdx.x;
   const int tr = tid % 16, tc = tid / 16;
-  double2 acc[4][4];
+  double2 acc[kQ][kQ];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < kQ; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = make_double2(0.0, 0.0);
+    for (int b = 0; b < kQ; ++b) acc[a][b] = make_double2(0.0, 0.0);
 
   for (int k0 = 0; k0 < r1; k0 += TT_K) {
     for (int e = tid; e < TT_M * TT_K; e += 256) {
@@ -137,16 +149,16 @@ __global__ void __launch_bounds__(256) k_theta_form(const double2 *__restrict__ 
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < TT_K; ++kk) {
-      double2 a[4], b[4];
+      double2 a[kQ], b[kQ];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < kQ; ++q) {
         a[q] = As[kk][tr + 16 * q];
         b[q] = Bs[kk][tc + 16 * q];
       }
 #pragma unroll
-      for (int p = 0; p < 4; ++p)
+      for (int p = 0; p < kQ; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < kQ; ++q) {
           acc[p][q].x = fma(a[p].x, b[q].x, acc[p][q].x);
           acc[p][q].x = fma(-a[p].y, b[q].y, acc[p][q].x);
           acc[p][q].y = fma(a[p].x, b[q].y, acc[p][q].y);
@@ -156,11 +168,11 @@ __global__ void __launch_bounds__(256) k_theta_form(const double2 *__restrict__ 
     __syncthreads();
   }
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
+  for (int p = 0; p < kQ; ++p) {
     const int r = r0b + tr + 16 * p;
     if (r >= m) continue;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kQ; ++q) {
       const int c = c0b + tc + 16 * q;
       if (c >= n) continue;
       const int lphys = c % d, bp = c / d;
@@ -168,6 +180,20 @@ __global__ void __launch_bounds__(256) k_theta_form(const double2 *__restrict__ 
     }
   }
 }
+
+static void launch_theta_form(cudaStream_t st, const double2 *gam, const double *lam, const int *links, Slot *slots,
+                              int chi, int d, int nb) {
+  const unsigned n = (unsigned)(chi * d);
+  auto grid = [&](unsigned tile) { return dim3((n + tile - 1) / tile, (n + tile - 1) / tile, nb); };
+  if (n <= 128)
+    k_theta_form<1><<<grid(16), 256, 0, st>>>(gam, lam, links, slots, chi, d);
+  else if (n <= 1024)
+    k_theta_form<2><<<grid(32), 256, 0, st>>>(gam, lam, links, slots, chi, d);
+  else
+    k_theta_form<4><<<grid(64), 256, 0, st>>>(gam, lam, links, slots, chi, d);
+}
+
+constexpr int TT_M = 64, TT_N = 64, TT_K = 8;
 
 // Precision form (TEBD_SVD_DF): the same contraction accumulated in double-float
 // on the FP32 pipe, tiles staged as double-float, the result stored in FP64.
@@ -431,7 +457,8 @@ __global__ void __launch_bounds__(1024) k_sigma_sort(Slot *slots, const double *
   }
 }
 
-// FormLambda1 (:347-379): sequential in the reference's order, one thread per slot.
+// FormLambda1 (:347-379): sequential in the reference's order, one warp per slot; the
+// values come through shared memory, so that the sum waits for no load.
 // Kept-rank form (rank_bound > 0, no reference counterpart): keep the fewest
 // leading values whose discarded weight -- the weight beyond chi, 1 - sum of the
 // chi values, plus the dropped kept values summed from the smallest up -- stays
@@ -439,9 +466,11 @@ __global__ void __launch_bounds__(1024) k_sigma_sort(Slot *slots, const double *
 // neighbouring updates compact those Schmidt indices away.
 __global__ void k_lambda(Slot *slots, const int *links, double *lam, double *truncerr, int chi,
                          int nb, double rank_bound, const int *status) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ double S[];  // chi
+  const int s = blockIdx.x, lane = threadIdx.x;
   if (s >= nb || (status[0] & 1)) return;  // non-finite batch: the chain is left as it was
-  const double *S = slots[s].S;
+  for (int a = lane; a < chi; a += 32) S[a] = slots[s].S[a];
+  __syncwarp();
   int keep = chi;
   if (rank_bound > 0.0) {
     double all = 0.0;
@@ -459,10 +488,10 @@ __global__ void k_lambda(Slot *slots, const int *links, double *lam, double *tru
   double norm = 0.0;
   for (int a = 0; a < keep; ++a)
     if (fabs(S[a]) > kGuardDense) norm = norm + S[a] * S[a];
-  truncerr[s] = fabs(1.0 - norm);
+  if (lane == 0) truncerr[s] = fabs(1.0 - norm);
   double *l1 = lam + (size_t)links[s] * chi;
   const double rs = sqrt(norm);
-  for (int a = 0; a < chi; ++a) l1[a] = (a < keep && fabs(S[a]) > kGuardDense) ? S[a] / rs : 0.0;
+  for (int a = lane; a < chi; a += 32) l1[a] = (a < keep && fabs(S[a]) > kGuardDense) ? S[a] / rs : 0.0;
 }
 
 // Keep the last spectrum and sweep count of every link for tebd_get_singular_values.
@@ -568,8 +597,7 @@ int launch_dense_prepare(tebd_handle *h, int nb, bool gate) {
     k_theta_form_df<<<dim3(cdiv(n, TT_M), cdiv(n, TT_N), nb), 256, 0, st>>>(h->gam, h->lam, h->links_d,
                                                                             h->slots_d, chi, d);
   else
-    k_theta_form<<<dim3(cdiv(n, TT_M), cdiv(n, TT_N), nb), 256, 0, st>>>(h->gam, h->lam, h->links_d,
-                                                                         h->slots_d, chi, d);
+    launch_theta_form(st, h->gam, h->lam, h->links_d, h->slots_d, chi, d, nb);
   TEBD_LAUNCHED(h);
   const bool gdf = h->opts.svd_mode == TEBD_SVD_DF || h->opts.svd_mode == TEBD_SVD_RSVD;
   int rc = gate ? check_cuda(h, set_gate_smem(d, gdf), "gate shared memory") : TEBD_OK;
@@ -614,7 +642,7 @@ int launch_dense_finish(tebd_handle *h, int nb) {
   cudaStream_t st = h->stream;
   k_sigma_sort<<<nb, 1024, sizeof(double) * n, st>>>(h->slots_d, h->nrm, n, h->status_d, h->path_d);
   TEBD_LAUNCHED(h);
-  k_lambda<<<cdiv(nb, 64), 64, 0, st>>>(h->slots_d, h->links_d, h->lam, h->truncerr_d, chi, nb,
+  k_lambda<<<nb, 32, sizeof(double) * chi, st>>>(h->slots_d, h->links_d, h->lam, h->truncerr_d, chi, nb,
                                         h->unnormalized ? 0.0 : h->rank_bound, h->status_d);
   TEBD_LAUNCHED(h);
   k_store_spectrum<<<nb, 256, 0, st>>>(h->slots_d, h->links_d, h->js.sweeps, h->sig_link_d,
@@ -673,8 +701,7 @@ cudaError_t raw_dense_prepare(cudaStream_t st, double2 *gam, const double *lam, 
                               int *status, int chi, int d) {
   const int n = chi * d;
   k_compact<<<1, 96, 0, st>>>(lam, links_d, slots_d, jp, chi, d);
-  k_theta_form<<<dim3(cdiv(n, TT_M), cdiv(n, TT_N), 1), 256, 0, st>>>(gam, lam, links_d, slots_d,
-                                                                      chi, d);
+  launch_theta_form(st, gam, lam, links_d, slots_d, chi, d, 1);
   cudaError_t e = set_gate_smem(d);
   if (e != cudaSuccess) return e;
   k_gate_apply<false><<<dim3(cdiv((size_t)chi * chi, kGatePairs), 1), 128, gate_smem_bytes(d), st>>>(
@@ -693,7 +720,7 @@ cudaError_t raw_dense_finish(cudaStream_t st, double2 *gam, double *lam, const i
                              int d) {
   const int n = chi * d;
   k_sigma_sort<<<1, 1024, sizeof(double) * n, st>>>(slots_d, nrm, n, status, nullptr);
-  k_lambda<<<1, 32, 0, st>>>(slots_d, links_d, lam, truncerr, chi, 1, 0.0, status);
+  k_lambda<<<1, 32, sizeof(double) * chi, st>>>(slots_d, links_d, lam, truncerr, chi, 1, 0.0, status);
   k_restore_gamma1<<<dim3(cdiv((size_t)n * chi, 256), 1), 256, 0, st>>>(gam, lam, links_d, slots_d,
                                                                        nrm, chi, d, status);
   k_restore_gamma2<<<dim3(cdiv(chi, 32), cdiv(n, 32), 1), 256, 0, st>>>(gam, lam, links_d, slots_d,
