@@ -76,13 +76,37 @@ __device__ __forceinline__ void warp_sum4(double &a, double &b, double &c, doubl
 __device__ __forceinline__ bool jacobi_pair(double2 *__restrict__ A, double2 *__restrict__ B, double2 *__restrict__ VA,
                                             double2 *__restrict__ VB, int m, int nv, int lane, double tol,
                                             double floor) {
+  // up to 128 rows of X and V together stay in registers between the products and the
+  // rotation (lanes over the rows of X, then those of V): one trip to L2 instead of three,
+  // and one pass where X and V have 16 rows each (166 -> 145 us for rank 10)
+  constexpr int kHold = 4;
+  const bool hold = m + nv <= 32 * kHold;
+  double2 ha[kHold], hb[kHold];
   double al = 0, be = 0, gr = 0, gi = 0;
-  for (int r = lane; r < m; r += 32) {
-    const double2 a = __ldcg(A + r), b = __ldcg(B + r);
+  auto products = [&](double2 a, double2 b) {
     al = fma(a.x, a.x, fma(a.y, a.y, al));
     be = fma(b.x, b.x, fma(b.y, b.y, be));
     gr = fma(a.x, b.x, fma(a.y, b.y, gr));
     gi = fma(a.x, b.y, fma(-a.y, b.x, gi));
+  };
+  if (hold) {
+#pragma unroll
+    for (int p = 0; p < kHold; ++p) {
+      const int r = lane + 32 * p;
+      ha[p] = hb[p] = make_double2(0.0, 0.0);
+      if (r < m + nv) {
+        ha[p] = __ldcg(r < m ? A + r : VA + (r - m));
+        hb[p] = __ldcg(r < m ? B + r : VB + (r - m));
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < kHold; ++p)
+      if (32 * p < m) {  // uniform
+        const bool in = lane + 32 * p < m;
+        products(in ? ha[p] : make_double2(0.0, 0.0), in ? hb[p] : make_double2(0.0, 0.0));
+      }
+  } else {
+    for (int r = lane; r < m; r += 32) products(__ldcg(A + r), __ldcg(B + r));
   }
   warp_sum4(al, be, gr, gi, lane);
   const double larger = al > be ? al : be;
@@ -104,16 +128,20 @@ __device__ __forceinline__ bool jacobi_pair(double2 *__restrict__ A, double2 *__
   const double q = fma(tr, tr, fma(ti, ti, 1.0)), y = as_double(rsqrtf(scaled_float(q, 0)));
   const double res = fma(-q * y, y, 1.0), c = fma(y * res, fma(0.375, res, 0.5), y);
   const double sr = c * tr, si = c * ti;
-  for (int r = lane; r < m; r += 32) {
-    const double2 a = __ldcg(A + r), b = __ldcg(B + r);
-    A[r] = make_double2(fma(c, a.x, fma(-sr, b.x, -si * b.y)), fma(c, a.y, fma(-sr, b.y, si * b.x)));
-    B[r] = make_double2(fma(sr, a.x, fma(-si, a.y, c * b.x)), fma(sr, a.y, fma(si, a.x, c * b.y)));
+  auto rotate = [&](double2 a, double2 b, double2 *pa, double2 *pb) {
+    *pa = make_double2(fma(c, a.x, fma(-sr, b.x, -si * b.y)), fma(c, a.y, fma(-sr, b.y, si * b.x)));
+    *pb = make_double2(fma(sr, a.x, fma(-si, a.y, c * b.x)), fma(sr, a.y, fma(si, a.x, c * b.y)));
+  };
+  if (hold) {
+#pragma unroll
+    for (int p = 0; p < kHold; ++p) {
+      const int r = lane + 32 * p;
+      if (r < m + nv) rotate(ha[p], hb[p], r < m ? A + r : VA + (r - m), r < m ? B + r : VB + (r - m));
+    }
+    return true;
   }
-  for (int r = lane; r < nv; r += 32) {
-    const double2 a = __ldcg(VA + r), b = __ldcg(VB + r);
-    VA[r] = make_double2(fma(c, a.x, fma(-sr, b.x, -si * b.y)), fma(c, a.y, fma(-sr, b.y, si * b.x)));
-    VB[r] = make_double2(fma(sr, a.x, fma(-si, a.y, c * b.x)), fma(sr, a.y, fma(si, a.x, c * b.y)));
-  }
+  for (int r = lane; r < m; r += 32) rotate(__ldcg(A + r), __ldcg(B + r), A + r, B + r);
+  for (int r = lane; r < nv; r += 32) rotate(__ldcg(VA + r), __ldcg(VB + r), VA + r, VB + r);
   return true;
 }
 
