@@ -116,34 +116,45 @@ struct NcWorkspace {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Block bookkeeping, one CTA per bond.  The order-defining loops (IndexLeft,
-// IndexRight) run on one thread in the reference's loop order (alpha outer,
-// i inner), so block rows/columns are in exactly the reference's order.
+// Block bookkeeping, one CTA of three warps per bond: left rows, right columns, classes of
+// betas.  The order-defining loops (IndexLeft, IndexRight) keep the reference's order
+// (alpha outer, i inner): a warp takes 32 entries of that order at a time, and an entry's
+// place is its block's fill plus the earlier lanes of the same block.  (One thread took
+// 1.1 ms for chi = 512, d = 5, waiting for a load per entry; now 0.06 ms.)
 // ---------------------------------------------------------------------------
-__global__ void k_nc_blocks(const int *__restrict__ lab_l, const int *__restrict__ lab_r,
+__global__ void __launch_bounds__(96) k_nc_blocks(const int *__restrict__ lab_l, const int *__restrict__ lab_r,
                             const int *links, Slot *slots, NcSlot *nc, JacobiProblem<double> *probs,
                             int chi, int d, int totNum, int maxFilling, int bmax, NcLocal nl) {
-  const int s = blockIdx.x;
-  if (threadIdx.x != 0) return;
+  extern __shared__ int cnt[];  // rows and columns per block (bmax each), betas per class (totNum + 2)
+  __shared__ int ends[4], err;
+  int *rows = cnt, *cols = cnt + bmax, *cls = cols + bmax;
+  const int s = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int link = links[s];
   const int *ll0 = lab_l + (size_t)(link - 1) * chi;  // LabelLeft(link)
   const int *ll1 = lab_l + (size_t)link * chi;        // LabelLeft(link+1)
   const int *lr2 = lab_r + (size_t)(link + 1) * chi;  // LabelRight(link+2)
-  NcSlot S = nc[s];
+  const NcSlot S = nc[s];
   // minmaxNLR (:1201-1250)
-  int mnl = ll0[0], mxl = 0, mnr = lr2[0], mxr = 0;
-  for (int a = 0; a < chi; ++a) {
-    mnl = min(mnl, ll0[a]);
-    const int v = ll0[a] == kLabelUnused ? 0 : ll0[a];
-    mxl = a == 0 ? v : max(mxl, v);
+  if (warp < 2) {
+    const int *l = warp == 0 ? ll0 : lr2;
+    int mn = l[0], mx = l[0] == kLabelUnused ? 0 : l[0];
+    for (int a = lane; a < chi; a += 32) {
+      mn = min(mn, l[a]);
+      mx = max(mx, l[a] == kLabelUnused ? 0 : l[a]);
+    }
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) {
+      ends[2 * warp] = mn;
+      ends[2 * warp + 1] = mx;
+    }
   }
-  for (int g = 0; g < chi; ++g) {
-    mnr = min(mnr, lr2[g]);
-    const int v = lr2[g] == kLabelUnused ? 0 : lr2[g];
-    mxr = g == 0 ? v : max(mxr, v);
-  }
-  mxl += maxFilling;
-  mxr += maxFilling;
+  if (tid == 64) err = 0;
+  for (int k = tid; k < 2 * bmax + totNum + 2; k += blockDim.x) cnt[k] = 0;
+  for (int k = tid; k < bmax; k += blockDim.x) probs[(size_t)s * bmax + k].n = 0;
+  for (int e = tid; e < chi * d; e += blockDim.x) S.rowpos[e] = S.colpos[e] = -1;
+  __syncthreads();
+  int mnl = ends[0], mxl = ends[1] + maxFilling, mnr = ends[2], mxr = ends[3] + maxFilling;
   if (mxl > totNum - mnr)
     mxl = totNum - mnr;
   else
@@ -153,102 +164,119 @@ __global__ void k_nc_blocks(const int *__restrict__ lab_l, const int *__restrict
   else
     mnl = totNum - mxr;
   const int nb = mxl - mnl + 1;
-  S.hdr[H_MINNL] = mnl;
-  S.hdr[H_MAXNL] = mxl;
-  S.hdr[H_MINNR] = mnr;
-  S.hdr[H_MAXNR] = mxr;
-  S.hdr[H_ERR] = 0;
-  for (int k = 0; k < bmax; ++k) probs[(size_t)s * bmax + k].n = 0;
-  if (nb < 1 || nb > bmax) {
-    S.hdr[H_NB] = 0;
-    S.hdr[H_ERR] = 1;
-    return;
+  const bool bad = nb < 1 || nb > bmax;
+  if (tid == 0) {
+    S.hdr[H_MINNL] = mnl;
+    S.hdr[H_MAXNL] = mxl;
+    S.hdr[H_MINNR] = mnr;
+    S.hdr[H_MAXNR] = mxr;
+    S.hdr[H_ERR] = bad;
+    S.hdr[H_NB] = bad ? 0 : nb;
   }
-  S.hdr[H_NB] = nb;
-  for (int k = 0; k < nb; ++k) S.rows[k] = S.cols[k] = 0;
+  if (bad) return;  // uniform
+  // block of entry e of the left (alpha, i) or right (gamma, j) order; -1: none, -2: out of range
+  auto left_block = [&](int e) -> int {
+    if (e >= chi * d || ll0[e / d] >= 1000) return -1;
+    const int NL = ll0[e / d] + nl.n[e % d];
+    return mnl <= NL && NL <= mxl ? NL - mnl : -1;
+  };
+  auto right_block = [&](int e) -> int {
+    if (e >= chi * d || lr2[e / d] >= 1000) return -1;
+    const int NR = lr2[e / d] + nl.n[e % d];
+    if (NR < mnr || NR > mxr) return -1;
+    const int k = totNum - NR - mnl;
+    return k < 0 || k >= nb ? -2 : k;
+  };
+  auto class_of = [&](int b) -> int { return b < chi && ll1[b] >= 0 && ll1[b] <= totNum ? ll1[b] : -1; };
   // SizeOfBlocks (:1252-1336)
-  for (int a = 0; a < chi; ++a)
-    for (int i = 0; i < d; ++i)
-      if (ll0[a] < 1000) {
-        const int NL = ll0[a] + nl.n[i];
-        if (mnl <= NL && NL <= mxl) S.rows[NL - mnl]++;
-      }
-  for (int g = 0; g < chi; ++g)
-    for (int j = 0; j < d; ++j)
-      if (lr2[g] < 1000) {
-        const int NR = lr2[g] + nl.n[j];
-        if (mnr <= NR && NR <= mxr) {
-          const int k = totNum - NR - mnl;
-          if (k < 0 || k >= nb) {
-            S.hdr[H_ERR] = 1;
-            S.hdr[H_NB] = 0;
-            return;
-          }
-          S.cols[k]++;
-        }
-      }
-  S.roff[0] = S.coff[0] = S.boffx[0] = S.boffv[0] = S.soff[0] = 0;
-  int maxdim = 0;
-  for (int k = 0; k < nb; ++k) {
-    const int m = S.rows[k], n = S.cols[k], mn = min(m, n);
-    S.roff[k + 1] = S.roff[k] + m;
-    S.coff[k + 1] = S.coff[k] + n;
-    S.boffx[k + 1] = S.boffx[k] + m * n;
-    S.boffv[k + 1] = S.boffv[k] + mn * mn;
-    S.soff[k + 1] = S.soff[k] + mn;
-    maxdim = max(maxdim, mn);
-  }
-  S.hdr[H_SZ] = S.soff[nb];
-  S.hdr[H_MAXDIM] = maxdim;
-  // IndexLeft (:1339-1391) and IndexRight (:1393-1443)
-  for (int e = 0; e < chi * d; ++e) S.rowpos[e] = S.colpos[e] = -1;
-  for (int k = 0; k < nb; ++k) S.rows[k] = 0;  // reused as fill counters
-  for (int a = 0; a < chi; ++a)
-    for (int i = 0; i < d; ++i)
-      if (ll0[a] < 1000 && mnl <= ll0[a] + nl.n[i] && ll0[a] + nl.n[i] <= mxl) {
-        const int k = ll0[a] + nl.n[i] - mnl;
-        const int p = S.roff[k] + S.rows[k]++;
-        S.l_alpha[p] = a;
-        S.l_i[p] = i;
-        S.rowpos[a * d + i] = p - S.roff[k];
-      }
-  for (int k = 0; k < nb; ++k) S.cols[k] = 0;
-  for (int g = 0; g < chi; ++g)
-    for (int j = 0; j < d; ++j)
-      if (lr2[g] < 1000 && mnr <= lr2[g] + nl.n[j] && lr2[g] + nl.n[j] <= mxr) {
-        const int k = totNum - (lr2[g] + nl.n[j]) - mnl;
-        const int p = S.coff[k] + S.cols[k]++;
-        S.r_gamma[p] = g;
-        S.r_j[p] = j;
-        S.colpos[g * d + j] = p - S.coff[k];
-      }
-  // betas of link+1 grouped by left label (stable counting sort, labels in [0, totNum])
-  for (int q = 0; q <= totNum + 1; ++q) S.cls_off[q] = 0;
-  for (int b = 0; b < chi; ++b)
-    if (ll1[b] >= 0 && ll1[b] <= totNum) S.cls_off[ll1[b] + 1]++;
-  for (int q = 0; q <= totNum; ++q) S.cls_off[q + 1] += S.cls_off[q];
-  for (int b = 0; b < chi; ++b)
-    if (ll1[b] >= 0 && ll1[b] <= totNum) S.cls_beta[S.cls_off[ll1[b]]++] = b;  // advances starts
-  for (int q = totNum + 1; q > 0; --q) S.cls_off[q] = S.cls_off[q - 1];          // restore
-  S.cls_off[0] = 0;
-  // Jacobi problems: block k is X_k (rows x cols) or its conjugate transpose
-  double2 *X = slots[s].X, *V = slots[s].V;
-  for (int k = 0; k < nb; ++k) {
-    const int m = S.rows[k], n = S.cols[k];
-    JacobiProblem<double> P;
-    P.X = X + S.boffx[k];
-    P.V = V + S.boffv[k];
-    if (m >= n) {
-      P.m = m;
-      P.n = n;
-    } else {
-      P.m = n;
-      P.n = m;
+  if (warp == 2) {
+    for (int b = lane; b < chi; b += 32)
+      if (class_of(b) >= 0) atomicAdd(&cls[class_of(b) + 1], 1);
+  } else {
+    for (int e = lane; e < chi * d; e += 32) {
+      const int k = warp == 0 ? left_block(e) : right_block(e);
+      if (k >= 0) atomicAdd(&(warp == 0 ? rows : cols)[k], 1);
+      if (k == -2) err = 1;
     }
+  }
+  __syncthreads();
+  if (err) {
+    if (tid == 0) {
+      S.hdr[H_ERR] = 1;
+      S.hdr[H_NB] = 0;
+    }
+    return;  // uniform
+  }
+  if (tid == 0) {
+    int ro = 0, co = 0, bx = 0, bv = 0, so = 0, maxdim = 0;
+    for (int k = 0; k <= nb; ++k) {
+      S.roff[k] = ro;
+      S.coff[k] = co;
+      S.boffx[k] = bx;
+      S.boffv[k] = bv;
+      S.soff[k] = so;
+      if (k == nb) break;
+      const int m = rows[k], n = cols[k], mn = min(m, n);
+      ro += m;
+      co += n;
+      bx += m * n;
+      bv += mn * mn;
+      so += mn;
+      maxdim = max(maxdim, mn);
+    }
+    S.hdr[H_SZ] = so;
+    S.hdr[H_MAXDIM] = maxdim;
+  } else if (tid == 64) {
+    for (int q = 0; q <= totNum; ++q) cls[q + 1] += cls[q];
+  }
+  __syncthreads();
+  for (int k = tid; k < nb; k += blockDim.x) {
+    S.rows[k] = rows[k];
+    S.cols[k] = cols[k];
+    // Jacobi problems: block k is X_k (rows x cols) or its conjugate transpose
+    JacobiProblem<double> P;
+    P.X = slots[s].X + S.boffx[k];
+    P.V = slots[s].V + S.boffv[k];
+    P.m = max(rows[k], cols[k]);
+    P.n = min(rows[k], cols[k]);
     P.ldx = P.m > 0 ? P.m : 1;
     P.ldv = P.n > 0 ? P.n : 1;
     P.floor = 0.0;
     probs[(size_t)s * bmax + k] = P;
+  }
+  for (int q = tid; q < totNum + 2; q += blockDim.x) S.cls_off[q] = cls[q];
+  __syncthreads();
+  for (int k = tid; k < nb; k += blockDim.x) rows[k] = cols[k] = 0;  // from here on: fills
+  __syncthreads();
+  // IndexLeft (:1339-1391), IndexRight (:1393-1443), betas of link+1 grouped by left label
+  int *fill = warp == 0 ? rows : warp == 1 ? cols : cls;
+  for (int e0 = 0; e0 < (warp == 2 ? chi : chi * d); e0 += 32) {
+    const int e = e0 + lane, k = warp == 0 ? left_block(e) : warp == 1 ? right_block(e) : class_of(e);
+    const unsigned on = __ballot_sync(0xffffffffu, k >= 0);
+    unsigned same = 0;
+    int at = 0;
+    if (k >= 0) {
+      same = __match_any_sync(on, k);
+      at = fill[k] + __popc(same & ((1u << lane) - 1u));
+    }
+    __syncwarp();
+    if (k >= 0) {
+      if ((same & ((1u << lane) - 1u)) == 0) fill[k] += __popc(same);
+      if (warp == 0) {
+        const int p = S.roff[k] + at;
+        S.l_alpha[p] = e / d;
+        S.l_i[p] = e % d;
+        S.rowpos[e] = at;
+      } else if (warp == 1) {
+        const int p = S.coff[k] + at;
+        S.r_gamma[p] = e / d;
+        S.r_j[p] = e % d;
+        S.colpos[e] = at;
+      } else {
+        S.cls_beta[at] = e;
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -699,13 +727,20 @@ __global__ void __launch_bounds__(1024) k_nc_select(int *lab_l, int *lab_r, doub
                                                     const double *nrm, double *truncerr,
                                                     double *sig_link, int *sig_count, int chi, int d,
                                                     int totNum, int bmax, int *status, double rank_bound) {
-  extern __shared__ double sh[];  // colnorm[sz] | flat rank scratch
+  extern __shared__ double sh[];  // sz values | chi values by rank | chi flat indices by rank
   if (status[0] & 1) return;  // non-finite ||Theta|| in the batch: the chain is left as it was
   const int s = blockIdx.x;
   const NcSlot S = nc[s];
   const int link = links[s];
   const int nb = S.hdr[H_NB], sz = S.hdr[H_SZ];
   double *cn = sh;  // column norms in flat (block-major, column) order, sz entries
+  // the same as integers: of nonnegative values the bits are ordered like the values, and an
+  // integer comparison costs a thirtieth of an FP64 one
+  const long long *bits = reinterpret_cast<const long long *>(sh);
+  double *val = sh + sz;
+  int *ord = reinterpret_cast<int *>(val + chi);
+  __shared__ double s_rs;
+  __shared__ int s_keep;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   // column norms: one warp per column
   for (int k = 0; k < nb; ++k) {
@@ -728,48 +763,52 @@ __global__ void __launch_bounds__(1024) k_nc_select(int *lab_l, int *lab_r, doub
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
       const double v = cn[o + c];
       if (!isfinite(v)) atomicOr(&status[0], 1);
+      const long long b = bits[o + c];
       int rank = 0;
+#pragma unroll 4
       for (int q = 0; q < n; ++q) {
-        const double w = cn[o + q];
-        rank += (w > v) || (w == v && q < c);
+        const long long w = bits[o + q];
+        rank += (w > b) || (w == b && q < c);
       }
       S.ssfl[o + rank] = v * inv;
       S.blkperm[o + rank] = c;
     }
   }
   __syncthreads();
+  for (int t = threadIdx.x; t < sz; t += blockDim.x) cn[t] = S.ssfl[t];
+  for (int beta = threadIdx.x; beta < chi; beta += blockDim.x) val[beta] = 0.0;
+  __syncthreads();
   // Ordering (:1515-1538): descending; equal values in descending flat index.
   // order(beta) = flat index (1-based) of the beta-th largest; only beta < chi is used.
-  int *ord = reinterpret_cast<int *>(sh);  // reuse: cn no longer needed
   for (int t = threadIdx.x; t < sz; t += blockDim.x) {
-    const double v = S.ssfl[t];
+    const long long b = bits[t];
     int rank = 0;
+#pragma unroll 4
     for (int q = 0; q < sz; ++q) {
-      const double w = S.ssfl[q];
-      rank += (w > v) || (w == v && q > t);
+      const long long w = bits[q];
+      rank += (w > b) || (w == b && q > t);
     }
-    if (rank < chi) ord[rank] = t + 1;
+    if (rank < chi) {
+      ord[rank] = t + 1;
+      val[rank] = cn[t];
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int mnl = S.hdr[H_MINNL];
-    int *ll1 = lab_l + (size_t)link * chi;
-    int *lr1 = lab_r + (size_t)link * chi;
-    double *l1 = lam + (size_t)link * chi;
+  if (threadIdx.x == 0) {  // the sums, in the reference's order
     // kept-rank form (no reference counterpart): the fewest leading values whose
     // discarded weight stays within rank_bound, as in the dense FormLambda1
+    const int top = min(chi, sz);
     int keep = chi;
     if (rank_bound > 0.0) {
-      const int top = min(chi, sz);
       double all = 0.0;
       for (int beta = 0; beta < top; ++beta) {
-        const double v = S.ssfl[ord[beta] - 1];
+        const double v = val[beta];
         if (v > kGuardNC) all = all + v * v;
       }
       double w = fmax(1.0 - all, 0.0);
       keep = top;
       while (keep > 1) {
-        const double v = S.ssfl[ord[keep - 1] - 1];
+        const double v = val[keep - 1];
         const double q = v > kGuardNC ? v * v : 0.0;
         if (w + q > rank_bound) break;
         w += q;
@@ -777,39 +816,46 @@ __global__ void __launch_bounds__(1024) k_nc_select(int *lab_l, int *lab_r, doub
       }
     }
     double renorm = 0.0;
-    for (int beta = 0; beta < chi; ++beta) {
-      int pb = 0, pp = 0;
-      double v = 0.0;
-      if (beta < sz) {
-        // JudgePosition (:1540-1565)
-        int ot = ord[beta];
-        for (int k = 0; k < nb; ++k) {
-          if (ot <= 0) break;
-          const int mn = S.soff[k + 1] - S.soff[k];
-          ot -= mn;
-          pb = k + 1;
-          pp = ot + mn;
-        }
-        v = S.ssfl[ord[beta] - 1];
-      }
-      S.pos_b[beta] = pb;
-      S.pos_p[beta] = pp;
-      // UpdateLabelLeft (:1583-1604) / UpdateLabelRight (:1615-1624)
-      const bool kept = beta < sz && beta < keep && v > kGuardNC;
-      const int lab = kept ? mnl + pb - 1 : kLabelUnused;
-      ll1[beta] = lab;
-      lr1[beta] = lab < 1000 ? totNum - lab : kLabelUnused;
-      // FormLambdaNC (:1642-1656)
-      const double tl = kept ? v : 0.0;
-      l1[beta] = tl;
+    for (int beta = 0; beta < min(top, keep); ++beta) {
+      const double v = val[beta], tl = v > kGuardNC ? v : 0.0;
       renorm = renorm + tl * tl;
     }
+    s_keep = keep;
+    s_rs = sqrt(renorm);
     truncerr[s] = fabs(1.0 - renorm);
-    const double rs = sqrt(renorm);
-    for (int beta = 0; beta < chi; ++beta) l1[beta] = l1[beta] / rs;
     sig_count[link - 1] = sz;
   }
-  for (int t = threadIdx.x; t < sz; t += blockDim.x) sig_link[(size_t)(link - 1) * d * chi + t] = S.ssfl[t];
+  __syncthreads();
+  const int mnl = S.hdr[H_MINNL], keep = s_keep;
+  const double rs = s_rs;
+  int *ll1 = lab_l + (size_t)link * chi;
+  int *lr1 = lab_r + (size_t)link * chi;
+  double *l1 = lam + (size_t)link * chi;
+  for (int beta = threadIdx.x; beta < chi; beta += blockDim.x) {
+    int pb = 0, pp = 0;
+    const double v = val[beta];
+    if (beta < sz) {
+      // JudgePosition (:1540-1565)
+      int ot = ord[beta];
+      for (int k = 0; k < nb; ++k) {
+        if (ot <= 0) break;
+        const int mn = S.soff[k + 1] - S.soff[k];
+        ot -= mn;
+        pb = k + 1;
+        pp = ot + mn;
+      }
+    }
+    S.pos_b[beta] = pb;
+    S.pos_p[beta] = pp;
+    // UpdateLabelLeft (:1583-1604) / UpdateLabelRight (:1615-1624)
+    const bool kept = beta < sz && beta < keep && v > kGuardNC;
+    const int lab = kept ? mnl + pb - 1 : kLabelUnused;
+    ll1[beta] = lab;
+    lr1[beta] = lab < 1000 ? totNum - lab : kLabelUnused;
+    // FormLambdaNC (:1642-1656)
+    l1[beta] = (kept ? v : 0.0) / rs;
+  }
+  for (int t = threadIdx.x; t < sz; t += blockDim.x) sig_link[(size_t)(link - 1) * d * chi + t] = cn[t];
 }
 
 // ---------------------------------------------------------------------------
@@ -934,8 +980,11 @@ __global__ void __launch_bounds__(1024) k_nc_cut(NcSlot *nc, const JacobiProblem
     double best = INFINITY;
     for (int t = threadIdx.x; t < sz; t += blockDim.x) {
       const double v = val[t];
+      const long long *bits = reinterpret_cast<const long long *>(val);  // nonnegative: ordered like the values
+      const long long b = bits[t];
       int above = 0;
-      for (int q = 0; q < sz; ++q) above += val[q] > v;
+#pragma unroll 4
+      for (int q = 0; q < sz; ++q) above += bits[q] > b;
       if (above < chi) best = fmin(best, v);
     }
     for (int q = 16; q > 0; q >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, q));
@@ -1321,8 +1370,8 @@ int run_nc_batch(tebd_handle *h, int nb, const int * /*links_host*/, double * /*
   NcLocal nl;
   for (int i = 0; i < 8; ++i) nl.n[i] = (h->nc_idf && i < d) ? h->nc_conserv[i] : i;
   cudaStream_t st = h->stream;
-  k_nc_blocks<<<nb, 32, 0, st>>>(h->lab_l, h->lab_r, h->links_d, h->slots_d, w->slots_d, w->probs_d,
-                                 chi, d, N, mf, bmax, nl);
+  k_nc_blocks<<<nb, 96, sizeof(int) * (2 * (size_t)bmax + N + 2), st>>>(h->lab_l, h->lab_r, h->links_d, h->slots_d,
+                                                                        w->slots_d, w->probs_d, chi, d, N, mf, bmax, nl);
   TEBD_LAUNCHED(h);
   if (d < 2) return set_error(h, TEBD_ERR_ARG, "NC mode needs d >= 2");
   const bool df = h->opts.svd_mode == TEBD_SVD_DF;
@@ -1387,7 +1436,10 @@ int run_nc_batch(tebd_handle *h, int nb, const int * /*links_host*/, double * /*
   } else if ((rc = run_jacobi_problems(h, w->probs_d, nb * bmax, maxdim))) {
     return rc;
   }
-  const size_t shb = std::max(sizeof(double) * (size_t)maxsz, sizeof(int) * (size_t)chi) + 16;
+  const size_t shb = sizeof(double) * ((size_t)maxsz + chi) + sizeof(int) * (size_t)chi;
+  if ((rc = check_cuda(h, cudaFuncSetAttribute(k_nc_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shb),
+                       "NC selection shared memory")))
+    return rc;
   k_nc_select<<<nb, 1024, shb, st>>>(h->lab_l, h->lab_r, h->lam, h->links_d, w->slots_d, w->probs_d,
                                      h->nrm, h->truncerr_d, h->sig_link_d, h->sig_count_d, chi, d, N,
                                      bmax, h->status_d, h->unnormalized ? 0.0 : h->rank_bound);
