@@ -109,7 +109,8 @@ __device__ __forceinline__ int gk_count_f32(const float *sqf, int n1, float x) {
 // step instead of bisection's 1).  While the values leave schedulers idle, the
 // sequential recurrences bound the kernel and extra lanes are free; once there is a warp
 // per scheduler, teams of 1 lane (bisection) do the least work.  The host picks kTeam
-// per launch.  Measured: 128 values of 32 bonds, n = 640: 7.8 -> 2.4 ms; 90 of 10, n =
+// per launch; where sizes differ a value counts by its problem's share of the largest (its
+// lanes are free that much earlier).  Measured: 128 values of 32 bonds, n = 640: 7.8 -> 2.4 ms; 90 of 10, n =
 // 270: 2.26 -> 0.60 ms.
 constexpr int kSigmaThreads = 32;
 template <int kTeam>
@@ -476,7 +477,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const double values = (double)nb * std::min(kk, nmax), lanes = 4.0 * 32.0 * std::max(sms, 1);
+    const double values = b.values > 0 ? b.values : (double)nb * std::min(kk, nmax), lanes = 4.0 * 32.0 * std::max(sms, 1);
     int team = 1;
     while (team < 16 && values * 2 * team <= lanes) team *= 2;
     const TuneParams tp = tune_lookup(h, b.dfp ? 1 : 0, nmax, nb);

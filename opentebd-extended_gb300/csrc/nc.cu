@@ -1210,6 +1210,8 @@ int nc_route_blocks(tebd_handle *h, NcWorkspace *w, int nb, int *nbd, int *small
   out->nmax = mmax;
   out->kk = nmaxb;
   out->dfp = h->opts.svd_mode == TEBD_SVD_DF;
+  out->values = 0.0;
+  for (const Compact &c : w->bcp_h) out->values += (double)c.n * c.n / nmaxb;
   out->phase = 0;
   out->cap = 0;
   return TEBD_OK;

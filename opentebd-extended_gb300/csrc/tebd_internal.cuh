@@ -254,6 +254,7 @@ struct BidiagBatch {
   bool dfp;
   int phase;  // 0: whole route; 1: through the singular values; 2: the vectors
   int cap;    // 1: vectors only for the first cp->k values of each problem (set between phases)
+  double values = 0;   // singular values of the batch, weighted by size / largest size; 0: nb min(kk, nmax)
   int right_only = 0;  // 1: right singular vectors only (double-float form; S.X keeps no left vectors)
 };
 int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b);
