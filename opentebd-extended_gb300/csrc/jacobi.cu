@@ -111,23 +111,39 @@ __device__ __forceinline__ bool jacobi_pair(double2 *__restrict__ A, double2 *__
   warp_sum4(al, be, gr, gi, lane);
   const double larger = al > be ? al : be;
   if (!(al > floor) || !(be > floor) || !(larger < INFINITY)) return false;
-  const int e = ((__double2hiint(larger) >> 20) & 0x7ff) - 1023;
-  const float fr = scaled_float(gr, e), fi = scaled_float(gi, e), big = fmaxf(fabsf(fr), fabsf(fi));
-  if (big == 0.0f) return false;
-  const float ratio = fminf(fabsf(fr), fabsf(fi)) / big, g = big * sqrtf(1.0f + ratio * ratio);
-  auto root = [&](double x) -> float {  // sqrt(x 2^-e), also where x 2^-e is out of FP32's range
-    int ex = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
-    ex -= (ex - e) & 1;
-    return sqrtf(scaled_float(x, ex)) * __int_as_float(max(0, (ex - e) / 2 + 127) << 23);
-  };
-  if (!(g > (float)tol * root(al) * root(be))) return false;
-  const float zeta = scaled_float(be - al, e + 1) / g;
-  const float t = fabsf(zeta) > 1e15f ? 0.5f / zeta : copysignf(1.0f, zeta) / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
-  const double tr = as_double(t * (fr / g)), ti = as_double(t * (fi / g));
-  // c = 1 / sqrt(q), q in [1, 2]: the FP32 value, then one step of third order
-  const double q = fma(tr, tr, fma(ti, ti, 1.0)), y = as_double(rsqrtf(scaled_float(q, 0)));
-  const double res = fma(-q * y, y, 1.0), c = fma(y * res, fma(0.375, res, 0.5), y);
-  const double sr = c * tr, si = c * ti;
+  double c, sr, si;
+  if (!(floor > 0.0)) {
+    // Without a floor the columns of a rank-deficient matrix have to be rotated down to
+    // rounding noise, which makes them independent; what an FP32 angle leaves (1e-7 of a
+    // column per sweep) stays in the span of the large ones and is rotated without end.
+    const double g = sqrt(gr * gr + gi * gi);
+    if (!(g > tol * sqrt(al) * sqrt(be))) return false;
+    const double zeta = (be - al) / (2.0 * g);
+    const double t = fabs(zeta) > 1e150 ? 0.5 / zeta : copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+    c = 1.0 / sqrt(1.0 + t * t);
+    sr = c * t * (gr / g);
+    si = c * t * (gi / g);
+  } else {
+    const int e = ((__double2hiint(larger) >> 20) & 0x7ff) - 1023;
+    const float fr = scaled_float(gr, e), fi = scaled_float(gi, e), big = fmaxf(fabsf(fr), fabsf(fi));
+    if (big == 0.0f) return false;
+    const float ratio = fminf(fabsf(fr), fabsf(fi)) / big, g = big * sqrtf(1.0f + ratio * ratio);
+    auto root = [&](double x) -> float {  // sqrt(x 2^-e), also where x 2^-e is out of FP32's range
+      int ex = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
+      ex -= (ex - e) & 1;
+      return sqrtf(scaled_float(x, ex)) * __int_as_float(max(0, (ex - e) / 2 + 127) << 23);
+    };
+    if (!(g > (float)tol * root(al) * root(be))) return false;
+    const float zeta = scaled_float(be - al, e + 1) / g;
+    const float t = fabsf(zeta) > 1e15f ? 0.5f / zeta : copysignf(1.0f, zeta) / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
+    const double tr = as_double(t * (fr / g)), ti = as_double(t * (fi / g));
+    // c = 1 / sqrt(q), q in [1, 2]: the FP32 value, then one step of third order
+    const double q = fma(tr, tr, fma(ti, ti, 1.0)), y = as_double(rsqrtf(scaled_float(q, 0)));
+    const double res = fma(-q * y, y, 1.0);
+    c = fma(y * res, fma(0.375, res, 0.5), y);
+    sr = c * tr;
+    si = c * ti;
+  }
   auto rotate = [&](double2 a, double2 b, double2 *pa, double2 *pb) {
     *pa = make_double2(fma(c, a.x, fma(-sr, b.x, -si * b.y)), fma(c, a.y, fma(-sr, b.y, si * b.x)));
     *pb = make_double2(fma(sr, a.x, fma(-si, a.y, c * b.x)), fma(sr, a.y, fma(si, a.x, c * b.y)));
