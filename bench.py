@@ -162,9 +162,9 @@ def cpu_sample(gam, lam, Udt, links, workers):
 def hbm_roofline(traffic_bytes, avg_launch_ms, peaks_path):
     """The dominant kernel on the HBM roofline: its measured DRAM traffic per
     launch over its average launch time, against the measured copy bandwidth of
-    this machine's GPUs (None when a figure is missing).  k_gebrd is bound by the FP64
-    pipe, so this fraction is far below one; it shows how far from memory-bound
-    the kernel is."""
+    this GPU's kind (None when a figure is missing).  k_gebrd is bound by a serial
+    chain per column and the integer pipe, so this fraction is far below one; it
+    shows how far from memory-bound the kernel is."""
     if not traffic_bytes or not avg_launch_ms or not os.path.exists(peaks_path):
         return None
     try:
@@ -306,7 +306,7 @@ def saturated_legs(pkg, device, args, fp64_peak, steps=3, Ls=L, chi=CHI, decay=1
     """The odd bonds of a saturated chain, updated `steps` times (one batched sweep
     each), in plain FP64 and in the mixed form, profiled: updates/s from CUDA events
     on each chain's stream, and the roofline of each form's dominant kernel from
-    that leg's own launch timings (k_gebrd on the FP64 pipe; the tensor-core
+    that leg's own launch timings (k_gebrd's 64-bit flops against the FP64 peak; the tensor-core
     product kernels against the measured bf16 peak).
 
     prepare: the legs start from the random state after one sweep of the same
@@ -585,8 +585,8 @@ def run_ours(args):
 
     prec = None
     if args.svd == "fp64" and not args.no_precision:
-        prec = {"svd": "TEBD_SVD_DF: bidiagonal route's trailing-matrix passes, trailing updates and "
-                       "back-transformation in double-float on the FP32 pipe; the rest FP64"}
+        prec = {"svd": "TEBD_SVD_DF: the gate and small Thetas in double-float on the FP32 pipe; the SVD as "
+                       "in plain FP64"}
         prec.update(leg(SVD_MODES["df"]))
     mixed = None
     if args.svd == "fp64" and not args.no_precision:
@@ -646,13 +646,13 @@ def run_ours(args):
         "metric": METRIC, "value": value, "unit": "updates/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None,
-        "dtype": "c128 (f64; bidiagonalisation passes in double-float)" if args.svd == "df" else "c128 (f64)",
+        "dtype": "c128 (f64; gate and small Thetas in double-float)" if args.svd == "df" else "c128 (f64)",
         "data": "synthetic",
         "config": {"workload": WORKLOAD, "L": L, "d": D, "chi": CHI, "J": J, "U": U, "mu": MU, "dt": DT,
                    "trotter_order": ORDER, "updates_per_step": UPDATES_PER_STEP,
-                   "svd": ("fp64 per bond: Householder bidiagonalisation + bisection + inverse iteration "
-                           "(both compacted dimensions >= 64 in a batch holding a saturated bond or one above "
-                           "384 columns), else pivoted QR + one-sided Jacobi on R^H"
+                   "svd": ("fp64 per bond: Householder bidiagonalisation in 64-bit fixed point + bisection + "
+                           "inverse iteration (batches holding a saturated bond or one above 384 columns), else "
+                           "pivoted QR + QR of R^H + one-sided Jacobi"
                            if args.svd == "fp64" else "svd_mode %s for every bond" % args.svd),
                    "timed_window": "Trotter steps 1..%d of the configured 200-step run (warm-up on a copy)" % args.steps,
                    "bidiag_updates": st["bidiag_updates"], "updates": st["updates"],

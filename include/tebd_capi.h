@@ -68,20 +68,19 @@ extern "C" {
 #define TEBD_MODE_NC 1            /* TwoSiteOpNC: U(1) number conservation             */
 
 /* SVD algorithm (all FP64 but the precision form) */
-#define TEBD_SVD_FP64 0           /* default: per bond, bidiagonalisation when both
-                                     dimensions of the compacted Theta are >= 64 (a wide
-                                     one as Theta^H) and its batch holds a saturated bond
-                                     (all chi of its Lambda in use) or one above 384,
-                                     else column-pivoted QR + one-sided Jacobi on R^H    */
+#define TEBD_SVD_FP64 0           /* default: per bond, bidiagonalisation (in 64-bit fixed
+                                     point; a wide Theta as Theta^H) when its batch holds
+                                     a saturated bond (all chi of its Lambda in use) or
+                                     one above 384 columns -- below 64 columns only with
+                                     Schmidt values that span at most 1e-8 -- else
+                                     column-pivoted QR + one-sided Jacobi                */
 #define TEBD_SVD_JACOBI 2         /* one-sided Jacobi on the whole (compacted) Theta    */
 #define TEBD_SVD_BIDIAG 3         /* bidiagonalisation for every Theta (>= 2 x 2)       */
 #define TEBD_SVD_QRJ 4            /* pivoted QR + Jacobi on R^H for every bond          */
-#define TEBD_SVD_DF 5             /* precision form: as TEBD_SVD_FP64, but the bidiagonal
-                                     route's passes over the trailing matrix, trailing
-                                     updates, back-transformation and Gram-Schmidt, and
-                                     the Theta formation, run in double-float (pairs of
-                                     FP32, 48-bit significands) on the FP32 pipe; number-
-                                     conserving blocks on the bidiagonal route too       */
+#define TEBD_SVD_DF 5             /* precision form: as TEBD_SVD_FP64, but the gate and the
+                                     Theta formation of small products run in double-float
+                                     (pairs of FP32, 48-bit significands) on the FP32 pipe,
+                                     the number-conserving Theta too; the SVD is the same */
 #define TEBD_SVD_RSVD 6           /* learned-rank form: bonds whose compacted Theta is
                                      much larger than the kept rank r take a randomized
                                      sketch of width r + p with FP64-class products on
@@ -247,7 +246,9 @@ int tebd_set_rsvd_model(tebd_handle *h, tebd_mlp *m, double target);
 
 /* Theta formation (FormTheta, local_operations_module.f90:184-211) on the tensor
  * cores (no counterpart in the reference, which forms Theta in FP64 loops).
- * form 0: CUDA cores (FP64, or double-float with TEBD_SVD_DF), the default; 3:
+ * form 0, the default: CUDA cores (FP64, or double-float with TEBD_SVD_DF) for small
+ * products, eight digit planes with balanced operands (at least FP64's accuracy) for
+ * dense ones of 2^21 multiply-adds or more; 3:
  * 3xTF32 split-precision product with FP32 accumulation (~FP32 accuracy; the
  * precision tier's Theta; dense handles only); 100 + S, S = 3..7: S bf16 digit
  * planes (error ~2^(-7S) of the largest terms; S = 7 is FP64 class).  On
@@ -271,8 +272,9 @@ int tebd_set_conserv(tebd_handle *h, const int *conserv);
 
 /* Singular values of the normalised Theta from the last update of `link`
  * (descending; NC mode: the flattened block values in the reference's order).
- * *count receives how many were written: all d*chi (zeros included) on the
- * Jacobi routes, the chi kept ones on the bidiagonal route; the buffer holds d*chi. */
+ * *count receives how many were written: all d*chi (zeros included) on the Jacobi
+ * routes and for a default-route bond below 64 columns, the chi kept ones on the
+ * bidiagonal route otherwise; the buffer holds d*chi. */
 int tebd_get_singular_values(tebd_handle *h, int link, double *sigma, int *count);
 
 /* Jacobi sweeps used by the last update of `link` (diagnostics). */

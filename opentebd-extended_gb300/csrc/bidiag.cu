@@ -28,7 +28,6 @@
 #include <algorithm>
 
 #include "bidiag.cuh"
-#include "df.cuh"
 
 namespace tebd {
 

@@ -536,10 +536,7 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
       if ((rc = launch_eye(h, nb))) return rc;
       if ((rc = run_jacobi(h, nb, h->opts.svd_mode, nmax))) return rc;
     } else {
-      // route per bond: bidiagonalisation when the compacted Theta is large in both
-      // dimensions (default: min(m, n) >= kBidiagMinDim in a batch that holds a
-      // saturated or large bond, below; a wide Theta is bidiagonalised as
-      // Theta^H), pivoted QR + Jacobi on R^H otherwise (low rank, cheap sweeps)
+      // route per bond (a wide Theta is bidiagonalised as Theta^H), below
       int nbd = 0, nbd_max = 0;
       // randomized route: bonds whose smaller compacted side exceeds the sketch
       // (kept rank + oversampling) by a margin; the judge may send some back
@@ -586,23 +583,21 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
           }
         }
       }
-      // default routing: the bidiagonal route from 64 columns when the batch holds
-      // a saturated bond (all chi of its Lambda in use: the gate fills Theta's
-      // spectrum, rank ~ n, where the bidiagonal route's fixed O(n^3) is ~8x
-      // cheaper than Jacobi sweeps; the batch's other bonds ride along in the same
-      // launches) or a bond beyond kQrjMaxDim; a batch of unsaturated Thetas up to
-      // kQrjMaxDim columns keeps the QR route, whose cost follows the numerical
-      // rank (the chi = 128 run's steps 1..20, mean 177 columns: 1.30x faster than
-      // bidiagonalising from 64 columns).  Mixing the routes in one batch would
-      // serialise them (the QR batch, then the bidiagonal one).  A batch that took
-      // the randomized route holds saturated bonds.
+      // default routing: the bidiagonal route from 64 columns when the batch holds a
+      // saturated bond (all chi of its Lambda in use: the gate fills Theta's spectrum,
+      // rank ~ n) or a bond beyond kQrjMaxDim; the batch's other bonds ride along in the
+      // same launches (the two routes of one batch run one after the other).  A batch of
+      // unsaturated Thetas up to kQrjMaxDim columns keeps the QR route: its cost follows
+      // the numerical rank, and its sweeps resolve the vectors of the smallest values to
+      // their own size.  The bidiagonal route leaves 1e-16 of the largest in every row of
+      // U, which the division by a small Lambda0 turns into Schmidt values above the
+      // guard, and the chain fills up with them (the chi = 128 run's first 8 steps: 83 ms
+      // against 740).  A batch that took the randomized route holds saturated bonds.
       //
-      // Below 64 columns the same holds for a saturated bond (32 columns, rank 32: 5.1 ms by
-      // the QR route, 1.1 by the bidiagonal one), and a batch's other small bonds ride
-      // along, as long as a bond's values span no more than kBidiagSpan: the Jacobi
-      // sweeps resolve the vectors of the smallest values to their own size, the
-      // bidiagonal route only to the largest one's.  These bonds still report all their
-      // values (kPathAll).
+      // Below 64 columns the same holds for a saturated bond (32 columns of rank 32: 1.30 ms
+      // by the QR route, 0.98 by the bidiagonal one), and a batch's other small bonds
+      // ride along, as long as a bond's values span no more than kBidiagSpan, well
+      // above that rounding.  These bonds still report all their values (kPathAll).
       const int mode = h->opts.svd_mode;
       const bool choose = mode != TEBD_SVD_BIDIAG && mode != TEBD_SVD_QRJ;
       bool full_batch = nrs > 0, any_full = full_batch;

@@ -197,7 +197,7 @@ struct tebd_handle {
   double rank_bound;       // kept-rank form: discarded weight bound per bond (0 = keep chi)
   cudaEvent_t ev[6];
   // tensor-core products (theta_tc.cu)
-  int theta_form;          // 0: CUDA cores (FP64, or double-float with TEBD_SVD_DF);
+  int theta_form;          // 0: by size, CUDA cores (FP64, or double-float with TEBD_SVD_DF) or 8 digit planes;
                            // 3: 3xTF32; 100 + S: S bf16 digit planes (tcgen05)
   void *tc_ws;             // operand planes / digits, grown on demand
   size_t tc_ws_bytes;

@@ -2,7 +2,7 @@
 //
 // Three launch parameters set how a batch of bonds maps onto the GPU without
 // changing what is computed:
-//   * the cluster size of the bidiagonalisation (k_gebrd / k_gebrd_df: one
+//   * the cluster size of the bidiagonalisation (k_gebrd: one
 //     cluster of 1..8 CTAs per bond; more CTAs share each column's passes but
 //     fewer bonds run at once);
 //   * the team size of the bisection (k_bd_sigma<team>: 1, 2, 4 or 8 lanes
