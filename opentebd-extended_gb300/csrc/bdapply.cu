@@ -267,7 +267,7 @@ int launch_bd_apply(tebd_handle *h, const BidiagBatch &b) {
   k_bd_wy<<<dim3((b.nmax + 4 * kB - 1) / (4 * kB), b.nb, sides), 128, 0, h->stream>>>(b.slots_d, b.path_d, sides);
   TEBD_LAUNCHED(h);
   auto go = [&](auto kern) {
-    int rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    int rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem),
                         "back-transformation shared memory");
     if (rc) return rc;
     kern<<<dim3(sides * ((b.kk + cols - 1) / cols), b.nb), kWarps * 32, smem, h->stream>>>(b.slots_d, b.path_d, b.kk,

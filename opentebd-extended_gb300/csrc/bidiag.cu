@@ -35,6 +35,10 @@ namespace {
 
 inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
+// limit of the dynamic shared memory, one value for all calls: the attribute belongs to
+// the process, and another thread's call may launch in between
+constexpr int kSmemMax = 200 * 1024;
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -486,7 +490,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
                 : team == 4 ? k_bd_sigma<4>
                 : team == 2 ? k_bd_sigma<2>
                             : k_bd_sigma<1>;
-    if ((rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    if ((rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax),
                          "bisection shared memory")))
       return rc;
     bool all = false;
@@ -498,7 +502,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
   }  // vectors
   {
     const size_t smem = sizeof(double) * (size_t)(2 * nmax);
-    if ((rc = check_cuda(h, cudaFuncSetAttribute(k_bd_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    if ((rc = check_cuda(h, cudaFuncSetAttribute(k_bd_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax),
                          "inverse iteration shared memory")))
       return rc;
     k_bd_invit<<<dim3(cdiv(kk, 32), nb), 32, smem, st>>>(slots_d, path_d, kk, cap);

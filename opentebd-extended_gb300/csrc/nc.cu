@@ -1439,7 +1439,7 @@ int run_nc_batch(tebd_handle *h, int nb, const int * /*links_host*/, double * /*
     return rc;
   }
   const size_t shb = sizeof(double) * ((size_t)maxsz + chi) + sizeof(int) * (size_t)chi;
-  if ((rc = check_cuda(h, cudaFuncSetAttribute(k_nc_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shb),
+  if ((rc = check_cuda(h, cudaFuncSetAttribute(k_nc_select, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024),
                        "NC selection shared memory")))
     return rc;
   k_nc_select<<<nb, 1024, shb, st>>>(h->lab_l, h->lab_r, h->lam, h->links_d, w->slots_d, w->probs_d,

@@ -442,7 +442,7 @@ int run_qrj(tebd_handle *h, int nb) {
   int warps = 8;
   while (warps > 1 && 16 * (size_t)mx * warps > kSmemMax) warps /= 2;
   const size_t smem = 16 * (size_t)mx * warps <= kSmemMax ? 16 * (size_t)mx * warps : 0;
-  if ((rc = check_cuda(h, cudaFuncSetAttribute(k_qrj_apply_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  if ((rc = check_cuda(h, cudaFuncSetAttribute(k_qrj_apply_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax),
                        "back-transformation shared memory")))
     return rc;
   k_qrj_apply_q<<<dim3((kx + warps - 1) / warps, nb, 2), 32 * warps, smem, st>>>(h->slots_d, h->path_d, smem > 0);
