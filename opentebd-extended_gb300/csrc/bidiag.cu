@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
   // from it and three solves leave each a like share of the cluster's vectors.  With
   // the value itself as the shift one member takes all: the set's condition is 1e6 to
   // 1e13, and its left and right vectors, each re-orthogonalised, no longer belong together
-  // (U diag(s) V^H off by up to 1e-8 ||B|| for 128 equal values; now 5e-15).  A single
+  // (Theta rebuilt from 64 equal values was off by 8e-10 of its norm, now by 5e-15; from 128
+  // by 1.4e-13).  A single
   // value 1e-11 ||T|| or more from the next is resolved to rounding by three solves.
   lam += 64.0 * ptol;
   const unsigned long long pbits = abs_bits(ptol);
