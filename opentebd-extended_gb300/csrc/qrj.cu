@@ -237,6 +237,9 @@ __global__ void __launch_bounds__(kQThreads, 1) k_qrj_factor(Slot *slots, Jacobi
     if (blockIdx.x == 0 && tid == 0) jp[s].n = 0;
     return;  // uniform per cluster
   }
+  // the others' shared memory may be accessed once they are known to run: the norms below
+  // are stored to every CTA
+  cluster.sync();
   const Slot S = slots[s];
   const int m = S.cp->m, n = S.cp->n, mx = max(m, n);
   extern __shared__ __align__(16) char sh[];
