@@ -245,15 +245,27 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
     return;
   }
   const double ptol = fmax(2.220446049250313e-16 * __longlong_as_double((long long)tb), 1e-300);
-  // The shift lies 64 ulps of ||T|| above the value, so that the members of a cluster (a
-  // degenerate value spreads over tens of ulps by the rounding of B) are all about as far
-  // from it and three solves leave each a like share of the cluster's vectors.  With
-  // the value itself as the shift one member takes all: the set's condition is 1e6 to
-  // 1e13, and its left and right vectors, each re-orthogonalised, no longer belong together
-  // (Theta rebuilt from 64 equal values was off by 8e-10 of its norm, now by 5e-15; from 128
-  // by 1.4e-13).  A single
-  // value 1e-11 ||T|| or more from the next is resolved to rounding by three solves.
-  lam += 64.0 * ptol;
+  // Inside a cluster (values within 8 ulps of the largest of one another; the bisection and the
+  // rounding of B spread a degenerate value that far) the shift lies 64 ulps above the value,
+  // so that the members are all about as far from it and the solves leave each a like share
+  // of the cluster's vectors.  With the value itself as the shift one member takes all: the
+  // set's condition is 1e6 to 1e13, and its left and right vectors, each re-orthogonalised,
+  // no longer belong together (Theta rebuilt from 64 equal values was off by 8e-10 of its
+  // norm).  It stays at a quarter of the way to the next value above the cluster, which would
+  // take over otherwise, and at 1/64 of the value, whose negative is an eigenvalue
+  // too: with 64 ulps everywhere the left and right vectors of values below 1e-14 of the
+  // largest were paired at random.  Other values are the shift themselves: a neighbour at a
+  // distance g leaves a share of (ulp / g)^3.
+  {
+    const double ulp = 2.220446049250313e-16 * sig[0], near = 8.0 * ulp, own = lam;
+    if ((i > 0 && sig[i - 1] - own <= near) || (i + 1 < K && own - sig[i + 1] <= near)) {
+      int j = i;  // the cluster's first value
+      while (j > 0 && sig[j - 1] - sig[j] <= near) --j;
+      double shift = fmin(64.0 * ulp, 0.015625 * own);
+      if (j > 0) shift = fmin(shift, 0.25 * (sig[j - 1] - own));
+      lam = own + shift;
+    }
+  }
   const unsigned long long pbits = abs_bits(ptol);
   auto guard = [&](double p) -> double { return abs_bits(p) >= pbits ? p : copysign(ptol, p); };
   // LU with partial pivoting of T - lam I (diagonal -lam, off-diagonals off[j])
