@@ -75,7 +75,7 @@ constexpr int kMostK = 2048;  // coefficients of more vectors stay in global mem
 
 // z's sets in fixed point, column by column: element (j, i) of set p at
 // Zi[(p K + i) n + j], the layout the kernel below and the back-transformation read
-__global__ void __launch_bounds__(256) k_bd_zfix(Slot *slots, const int *path, int kk, int cap) {
+__global__ void __launch_bounds__(256) k_bd_zfix(Slot *slots, const int *path, int kk, int cap, int second) {
   __shared__ double tile[2][32][33];
   const int s = blockIdx.z;
   const int route = path[s];
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256) k_bd_zfix(Slot *slots, const int *path, i
   bd_dims(*S.cp, route, m, n);
   const int K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  if (i0 >= K || j0 >= n) return;  // uniform
+  if (i0 >= K || j0 >= n || (second && !bd_clustered(S.bdws + 2 * n, K))) return;  // uniform
   double *base = S.bdws + bd_scratch(n, kk);
   const double *Z = base + 5 * (size_t)(2 * n) * K;
   int2 *Zi = reinterpret_cast<int2 *>(base);
@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(256) k_bd_zfix(Slot *slots, const int *path, i
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_bd_orth(Slot *slots, const int *path, int kk, int cap, int d_in_smem) {
+__global__ void __launch_bounds__(kThreads, 1) k_bd_orth(Slot *slots, const int *path, int kk, int cap, int d_in_smem,
+                                                        int second) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bd_orth(Slot *slots, const int 
   int m, n;
   bd_dims(*S.cp, route, m, n);
   const int K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
+  if (second && !bd_clustered(S.bdws + 2 * n, K)) return;  // uniform per cluster
   double *base = S.bdws + bd_scratch(n, kk);
   int2 *Zi = reinterpret_cast<int2 *>(base) + (size_t)part * K * n;
   // the CTAs' dot products, two buffers in turn: [buffer][CTA][vector][panel vector]
@@ -347,12 +349,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_bd_orth(Slot *slots, const int 
 // coefficients that shared memory cannot hold
 size_t bd_orth_ws_doubles(int K) { return 4 * (size_t)kMaxC * (K + kPan) * kPan + 2 * (size_t)kPan * K; }
 
-// Both kernels on the batch; C CTAs per set, or the autotuner's number.
-int launch_bd_orth(tebd_handle *h, const BidiagBatch &b) {
+// Both kernels on the batch; C CTAs per set, or the autotuner's number.  second: the second
+// pass, only problems with clustered values; *clusters: C, 0 before the first pass.
+int launch_bd_orth(tebd_handle *h, const BidiagBatch &b, int second, int *clusters) {
   const int sides = b.right_only ? 1 : 2;
   int nbd = 0;
   for (int s = 0; s < b.nb; ++s) nbd += b.path_h[s] != kPathQRJ;
-  k_bd_zfix<<<dim3((b.kk + 31) / 32, (b.nmax + 31) / 32, b.nb), 256, 0, h->stream>>>(b.slots_d, b.path_d, b.kk, b.cap);
+  k_bd_zfix<<<dim3((b.kk + 31) / 32, (b.nmax + 31) / 32, b.nb), 256, 0, h->stream>>>(b.slots_d, b.path_d, b.kk, b.cap,
+                                                                                               second);
   TEBD_LAUNCHED(h);
   constexpr size_t kSmemMax = 220 * 1024;
   int rc = check_cuda(h, cudaFuncSetAttribute(k_bd_orth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax),
@@ -382,21 +386,22 @@ int launch_bd_orth(tebd_handle *h, const BidiagBatch &b) {
   };
   // Enough CTAs to fill the GPU once, at least 64 rows each; more where shared memory
   // asks for it.
-  int C = 0;
-  for (int c = 1; c <= kMaxC; c *= 2)
+  int C = *clusters;
+  for (int c = 1; c <= kMaxC && !*clusters; c *= 2)
     if (fits(c) >= 1 && (C == 0 || (nbd * sides * c <= 152 && b.nmax >= 64 * c))) C = c;
   const TuneParams tp = tune_lookup(h, b.dfp ? 1 : 0, b.nmax, b.nb);
-  if (tp.orth_cluster > 0) {
+  if (tp.orth_cluster > 0 && !*clusters) {
     if (tp.orth_cluster <= kMaxC && fits(tp.orth_cluster) >= 1)
       C = tp.orth_cluster;
     else
       tune_reject(h);
   }
   if (C == 0) return set_error(h, TEBD_ERR_CUDA, "orthogonalisation: no cluster size fits");
+  *clusters = C;
   cfg.gridDim = dim3(sides * C, b.nb, 1);
   attr[0].val.clusterDim.x = C;
   cfg.dynamicSmemBytes = orth_smem(b.nmax, d_in_smem ? K : 0, C);
-  rc = check_cuda(h, cudaLaunchKernelEx(&cfg, k_bd_orth, b.slots_d, b.path_d, b.kk, b.cap, d_in_smem), "orthogonalisation launch");
+  rc = check_cuda(h, cudaLaunchKernelEx(&cfg, k_bd_orth, b.slots_d, b.path_d, b.kk, b.cap, d_in_smem, second), "orthogonalisation launch");
   TEBD_LAUNCHED(h);
   return rc;
 }

@@ -14,8 +14,8 @@
 //      eigenvalues are +-sigma), one thread per kept value, stopped at relative
 //      width 2 eps.
 //   3. Singular vectors of B: inverse iteration on the Golub-Kahan matrix shifted
-//      by sigma_i (tridiagonal LU with partial pivoting, 3 solves from a fixed
-//      start), eigenvector z = (v0,u0,v1,u1,...)/sqrt2; then (bdorth.cu)
+//      by sigma_i (tridiagonal LU with partial pivoting, two solves from a fixed
+//      start, one more for clusters), eigenvector z = (v0,u0,v1,u1,...)/sqrt2; then (bdorth.cu)
 //      the u's and the v's are each re-orthogonalised in descending sigma order.
 //   4. (bdapply.cu) U = Q [Ub; 0], V = P Vb by applying the reflectors in reverse, four at
 //      a time; X(:,i) = U(:,i) sigma_i, V(:,i), the same layout the sort and restore
@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "bidiag.cuh"
+#include "fixed.cuh"
 
 namespace tebd {
 
@@ -193,7 +194,16 @@ __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const i
 }
 
 // ---------------------------------------------------------------------------
-// 3a. inverse iteration on (T_GK - sigma_i I), one thread per value.
+// 3a. inverse iteration on (T_GK - sigma_i I), one thread per value: two solves.  Inside a
+// cluster the raw vectors are combinations of the cluster's, the same ones of the v's and of
+// the u's, but each set is re-orthogonalised by itself, and the two agree only to eps
+// times the raw vectors' condition (1e5 and more where rounding spreads a cluster over the
+// distance of the shift).  Problems with values within 64 ulps of the next
+// (bd_clustered) go through a second pass, one solve from the orthogonal vectors and the
+// re-orthogonalisation again, whose raw vectors are nearly orthogonal.  Theta rebuilt,
+// relative to its norm, before (rows of a cosine transform as starts, one pass) and now: 64
+// values in multiplets of 2 to 21, up to 1.5e-12 -> 5e-15; 256 equal values, 9e-13 -> 4e-14 and
+// in the double-float form 2e-8 -> 8e-14.
 // Scratch per value (transposed so that threads of a warp touch adjacent words):
 //   U0 (reciprocal pivots), U1, U2 (upper factor of the pivoted LU), PV (multipliers),
 //   Y (swap flags, ints), then the vector Z itself.
@@ -211,7 +221,7 @@ __device__ __forceinline__ double times_pow2(double x, int e) {  // x 2^e; 0 whe
   const int h = __double2hiint(x), f = ((h >> 20) & 0x7ff) + e;
   return f <= 0 || (h & 0x7ff00000) == 0 ? 0.0 : __hiloint2double(h + (e << 20), __double2loint(x));
 }
-__global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, int kk, int cap) {
+__global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, int kk, int cap, int second) {
   const int s = blockIdx.y;
   const int route = path[s];
   if (!on_route(route)) return;
@@ -224,6 +234,7 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
   const int i = min((int)(blockIdx.x * blockDim.x + threadIdx.x), K - 1);
   const bool mine = (int)(blockIdx.x * blockDim.x + threadIdx.x) < K;
   const double *dd = S.bdws, *ee = S.bdws + n, *sig = S.bdws + 2 * n;
+  if (second && !bd_clustered(sig, K)) return;  // uniform
   double *base = S.bdws + bd_scratch(n, kk);
   double *U0 = base, *U1 = base + (size_t)N * K, *U2 = base + 2 * (size_t)N * K, *PV = base + 3 * (size_t)N * K,
          *Z = base + 5 * (size_t)N * K;
@@ -255,10 +266,13 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
   // take over otherwise, and at 1/64 of the value, whose negative is an eigenvalue
   // too: with 64 ulps everywhere the left and right vectors of values below 1e-14 of the
   // largest were paired at random.  Other values are the shift themselves: a neighbour at a
-  // distance g leaves a share of (ulp / g)^3.
+  // distance g leaves a share of (ulp / g)^2, which costs Theta that share of g.
+  // The second pass (below) starts from orthogonal vectors: one solve, 16 ulps above.
   {
     const double ulp = 2.220446049250313e-16 * sig[0], near = 8.0 * ulp, own = lam;
-    if ((i > 0 && sig[i - 1] - own <= near) || (i + 1 < K && own - sig[i + 1] <= near)) {
+    if (second) {
+      lam = own + fmin(16.0 * ulp, 0.015625 * own);
+    } else if ((i > 0 && sig[i - 1] - own <= near) || (i + 1 < K && own - sig[i + 1] <= near)) {
       int j = i;  // the cluster's first value
       while (j > 0 && sig[j - 1] - sig[j] <= near) --j;
       double shift = fmin(64.0 * ulp, 0.015625 * own);
@@ -284,23 +298,21 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
     d1 = keep ? nd1 : -mult * nd1;
   }
   AT(U0, N - 1) = 1.0 / guard(d0);  // U0 holds the reciprocal pivots
-  // start vector: row i of the cosine transform with fixed pseudo-random signs on the v's,
-  // zero on the u's.  The rows are orthogonal, so that the starts of a cluster's members
-  // are as independent inside its eigenspace as they can be; of independent random
-  // vectors one in ten is close to a combination of the others.
-  for (int j = 0; j < n; ++j) {
-    unsigned x = (unsigned)(j + 1) * 0x9E3779B9u;  // a published integer hash (Wellons' lowbias32)
+  // start vector: pseudo-random entries in [-1, 1), independent for each value i and entry
+  // j (a published integer hash, Wellons' lowbias32, of both).  The vectors of a multiplet
+  // are local in B, and over a short window the starts have to be independent too:
+  // rows of a cosine transform with common signs are nearly parallel there.
+  for (int j = 0; j < N && !second; ++j) {
+    unsigned x = ((unsigned)j * 0x9E3779B9u) ^ ((unsigned)(i + 1) * 0x85EBCA6Bu);
     x ^= x >> 16;
     x *= 0x7feb352du;
     x ^= x >> 15;
     x *= 0x846ca68bu;
     x ^= x >> 16;
-    const float a = (float)(((long long)(2 * j + 1) * i) % (4 * n)) / (float)(2 * n);
-    AT(Z, 2 * j) = (double)(x & 1 ? cospif(a) : -cospif(a));
-    AT(Z, 2 * j + 1) = 0.0;
+    AT(Z, j) = (double)(int)x * 4.656612873077393e-10;
   }
   int scale = 0;  // the right-hand side is Z 2^scale
-  for (int it = 0; it < 3; ++it) {
+  for (int it = 0; it < (second ? 1 : 2); ++it) {
     // forward: the row operations (with swaps) applied to the right-hand side
     double carry = times_pow2(AT(Z, 0), scale);
     for (int j = 0; j < N - 1; j += kAhead) {
@@ -382,6 +394,36 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
       if (j + u < N) AT(Z, j + u) = times_pow2(z[u], scale) * inv;
   }
 #undef AT
+}
+
+// the orthogonal vectors (bdorth.cu) back into z, the starts of the second pass
+__global__ void __launch_bounds__(256) k_bd_zback(Slot *slots, const int *path, int kk, int cap) {
+  __shared__ double tile[2][32][33];
+  const int s = blockIdx.z;
+  const int route = path[s];
+  if (!on_route(route)) return;
+  const Slot S = slots[s];
+  int m, n;
+  bd_dims(*S.cp, route, m, n);
+  const int K = cap ? min(min(kk, n), S.cp->k) : min(kk, n);
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  if (i0 >= K || j0 >= n || !bd_clustered(S.bdws + 2 * n, K)) return;  // uniform
+  double *base = S.bdws + bd_scratch(n, kk), *Z = base + 5 * (size_t)(2 * n) * K;
+  const int2 *Zi = reinterpret_cast<const int2 *>(base);
+  const double unit = 2.168404344971009e-19;  // 2^-62
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int y = ty; y < 64; y += 8) {
+    const int p = y >> 5, i = i0 + (y & 31), j = j0 + tx;
+    if (j < n && i < K) {
+      const int2 z = Zi[((size_t)p * K + i) * n + j];
+      tile[p][tx][y & 31] = (double)dec(z.x, z.y) * unit;
+    }
+  }
+  __syncthreads();
+  for (int y = ty; y < 64; y += 8) {
+    const int j = j0 + (y >> 1), i = i0 + tx;
+    if (j < n && i < K) Z[(size_t)(2 * j + (y & 1)) * K + i] = tile[y & 1][y >> 1][tx];
+  }
 }
 
 // 3b. the v's (even rows) and u's (odd rows) re-orthogonalised: bdorth.cu
@@ -518,10 +560,17 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
     if ((rc = check_cuda(h, cudaFuncSetAttribute(k_bd_invit, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax),
                          "inverse iteration shared memory")))
       return rc;
-    k_bd_invit<<<dim3(cdiv(kk, 32), nb), 32, smem, st>>>(slots_d, path_d, kk, cap);
+    int clusters = 0;  // of k_bd_orth, the same in both passes
+    for (int second = 0; second < (b.right_only ? 1 : 2); ++second) {  // the second: problems with clustered values
+      if (second) {
+        k_bd_zback<<<dim3(cdiv(kk, 32), cdiv(nmax, 32), nb), 256, 0, st>>>(slots_d, path_d, kk, cap);
+        TEBD_LAUNCHED(h);
+      }
+      k_bd_invit<<<dim3(cdiv(kk, 32), nb), 32, smem, st>>>(slots_d, path_d, kk, cap, second);
+      TEBD_LAUNCHED(h);
+      if ((rc = launch_bd_orth(h, b, second, &clusters))) return rc;
+    }
   }
-  TEBD_LAUNCHED(h);
-  if ((rc = launch_bd_orth(h, b))) return rc;
   if ((rc = launch_bd_apply(h, b))) return rc;
   k_bd_store<<<dim3(256, nb), 256, 0, st>>>(slots_d, path_d, kk, cap, b.right_only);
   TEBD_LAUNCHED(h);

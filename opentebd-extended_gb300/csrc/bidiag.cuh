@@ -22,5 +22,14 @@ __host__ __device__ __forceinline__ size_t bd_scratch(int n, int kk) {
   return ((size_t)2 * n + (kk > n ? kk : n) + 1) & ~(size_t)1;
 }
 
+// Whether a value of the K kept ones lies within 64 ulps of the next, by a whole warp (values
+// below 64 ulps of the largest are left out: their vectors weigh as little).
+__device__ __forceinline__ bool bd_clustered(const double *sig, int K) {
+  const double near = 64.0 * 2.220446049250313e-16 * sig[0];
+  bool close = false;
+  for (int i = threadIdx.x & 31; i + 1 < K; i += 32) close |= sig[i] > near && sig[i] - sig[i + 1] <= near;
+  return __any_sync(0xffffffffu, close);
+}
+
 }  // namespace
 }  // namespace tebd

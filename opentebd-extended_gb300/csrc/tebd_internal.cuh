@@ -261,7 +261,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b);
 // the bidiagonalisation of the batch's slots (gebrd.cu) and its workspace in S.aux (complex elements)
 int launch_gebrd(tebd_handle *h, const BidiagBatch &b);
 size_t gebrd_aux_elems(int M, int N);
-int launch_bd_orth(tebd_handle *h, const BidiagBatch &b);   // the vectors' re-orthogonalisation (bdorth.cu)
+int launch_bd_orth(tebd_handle *h, const BidiagBatch &b, int second, int *clusters);  // the vectors' re-orthogonalisation (bdorth.cu)
 size_t bd_orth_ws_doubles(int K);
 int launch_bd_apply(tebd_handle *h, const BidiagBatch &b);  // the back-transformation (bdapply.cu)
 // Autotuner table (tune.cu): the shape for route (0 FP64 bidiagonal, 1
