@@ -71,9 +71,8 @@ extern "C" {
 #define TEBD_SVD_FP64 0           /* default: per bond, bidiagonalisation (in 64-bit fixed
                                      point; a wide Theta as Theta^H) when its batch holds
                                      a saturated bond (all chi of its Lambda in use) or
-                                     one above 384 columns -- below 64 columns only with
-                                     Schmidt values that span at most 1e-8 -- else
-                                     column-pivoted QR + one-sided Jacobi                */
+                                     one above 384 columns, for its bonds of 64 columns
+                                     or more; else column-pivoted QR + one-sided Jacobi  */
 #define TEBD_SVD_JACOBI 2         /* one-sided Jacobi on the whole (compacted) Theta    */
 #define TEBD_SVD_BIDIAG 3         /* bidiagonalisation for every Theta (>= 2 x 2)       */
 #define TEBD_SVD_QRJ 4            /* pivoted QR + Jacobi on R^H for every bond          */
@@ -272,9 +271,8 @@ int tebd_set_conserv(tebd_handle *h, const int *conserv);
 
 /* Singular values of the normalised Theta from the last update of `link`
  * (descending; NC mode: the flattened block values in the reference's order).
- * *count receives how many were written: all d*chi (zeros included) on the Jacobi
- * routes and for a default-route bond below 64 columns, the chi kept ones on the
- * bidiagonal route otherwise; the buffer holds d*chi. */
+ * *count receives how many were written: all d*chi (zeros included) on the
+ * Jacobi routes, the chi kept ones on the bidiagonal route; the buffer holds d*chi. */
 int tebd_get_singular_values(tebd_handle *h, int link, double *sigma, int *count);
 
 /* Jacobi sweeps used by the last update of `link` (diagnostics). */

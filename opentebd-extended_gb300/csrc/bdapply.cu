@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) k_bd_apply(Slot *slots, const 
   }
   // left -> Yu (scratch), right -> S.V (Theta route) or scratch (Theta^H route: z's, free by now)
   double2 *out = left ? reinterpret_cast<double2 *>(base + 6 * (size_t)(2 * n) * K) + (size_t)m * i
-                      : (transposed(route) ? reinterpret_cast<double2 *>(base + 10 * (size_t)n * K) : S.V) + (size_t)n * i;
+                      : (route == kPathBidiagT ? reinterpret_cast<double2 *>(base + 10 * (size_t)n * K) : S.V) + (size_t)n * i;
   const double unit = pow2(-62);
   for (int r = t0; r < len; r += step)
     out[r] = make_double2((double)(y[r].re - kOff) * unit, (double)(y[r].im - kOff) * unit);

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kSigmaThreads) k_bd_sigma(Slot *slots, const i
   const Slot S = slots[s];
   int m, n;
   bd_dims(*S.cp, route, m, n);
-  const int K = route & kPathAll ? n : min(kk, n);
+  const int K = min(kk, n);
   if ((int)(blockIdx.x * kSigmaValues) >= K) return;  // uniform per block
   const int n1 = 2 * n - 1;
   extern __shared__ double sq[];  // n1 scaled squared off-diagonals, then in FP32
@@ -442,14 +442,14 @@ __global__ void k_bd_store(Slot *slots, const int *path, int kk, int cap, int ri
   double *base = S.bdws + bd_scratch(N, kk);
   const double *sig = S.bdws + 2 * N;
   const double2 *Yu = reinterpret_cast<const double2 *>(base + 12 * (size_t)N * K);
-  const double2 *U = transposed(route) ? reinterpret_cast<const double2 *>(base + 10 * (size_t)N * K) : Yu;
+  const double2 *U = route == kPathBidiagT ? reinterpret_cast<const double2 *>(base + 10 * (size_t)N * K) : Yu;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; !right_only && e < (size_t)m * K; e += stride) {
     const int i = (int)(e / m);
     const double2 y = U[e];
     S.X[e] = make_double2(y.x * sig[i], y.y * sig[i]);
   }
-  if (transposed(route))
+  if (route == kPathBidiagT)
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)n * K; e += stride)
       S.V[e] = Yu[e];
   if (cap) {  // columns past the capped count read as zero singular values
@@ -464,7 +464,7 @@ __global__ void k_bd_store(Slot *slots, const int *path, int kk, int cap, int ri
 // then X <- V^H (n x m, ld n).
 __global__ void k_bd_stage(Slot *slots, const int *path) {
   const int s = blockIdx.y;
-  if (!transposed(path[s])) return;
+  if (path[s] != kPathBidiagT) return;
   const Slot S = slots[s];
   const size_t e_end = (size_t)S.cp->m * S.cp->n;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < e_end;
@@ -475,7 +475,7 @@ __global__ void k_bd_stage(Slot *slots, const int *path) {
 __global__ void k_bd_transpose(Slot *slots, const int *path) {
   __shared__ double2 tile[32][33];
   const int s = blockIdx.z;
-  if (!transposed(path[s])) return;
+  if (path[s] != kPathBidiagT) return;
   const Slot S = slots[s];
   const int m = S.cp->m, n = S.cp->n;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
@@ -516,7 +516,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
   if (b.phase != 2) {  // bidiagonalisation and singular values
   if (h->profiling) cudaEventRecord(h->ev[0], st);
   bool any_t = false;
-  for (int s = 0; s < nb; ++s) any_t |= transposed(b.path_h[s]);
+  for (int s = 0; s < nb; ++s) any_t |= b.path_h[s] == kPathBidiagT;
   if (any_t) {
     k_bd_stage<<<dim3(128, nb), 256, 0, st>>>(slots_d, path_d);
     TEBD_LAUNCHED(h);
@@ -548,9 +548,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
     if ((rc = check_cuda(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax),
                          "bisection shared memory")))
       return rc;
-    bool all = false;
-    for (int s = 0; s < nb; ++s) all |= (b.path_h[s] & kPathAll) != 0;
-    kern<<<dim3(cdiv(all ? std::max(kk, nmax) : kk, kSigmaThreads / team), nb), kSigmaThreads, smem, st>>>(slots_d, path_d, kk);
+    kern<<<dim3(cdiv(kk, kSigmaThreads / team), nb), kSigmaThreads, smem, st>>>(slots_d, path_d, kk);
   }
   TEBD_LAUNCHED(h);
   if (b.phase == 1) return check_cuda(h, cudaGetLastError(), "bidiag launch");

@@ -5,21 +5,20 @@
 namespace tebd {
 namespace {
 
-__device__ __forceinline__ bool on_route(int p) { return (p & 3) == kPathBidiag || (p & 3) == kPathBidiagT; }
-__host__ __device__ __forceinline__ bool transposed(int p) { return (p & 3) == kPathBidiagT; }
+__device__ __forceinline__ bool on_route(int p) { return p == kPathBidiag || p == kPathBidiagT; }
 
 // The matrix that is bidiagonalised, M x N with M >= N, in place in S.X (ld M):
 // Theta itself (m x n) or, on the transposed route, Theta^H (n x m).
 __device__ __forceinline__ void bd_dims(const Compact &cp, int p, int &M, int &N) {
-  M = transposed(p) ? cp.n : cp.m;
-  N = transposed(p) ? cp.m : cp.n;
+  M = p == kPathBidiagT ? cp.n : cp.m;
+  N = p == kPathBidiagT ? cp.m : cp.n;
 }
 
-// bdws layout of one bond (doubles): d (n), e (n), sigma (kk or n), then from an even
+// bdws layout of one bond (doubles): d (n), e (n), sigma (kk), then from an even
 // offset the inverse-iteration scratch U0, U1, U2, PV, Y (2n x K each), the
 // eigenvectors Z (2n x K) and the left vectors Yu (m x K complex, 16-byte aligned)
 __host__ __device__ __forceinline__ size_t bd_scratch(int n, int kk) {
-  return ((size_t)2 * n + (kk > n ? kk : n) + 1) & ~(size_t)1;
+  return ((size_t)2 * n + kk + 1) & ~(size_t)1;
 }
 
 // Whether a value of the K kept ones lies within 64 ulps of the next, by a whole warp (values

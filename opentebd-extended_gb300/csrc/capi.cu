@@ -585,48 +585,48 @@ static int run_batch(tebd_handle *h, int nb, const int *links, const double *con
       }
       // default routing: the bidiagonal route from 64 columns when the batch holds a
       // saturated bond (all chi of its Lambda in use: the gate fills Theta's spectrum,
-      // rank ~ n) or a bond beyond kQrjMaxDim; the batch's other bonds ride along in the
-      // same launches (the two routes of one batch run one after the other).  A batch of
-      // unsaturated Thetas up to kQrjMaxDim columns keeps the QR route: its cost follows
-      // the numerical rank, and its sweeps resolve the vectors of the smallest values to
-      // their own size.  The bidiagonal route leaves 1e-16 of the largest in every row of
-      // U, which the division by a small Lambda0 turns into Schmidt values above the
+      // rank ~ n) or a bond beyond kQrjMaxDim; the batch's other bonds from 64 columns on ride
+      // along in the same launches (the two routes of one batch run one after the other).  A
+      // batch of unsaturated Thetas up to kQrjMaxDim columns keeps the QR route: its cost
+      // follows the numerical rank, and its sweeps resolve the vectors of the smallest
+      // values to their own size.  The bidiagonal route leaves 1e-16 of the largest in every
+      // row of U, which the division by a small Lambda0 turns into Schmidt values above the
       // guard, and the chain fills up with them (the chi = 128 run's first 8 steps: 83 ms
       // against 740).  A batch that took the randomized route holds saturated bonds.
-      //
-      // Below 64 columns the same holds for a saturated bond (32 columns of rank 32: 1.30 ms
-      // by the QR route, 0.98 by the bidiagonal one), and a batch's other small bonds
-      // ride along, as long as a bond's values span no more than kBidiagSpan, well
-      // above that rounding.  These bonds still report all their values (kPathAll).
-      const int mode = h->opts.svd_mode;
-      const bool choose = mode != TEBD_SVD_BIDIAG && mode != TEBD_SVD_QRJ;
-      bool full_batch = nrs > 0, any_full = full_batch;
+      // Below 64 columns a saturated bond keeps the QR route too: the bidiagonal one takes
+      // 0.98 ms instead of 1.30 for 32 columns of rank 32, but Schmidt values down to 1e-6 of
+      // the largest come out to 1e-10 of their size instead of 1e-14, and rows of Gamma to
+      // 1e-11 instead of 1e-15, more where Lambda0 or Lambda2 spans more.
+      bool full_batch = nrs > 0;
       for (int s = 0; s < nb; ++s) {
         const int mn = std::min(cps[s].m, cps[s].n);
-        if (std::max(cps[s].m, cps[s].n) > kBidiagMaxDim) continue;
-        const bool full = cps[s].r1 >= h->chi;
-        if (mn >= kBidiagMinDim && (full || mn > kQrjMaxDim)) full_batch = true;
-        if (full && mn >= kBidiagSmallDim && cps[s].span >= kBidiagSpan) any_full = true;
+        if (mn >= kBidiagMinDim && std::max(cps[s].m, cps[s].n) <= kBidiagMaxDim &&
+            (cps[s].r1 >= h->chi || mn > kQrjMaxDim))
+          full_batch = true;
       }
-      any_full |= full_batch;
       for (int s = 0; s < nb; ++s) {
+        if (nrs && h->path_h[s] != kPathQRJ) {  // randomized route, or its fallback to the full SVD
+          if (h->path_h[s] != kPathRsvd) {
+            const int mn = std::min(cps[s].m, cps[s].n), mx = std::max(cps[s].m, cps[s].n);
+            ++nbd;
+            nbd_max = std::max(nbd_max, mx);
+            h->stats.gebrd_flops += 16.0 * mx * (double)mn * mn - 16.0 / 3.0 * (double)mn * mn * mn;
+          }
+          continue;
+        }
         const int mn = std::min(cps[s].m, cps[s].n), mx = std::max(cps[s].m, cps[s].n);
-        const bool done = nrs && h->path_h[s] == kPathRsvd;
-        if (done) continue;
-        const bool back = nrs && h->path_h[s] != kPathQRJ;  // the randomized route's fallback to the full SVD
-        const bool bd = back || (mx <= kBidiagMaxDim && mn >= 2 &&
-                                 (mode == TEBD_SVD_BIDIAG || (choose && mn >= kBidiagMinDim && full_batch)));
-        const bool small = !bd && choose && any_full && mx <= kBidiagMaxDim && mn >= 2 && cps[s].span >= kBidiagSpan;
-        h->path_h[s] = !(bd || small) ? kPathQRJ : cps[s].m >= cps[s].n ? kPathBidiag : kPathBidiagT;
-        if (small) h->path_h[s] |= kPathAll;
-        h->stats.bidiag_updates += bd;
-        if (bd || small) {
+        const bool bd = mx > kBidiagMaxDim                   ? false
+                        : h->opts.svd_mode == TEBD_SVD_BIDIAG ? mn >= 2
+                        : h->opts.svd_mode == TEBD_SVD_QRJ    ? false
+                                                              : mn >= kBidiagMinDim && full_batch;
+        h->path_h[s] = !bd ? kPathQRJ : (cps[s].m >= cps[s].n ? kPathBidiag : kPathBidiagT);
+        if (bd) {
           ++nbd;
           nbd_max = std::max(nbd_max, mx);
           h->stats.gebrd_flops += 16.0 * mx * (double)mn * mn - 16.0 / 3.0 * (double)mn * mn * mn;
         }
-        if (small) h->stats.rank_sum += mn;
       }
+      h->stats.bidiag_updates += nbd;
       CK(cudaMemcpyAsync(h->path_d, h->path_h.data(), sizeof(int) * nb, cudaMemcpyHostToDevice,
                          h->stream),
          "upload SVD routes");

@@ -419,7 +419,7 @@ __global__ void k_eye(Slot *slots) {
 // n_full - n dropped values are exact zeros.  One CTA per slot.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_sigma_sort(Slot *slots, const double *nrm, int n_full,
-                                                     int *status, const int *path) {
+                                                     int *status) {
   extern __shared__ double sig[];  // n
   const int s = blockIdx.x;
   const Compact cp = *slots[s].cp;
@@ -448,12 +448,9 @@ __global__ void __launch_bounds__(1024) k_sigma_sort(Slot *slots, const double *
     slots[s].perm[rank] = k;
     slots[s].S[rank] = v * inv;
   }
-  // values without vectors: those beyond chi, where every value is reported
-  const int more = path && (path[s] & kPathAll) ? min(m, cp.n) : n;
-  const double *rest = slots[s].bdws + 2 * min(m, cp.n);
   for (int k = n + threadIdx.x; k < n_full; k += blockDim.x) {
     slots[s].perm[k] = -1;
-    slots[s].S[k] = k < more ? rest[k] * inv : 0.0;
+    slots[s].S[k] = 0.0;
   }
 }
 
@@ -502,8 +499,8 @@ __global__ void k_store_spectrum(Slot *slots, const int *links, const int *sweep
   for (int k = threadIdx.x; k < n; k += blockDim.x)
     sig_link[(size_t)(link - 1) * n + k] = slots[s].S[k];
   if (threadIdx.x == 0) {
-    // the bidiagonal route computes only the kept values, unless flagged; the Jacobi routes all
-    sig_count[link - 1] = path[s] == kPathQRJ || (path[s] & kPathAll) ? n : slots[s].cp->k;
+    // the bidiagonal route computes only the kept values; the Jacobi routes all of them
+    sig_count[link - 1] = path[s] != kPathQRJ ? slots[s].cp->k : n;
     sweeps_link[link - 1] = sweeps[s];
   }
 }
@@ -640,7 +637,7 @@ int launch_eye(tebd_handle *h, int nb) {
 int launch_dense_finish(tebd_handle *h, int nb) {
   const int chi = h->chi, d = h->d, n = h->n;
   cudaStream_t st = h->stream;
-  k_sigma_sort<<<nb, 1024, sizeof(double) * n, st>>>(h->slots_d, h->nrm, n, h->status_d, h->path_d);
+  k_sigma_sort<<<nb, 1024, sizeof(double) * n, st>>>(h->slots_d, h->nrm, n, h->status_d);
   TEBD_LAUNCHED(h);
   k_lambda<<<nb, 32, sizeof(double) * chi, st>>>(h->slots_d, h->links_d, h->lam, h->truncerr_d, chi, nb,
                                         h->unnormalized ? 0.0 : h->rank_bound, h->status_d);
@@ -719,7 +716,7 @@ cudaError_t raw_dense_finish(cudaStream_t st, double2 *gam, double *lam, const i
                              Slot *slots_d, const double *nrm, double *truncerr, int *status, int chi,
                              int d) {
   const int n = chi * d;
-  k_sigma_sort<<<1, 1024, sizeof(double) * n, st>>>(slots_d, nrm, n, status, nullptr);
+  k_sigma_sort<<<1, 1024, sizeof(double) * n, st>>>(slots_d, nrm, n, status);
   k_lambda<<<1, 32, sizeof(double) * chi, st>>>(slots_d, links_d, lam, truncerr, chi, 1, 0.0, status);
   k_restore_gamma1<<<dim3(cdiv((size_t)n * chi, 256), 1), 256, 0, st>>>(gam, lam, links_d, slots_d,
                                                                        nrm, chi, d, status);

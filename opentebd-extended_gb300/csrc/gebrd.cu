@@ -45,8 +45,8 @@
 
 #include <algorithm>
 
-#include "bidiag.cuh"
 #include "fixed.cuh"
+#include "tebd_internal.cuh"
 
 namespace tebd {
 
@@ -666,13 +666,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_gebrd(Slot *slots, const int *p
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int route = path[blockIdx.y];
-  if (!on_route(route)) return;  // uniform per cluster
+  if (route != kPathBidiag && route != kPathBidiagT) return;  // uniform per cluster
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Ctx &x = ctx();
   if (tid == 0) {
     const Slot S = slots[blockIdx.y];
     Ctx &c = ctx();
-    bd_dims(*S.cp, route, c.M, c.N);
+    c.M = route == kPathBidiagT ? S.cp->n : S.cp->m;
+    c.N = route == kPathBidiagT ? S.cp->m : S.cp->n;
     c.Mp = up(c.M, 32);
     c.Np = up(c.N, 32);
     c.C = (int)cluster.num_blocks();

@@ -120,11 +120,8 @@ struct Slot {
 constexpr int kPathQRJ = 0;      // pivoted QR + one-sided Jacobi on R^H (qrj.cu)
 constexpr int kPathBidiag = 1;   // bidiagonalisation + bisection + inverse iteration (bidiag.cu)
 constexpr int kPathBidiagT = 2;  // the same on Theta^H, for a wide compacted Theta (m < n)
-constexpr int kPathAll = 4;      // added to a bidiagonal route: every singular value is reported, not only chi
 constexpr int kPathRsvd = 3;     // randomized sketch + Rayleigh-Ritz (rsvd.cu), full SVD as fallback
 constexpr int kBidiagMinDim = 64;  // default route switch: min(m, n) of the compacted Theta
-constexpr int kBidiagSmallDim = 8; // and of a saturated bond whose values span at most
-constexpr float kBidiagSpan = 1e-8f; // this (smallest / largest)
 constexpr int kQrjMaxDim = 384;    // a batch of unsaturated bonds up to this min(m, n) keeps the QR route
 
 // learned model (mlp.cu): sizes and the relative ranks k / chi of its outputs
