@@ -20,6 +20,7 @@
 //   4. (bdapply.cu) U = Q [Ub; 0], V = P Vb by applying the reflectors in reverse, four at
 //      a time; X(:,i) = U(:,i) sigma_i, V(:,i), the same layout the sort and restore
 //      kernels read from the Jacobi routes.
+//   5. (bdrows.cu) small rows of U and V from Theta, to their own size.
 // The values and the solves are FP64, everything else 64-bit fixed point, whose products the
 // integer pipe does 5 times faster.  Cost: 32/3 n^3 (bidiagonalisation) + 16 (m+n) n chi'
 // (back-transformation) instead of the Jacobi route's many O(n k^2) sweeps.
@@ -500,7 +501,7 @@ __global__ void k_bd_transpose(Slot *slots, const int *path) {
 // ---------------------------------------------------------------------------
 // host orchestration: bidiagonal route for the slots flagged kPathBidiag / kPathBidiagT
 // ---------------------------------------------------------------------------
-size_t bidiag_aux_elems(int n) { return gebrd_aux_elems(n, n); }
+size_t bidiag_aux_elems(int n) { return gebrd_aux_elems(n, n) + bd_rows_aux_elems(n, n); }
 
 size_t bidiag_ws_doubles(int n, int chi) {
   const int K = std::min(chi, n);
@@ -570,6 +571,7 @@ int run_bidiag_batch(tebd_handle *h, const BidiagBatch &b) {
     }
   }
   if ((rc = launch_bd_apply(h, b))) return rc;
+  if (!b.right_only && (rc = launch_bd_rows(h, b))) return rc;
   k_bd_store<<<dim3(256, nb), 256, 0, st>>>(slots_d, path_d, kk, cap, b.right_only);
   TEBD_LAUNCHED(h);
   if (h->profiling) {
@@ -601,7 +603,7 @@ int run_bidiag(tebd_handle *h, int nb, int nmax) {
 // (kk = the batch's largest N): aux, tau, taup (complex) and bdws (doubles).
 void bidiag_block_ws(int M, int N, int kk, size_t *aux_elems, size_t *bdws_doubles) {
   const int K = std::min(kk, N);
-  *aux_elems = gebrd_aux_elems(M, N);
+  *aux_elems = gebrd_aux_elems(M, N) + bd_rows_aux_elems(M, N);
   *bdws_doubles = bd_scratch(N, kk) + 6 * (size_t)(2 * N) * K + 2 * (size_t)M * K + bd_orth_ws_doubles(K) + 4;
 }
 

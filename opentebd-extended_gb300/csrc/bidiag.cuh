@@ -14,6 +14,14 @@ __device__ __forceinline__ void bd_dims(const Compact &cp, int p, int &M, int &N
   N = p == kPathBidiagT ? cp.m : cp.n;
 }
 
+// Where Theta's copy lies in S.aux, behind k_gebrd's workspace (units of 16 bytes): the
+// right reflectors, the fixed-point matrix, the panel's vectors, the current column and row,
+// the posted norms.
+__host__ __device__ __forceinline__ size_t bd_theta_at(int M, int N) {
+  const size_t Mp = (M + 31) / 32 * 32, Np = (N + 31) / 32 * 32;
+  return (size_t)N * N + Mp * Np + 17 * (Mp + Np) + 128;
+}
+
 // bdws layout of one bond (doubles): d (n), e (n), sigma (kk), then from an even
 // offset the inverse-iteration scratch U0, U1, U2, PV, Y (2n x K each), the
 // eigenvectors Z (2n x K) and the left vectors Yu (m x K complex, 16-byte aligned)

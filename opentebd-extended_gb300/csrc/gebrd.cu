@@ -45,8 +45,8 @@
 
 #include <algorithm>
 
+#include "bidiag.cuh"
 #include "fixed.cuh"
-#include "tebd_internal.cuh"
 
 namespace tebd {
 
@@ -155,11 +155,9 @@ __device__ __forceinline__ void split_pair(unsigned long long a, unsigned long l
 // Workspace of one problem, from S.aux (units of 16 bytes): U (N x N, read by the
 // back-transformation), the fixed-point matrix (ld Mp, Np columns), the panel's [V X]
 // (16 x ld Mp) and [Y U] (16 x ld Np), the raw current column and conjugated row, and
-// the squared norms posted per warp of the cluster.
-__host__ __device__ __forceinline__ size_t ws_elems(int M, int N) {
-  const size_t Mp = up(M, 32), Np = up(N, 32);
-  return (size_t)N * N + Mp * Np + 17 * (Mp + Np) + kThreads / 32 * kMaxC;
-}
+// the squared norms posted per warp of the cluster; with `keep` a copy of the matrix as it
+// was behind them (bd_theta_at), for bdrows.cu.
+static_assert(kThreads / 32 * kMaxC <= 128, "bd_theta_at");
 
 // The problem, in shared memory: held in registers it would push the loops' own values
 // into local memory.
@@ -662,18 +660,17 @@ __device__ __noinline__ double2 column_start(int q, int tid) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(kThreads, 1) k_gebrd(Slot *slots, const int *path) {
+__global__ void __launch_bounds__(kThreads, 1) k_gebrd(Slot *slots, const int *path, int keep) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int route = path[blockIdx.y];
-  if (route != kPathBidiag && route != kPathBidiagT) return;  // uniform per cluster
+  if (!on_route(route)) return;  // uniform per cluster
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Ctx &x = ctx();
   if (tid == 0) {
     const Slot S = slots[blockIdx.y];
     Ctx &c = ctx();
-    c.M = route == kPathBidiagT ? S.cp->n : S.cp->m;
-    c.N = route == kPathBidiagT ? S.cp->m : S.cp->n;
+    bd_dims(*S.cp, route, c.M, c.N);
     c.Mp = up(c.M, 32);
     c.Np = up(c.N, 32);
     c.C = (int)cluster.num_blocks();
@@ -731,10 +728,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_gebrd(Slot *slots, const int *p
     const int eA = norm_exponent(x.nl, x.nnorm, lane), sh62 = 62 - eA;
     if (tid == 0) ctx().eA = eA;
     const size_t totp = (size_t)x.Mp * x.Np;
+    double2 *copy = reinterpret_cast<double2 *>(x.Pv) + bd_theta_at(M, N);
     for (size_t e = x.rank * kThreads + tid; e < totp; e += (size_t)x.C * kThreads) {
       const int r = (int)(e % x.Mp), c = (int)(e / x.Mp);
       double2 a = make_double2(0.0, 0.0);
-      if (r < M && c < N) a = x.X[r + (size_t)M * c];
+      if (r < M && c < N) {
+        a = x.X[r + (size_t)M * c];
+        if (keep) copy[r + (size_t)M * c] = a;
+      }
       x.A[e] = enc2(to_fix(a.x, sh62), to_fix(a.y, sh62));
     }
   }
@@ -818,7 +819,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gebrd(Slot *slots, const int *p
   }
 }
 
-size_t gebrd_aux_elems(int M, int N) { return ws_elems(M, N); }
+size_t gebrd_aux_elems(int M, int N) { return bd_theta_at(M, N); }
 
 // k_gebrd on the batch's slots, the largest dimension nmax
 int launch_gebrd(tebd_handle *h, const BidiagBatch &b) {
@@ -876,7 +877,8 @@ int launch_gebrd(tebd_handle *h, const BidiagBatch &b) {
   cfg.gridDim = dim3(C, nb, 1);
   attr[0].val.clusterDim.x = C;
   cfg.dynamicSmemBytes = smem_bytes(nmax, C);
-  rc = check_cuda(h, cudaLaunchKernelEx(&cfg, k_gebrd, b.slots_d, b.path_d), "bidiagonalisation launch");
+  rc = check_cuda(h, cudaLaunchKernelEx(&cfg, k_gebrd, b.slots_d, b.path_d, (int)!b.right_only),
+                  "bidiagonalisation launch");
   TEBD_LAUNCHED(h);
   return rc;
 }

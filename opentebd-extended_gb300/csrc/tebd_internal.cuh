@@ -261,6 +261,8 @@ size_t gebrd_aux_elems(int M, int N);
 int launch_bd_orth(tebd_handle *h, const BidiagBatch &b, int second, int *clusters);  // the vectors' re-orthogonalisation (bdorth.cu)
 size_t bd_orth_ws_doubles(int K);
 int launch_bd_apply(tebd_handle *h, const BidiagBatch &b);  // the back-transformation (bdapply.cu)
+int launch_bd_rows(tebd_handle *h, const BidiagBatch &b);   // small rows to their own size (bdrows.cu)
+size_t bd_rows_aux_elems(int M, int N);
 // Autotuner table (tune.cu): the shape for route (0 FP64 bidiagonal, 1
 // double-float bidiagonal, 2 randomized-route Cholesky leaf, 3 its blocking),
 // largest dimension n and bonds nb; zeros where no entry exists.  tune_reject: the launch could not
