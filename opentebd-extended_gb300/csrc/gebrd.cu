@@ -166,7 +166,11 @@ struct Ctx {
   int4 *Pv;
   double *d, *e;
   int4 *A;             // fixed-point matrix
-  int4 *Li, *Ri;       // [V X], [Y U]: V, U in units of 2^-62, X, Y in units of 2^(eA - 58)
+  // [V X], [Y U]: V, U in units of 2^-62, X, Y in units of 2^(eA - 61): with |tau| |v| <= 2
+  // they are at most twice the matrix's norm, 2^62 units (coarser ones cost small singular
+  // values: 512 x 512 of norm 6.5, values below 0.01 off by 2.5e-15 in units of 2^(eA - 58),
+  // by 5e-16 now)
+  int4 *Li, *Ri;
   double2 *col, *row;
   double *nl, *nr;
   int M, N, Mp, Np, C, rank, ownR, ownC, nnorm, eA;
@@ -283,7 +287,7 @@ __device__ __noinline__ void left_products(int i, bool panel, int warp, int lane
       if (o < ownC && c < Np) {
         Acc acc;
         row_sum(acc, x.Ri + c, Np, 4 * (e & 3), 4 * (e & 3) + 4, vector_at(kRvec));
-        zp[(e & 3) * ownC + o] = acc.value<6>();
+        zp[(e & 3) * ownC + o] = acc.value<3>();
       }
     }
   }
@@ -327,7 +331,7 @@ __device__ __noinline__ void right_products(int i, int warp, int lane) {
       } else {
         Acc acc;
         row_sum(acc, x.Li + r, Mp, 4 * ch, 4 * ch + 4, vector_at(kRvec));
-        zp[ch * ownR + o] = acc.value<6>();
+        zp[ch * ownR + o] = acc.value<3>();
       }
     }
   }
@@ -346,7 +350,7 @@ __device__ __noinline__ void correct(bool left, int i, int warp, int lane) {
     if (o < own && r < lim) {
       Acc acc;
       row_sum(acc, P + r, lim, 4 * q, 4 * q + 4, vector_at(kSvec));
-      zq[q * own + o] = acc.value<6>();
+      zq[q * own + o] = acc.value<3>();
     }
   }
 }
@@ -463,8 +467,8 @@ __device__ __noinline__ void panel_update(int q, int warp, int lane) {
 #pragma unroll
                 for (int x = 0; x < 4; ++x)
                   if ((x < 2 ? ra : rb) < Mp) {
-                    av[x] = enc2(dec(av[x].x, av[x].y) - (tr[x] << 6) - ((lr[x] + 512) >> 10),
-                               dec(av[x].z, av[x].w) - (ti[x] << 6) - ((li[x] + 512) >> 10));
+                    av[x] = enc2(dec(av[x].x, av[x].y) - (tr[x] << 3) - ((lr[x] + 4096) >> 13),
+                               dec(av[x].z, av[x].w) - (ti[x] << 3) - ((li[x] + 4096) >> 13));
                   __stcg(&A[(x < 2 ? ra : rb) + (size_t)Mp * (cb * 8 + 2 * t + (x & 1))], av[x]);
                   }
               }
@@ -574,7 +578,7 @@ __device__ __noinline__ double2 finish_row(int i, int j, int4 ai, int tid) {
     if (j > 0) take_off(z, q, ownC, o);
     // u = q - tau (q + scz z) in units of 2^(eA - 62); y = q - u
     const double2 u = minus_reflected(q, z, tau, scz);
-    x.Ri[(size_t)x.Np * j + c] = enc2((q.x - to_fix(u.x, 0) + 8) >> 4, (q.y - to_fix(u.y, 0) + 8) >> 4);
+    x.Ri[(size_t)x.Np * j + c] = enc2((q.x - to_fix(u.x, 0) + 1) >> 1, (q.y - to_fix(u.y, 0) + 1) >> 1);
     const double2 us = make_double2(u.x * uA, u.y * uA);
     x.row[c] = us;
     if (o == oc + tid) mine = us;
@@ -608,7 +612,7 @@ __device__ __noinline__ double2 finish_column(int i, int j, bool next, int4 ai, 
     }
     take_off(w, q, ownR, o);
     const double2 a = minus_reflected(q, w, tau, scz);
-    x.Li[(size_t)x.Mp * (8 + j) + r] = enc2((q.x - to_fix(a.x, 0) + 8) >> 4, (q.y - to_fix(a.y, 0) + 8) >> 4);
+    x.Li[(size_t)x.Mp * (8 + j) + r] = enc2((q.x - to_fix(a.x, 0) + 1) >> 1, (q.y - to_fix(a.y, 0) + 1) >> 1);
     const double2 as = make_double2(a.x * uA, a.y * uA);
     x.col[r] = as;
     if (o == o0 + tid) mine = as;
