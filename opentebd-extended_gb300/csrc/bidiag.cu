@@ -252,7 +252,9 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
   for (int o = 16; o > 0; o >>= 1) tb = max(tb, __shfl_xor_sync(0xffffffffu, tb, o));
   if (!mine) return;
   double lam = sig[i];
-  if (lam <= 0.0) {  // an exactly zero value: FormLambda1 drops it, its vectors are zero
+  // an exactly zero value: FormLambda1 drops it, its vectors are zero; neither are there vectors
+  // of a non-finite B (reported by the norm check), whose solves would rescale at every step
+  if (lam <= 0.0 || tb >= 0x7ff0000000000000ull) {
     for (int j = 0; j < N; ++j) AT(Z, j) = 0.0;
     return;
   }
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(32) k_bd_invit(Slot *slots, const int *path, i
         if (j - u >= 0) {
           double x = fma(-u2[u], x2, fma(-u1[u], x1, z[u])) * u0[u];
           int f = (__double2hiint(x) >> 20) & 0x7ff;
-          if (f > 1023 + 500) {
+          if (f > 1023 + 500 && f != 0x7ff) {
             for (int q = j - u + 1; q < N; ++q) AT(Z, q) = times_pow2(AT(Z, q), -500);
             for (int q = 0; q < j - u; ++q) AT(Z, q) = times_pow2(AT(Z, q), -500);
 #pragma unroll
