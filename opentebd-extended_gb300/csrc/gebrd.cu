@@ -171,7 +171,7 @@ struct Ctx {
   // values: 512 x 512 of norm 6.5, values below 0.01 off by 2.5e-15 in units of 2^(eA - 58),
   // by 5e-16 now)
   int4 *Li, *Ri;
-  double2 *col, *row;
+  double2 *col, *row;  // in units of 2^eA, so that their squares stay in range
   double *nl, *nr;
   int M, N, Mp, Np, C, rank, ownR, ownC, nnorm, eA;
   int lf_at, zc_at, zp_at, npb;  // shared memory, in 16-byte units
@@ -514,12 +514,13 @@ __device__ __noinline__ void reflector(int which, double2 alpha, int ez, int i, 
   larfg(alpha, xn2, beta, tau, sc);
   if (lane == 0) {
     const double zs = pow2(ez + 1);  // the sums' unit 2^(eA + ez - 61) over A's 2^(eA - 62)
+    const double size = beta * pow2(x.eA);
     Scal &out = scal(which);
     out.tau = tau;
     out.sc = sc;
     out.scz = make_double2(sc.x * zs, sc.y * zs);
     if (x.rank == 0) {
-      (which ? x.e : x.d)[i] = beta;
+      (which ? x.e : x.d)[i] = size;
       (which ? x.taup : x.tau)[i] = tau;
     }
   }
@@ -562,7 +563,7 @@ __device__ __noinline__ double2 finish_row(int i, int j, int4 ai, int tid) {
   const int oc = first_own(i + 1, C, rank);
   const int parts = left_parts(x.Mp - ((i + 1) & ~31), (ownC >> 1) - (oc >> 1));
   const double2 tau = scal(0).tau, scz = scal(0).scz;
-  const double uA = pow2(x.eA - 62);
+  const double uA = pow2(-62);
   const longlong2 *zc = sums(x.zc_at);
   double acc = 0.0;
   double2 mine = make_double2(0.0, 0.0);
@@ -596,7 +597,7 @@ __device__ __noinline__ double2 finish_column(int i, int j, bool next, int4 ai, 
   const int o0 = first_own(i + 1, C, rank), kb = (i + 2) & ~31, groups = (ownR - (o0 & ~7) + 31) / 32;
   const int size = row_chunk_size(x.Np - kb, groups), chunks = (x.Np - kb + size - 1) / size;
   const double2 tau = scal(1).tau, scz = scal(1).scz;
-  const double uA = pow2(x.eA - 62);
+  const double uA = pow2(-62);
   const longlong2 *zc = sums(x.zc_at);
   double acc = 0.0;
   double2 mine = make_double2(0.0, 0.0);
@@ -646,7 +647,7 @@ __device__ __noinline__ void put_reflector(bool left, int i, int j, double2 mine
 __device__ __noinline__ double2 column_start(int q, int tid) {
   const Ctx &x = ctx();
   const int o0 = first_own(q, x.C, x.rank);
-  const double uA = pow2(x.eA - 62);
+  const double uA = pow2(-62);
   double acc = 0.0;
   double2 mine = make_double2(0.0, 0.0);
   for (int o = o0 + tid; o < x.ownR; o += kThreads) {
