@@ -354,11 +354,12 @@ __global__ void __launch_bounds__(128) k_gate_apply(Slot *slots, int chi, int d)
   }
 }
 
-// Opt k_gate_apply into the shared memory it needs on the current device (a
-// per-function attribute; cheap, made before every launch).
-static cudaError_t set_gate_smem(int d, bool df = false) {
+// Opt k_gate_apply into the shared memory it may need on the current device (a
+// per-function attribute; cheap, made before every launch).  One value for all d: the
+// attribute belongs to the process, and another thread's call may launch in between.
+static cudaError_t set_gate_smem(bool df = false) {
   return cudaFuncSetAttribute(df ? k_gate_apply<true> : k_gate_apply<false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gate_smem_bytes(d));
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gate_smem_bytes(kMaxD));
 }
 
 // ---------------------------------------------------------------------------
@@ -597,7 +598,7 @@ int launch_dense_prepare(tebd_handle *h, int nb, bool gate) {
     launch_theta_form(st, h->gam, h->lam, h->links_d, h->slots_d, chi, d, nb);
   TEBD_LAUNCHED(h);
   const bool gdf = h->opts.svd_mode == TEBD_SVD_DF || h->opts.svd_mode == TEBD_SVD_RSVD;
-  int rc = gate ? check_cuda(h, set_gate_smem(d, gdf), "gate shared memory") : TEBD_OK;
+  int rc = gate ? check_cuda(h, set_gate_smem(gdf), "gate shared memory") : TEBD_OK;
   if (rc) return rc;
   if (gate) {
     (gdf ? k_gate_apply<true> : k_gate_apply<false>)<<<dim3(cdiv((size_t)chi * chi, kGatePairs), nb), 128,
@@ -699,7 +700,7 @@ cudaError_t raw_dense_prepare(cudaStream_t st, double2 *gam, const double *lam, 
   const int n = chi * d;
   k_compact<<<1, 96, 0, st>>>(lam, links_d, slots_d, jp, chi, d);
   launch_theta_form(st, gam, lam, links_d, slots_d, chi, d, 1);
-  cudaError_t e = set_gate_smem(d);
+  cudaError_t e = set_gate_smem();
   if (e != cudaSuccess) return e;
   k_gate_apply<false><<<dim3(cdiv((size_t)chi * chi, kGatePairs), 1), 128, gate_smem_bytes(d), st>>>(
       slots_d, chi, d);

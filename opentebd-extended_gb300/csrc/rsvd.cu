@@ -640,7 +640,8 @@ int run_rsvd(tebd_handle *h, int nb, const std::vector<Compact> &cps, std::vecto
         tune_reject(h);
     }
     const size_t smem = sizeof(float4) * (size_t)PB * ss;
-    int e2 = check_cuda(h, cudaFuncSetAttribute(k_rs_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    // one limit for all widths: another thread's call may launch in between
+    int e2 = check_cuda(h, cudaFuncSetAttribute(k_rs_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024),
                         "Cholesky shared memory");
     if (e2) return e2;
     // cluster size: the SMs shared out among the bonds on the route (at most 8),

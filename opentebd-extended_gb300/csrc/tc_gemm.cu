@@ -327,7 +327,8 @@ cudaError_t tc_gemm_launch(const TcBatch &b, int *err_d, cudaStream_t st) {
       !make_map(&mb, b.b_planes, b.k_pad, b.n_pad, planes * b.nprob, kTcBN))
     return cudaErrorInvalidValue;
   const size_t smem = smem_bytes(planes);
-  cudaError_t e = cudaFuncSetAttribute(k_tc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // one limit for both forms: another thread's call may launch in between
+  cudaError_t e = cudaFuncSetAttribute(k_tc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(2));
   if (e != cudaSuccess) return e;
   dim3 grid(b.m_pad / kTcBM, b.n_pad / kTcBN, b.nprob);
   k_tc_gemm<<<grid, kThreads, smem, st>>>(ma, mb, b, err_d);
