@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restric
 }  // namespace
 
 // Theta of the batch on the tensor cores; returns -1 (nothing launched) when a
-// dimension of the batch is zero, so that the caller forms it on the CUDA cores.
+// dimension of the batch is zero, the product is small or the default form has no memory for
+// the digit planes, so that the caller forms it on the CUDA cores.
 // The default form (0) takes this path for large products: 8 planes hold 56 bits below
 // each row's and column's largest magnitude, so that the error of a sum of r1 products,
 // about 2^-56 sqrt(r1) of the largest, is below FP64's own (640 x 128 x 640: 3e-17
@@ -210,17 +211,6 @@ int launch_theta_tc(tebd_handle *h, int nb) {
   if (m_max == 0 || n_max == 0 || r1_max == 0 || (double)m_max * n_max * r1_max < kThetaTcMin) return -1;
   const Slot &s0 = h->slots[0];
   const long long aux_stride = nb > 1 ? (long long)(h->slots[1].aux - s0.aux) : 0;
-  const size_t total = (size_t)m_max * r1_max + (size_t)r1_max * n_max;
-  unsigned gx = (unsigned)std::min<size_t>((total + 255) / 256, 2048);
-  if (!h->theta_form) {
-    k_theta_balance<<<dim3((r1_max + 7) / 8, nb), 256, 0, h->stream>>>(h->gam, h->lam, h->links_d, h->slots_d, h->chi,
-                                                                      h->d);
-    TEBD_LAUNCHED(h);
-  }
-  k_theta_operands<<<dim3(gx, nb), 256, 0, h->stream>>>(h->gam, h->lam, h->links_d, h->slots_d, h->chi, h->d,
-                                                         m_max, r1_max, n_max,
-                                                         h->theta_form ? nullptr : h->status_d);
-  TEBD_LAUNCHED(h);
   ZProd z = {};
   z.a = s0.aux;
   z.a_stride = aux_stride;
@@ -241,7 +231,19 @@ int launch_theta_tc(tebd_handle *h, int nb) {
   z.alpha = 1.0;
   z.optr = reinterpret_cast<const unsigned char *>(h->slots_d) + offsetof(Slot, X);
   z.optr_stride = (int)sizeof(Slot);
-  if ((rc = tc_reserve(h, zprod_ws_bytes(z)))) return rc;
+  if ((rc = tc_reserve(h, zprod_ws_bytes(z))))
+    return h->theta_form || rc != TEBD_ERR_OOM ? rc : -1;  // the default form does without the digit planes
+  const size_t total = (size_t)m_max * r1_max + (size_t)r1_max * n_max;
+  unsigned gx = (unsigned)std::min<size_t>((total + 255) / 256, 2048);
+  if (!h->theta_form) {
+    k_theta_balance<<<dim3((r1_max + 7) / 8, nb), 256, 0, h->stream>>>(h->gam, h->lam, h->links_d, h->slots_d, h->chi,
+                                                                      h->d);
+    TEBD_LAUNCHED(h);
+  }
+  k_theta_operands<<<dim3(gx, nb), 256, 0, h->stream>>>(h->gam, h->lam, h->links_d, h->slots_d, h->chi, h->d,
+                                                         m_max, r1_max, n_max,
+                                                         h->theta_form ? nullptr : h->status_d);
+  TEBD_LAUNCHED(h);
   tc_events(h, zprod_mma_flops(z, nb), &z.ev0, &z.ev1);
   if ((rc = check_cuda(h, zprod_run(z, h->tc_ws, h->tc_err, h->stream), "tensor-core Theta"))) return rc;
   h->launches += zprod_oz(z.form) ? 5 : 3;  // packs (+ exponent passes) and the product
