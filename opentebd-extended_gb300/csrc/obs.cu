@@ -46,7 +46,7 @@ template <int kD>
 __global__ void __launch_bounds__(kObsThreads) k_obs_rho1(const double2 *gam, const double *lam, double2 *part,
                                                           int chi, int cols) {
   constexpr int kPairs = kD * (kD + 1) / 2;
-  const int s = blockIdx.y, b0 = blockIdx.x * cols, b1 = min(chi, b0 + cols);
+  const int s = blockIdx.x, b0 = blockIdx.y * cols, b1 = min(chi, b0 + cols);
   const double2 *G = gam + (size_t)s * chi * kD * chi;
   const double *l0 = lam + (size_t)s * chi, *l1 = lam + (size_t)(s + 1) * chi;
   double2 acc[kPairs];
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kObsThreads) k_obs_rho1(const double2 *gam, co
       v.x += red[w][threadIdx.x].x;
       v.y += red[w][threadIdx.x].y;
     }
-    part[((size_t)s * gridDim.x + blockIdx.x) * kPairs + threadIdx.x] = v;
+    part[((size_t)s * gridDim.y + blockIdx.y) * kPairs + threadIdx.x] = v;
   }
 }
 
@@ -416,7 +416,7 @@ extern "C" int tebd_single_site_rho(tebd_handle *h, double *rho) {
   double2 *rho_d = reinterpret_cast<double2 *>(h->obs_buf);
   double2 *part = rho_d + d2 * h->L;
   const int cols = (int)cdiv(h->chi, kRho1Parts), nparts = (int)cdiv(h->chi, cols);
-  auto rho1 = [&](auto kern) { kern<<<dim3(nparts, h->L), kObsThreads, 0, h->stream>>>(h->gam, h->lam, part, h->chi, cols); };
+  auto rho1 = [&](auto kern) { kern<<<dim3(h->L, nparts), kObsThreads, 0, h->stream>>>(h->gam, h->lam, part, h->chi, cols); };
   switch (h->d) {
     case 1: rho1(k_obs_rho1<1>); break;
     case 2: rho1(k_obs_rho1<2>); break;
