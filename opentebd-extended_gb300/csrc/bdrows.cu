@@ -236,10 +236,10 @@ __global__ void __launch_bounds__(256, 2) k_bd_rows(Slot *slots, const int *path
 
 // 2. T of both sets (side 0: V, 1: U)
 __global__ void __launch_bounds__(256, 2) k_bd_gram(Slot *slots, const int *path, int kk, int cap) {
-  const int s = blockIdx.z >> 1, side = blockIdx.z & 1;
+  const int s = blockIdx.z, side = blockIdx.x & 1;
   Vectors w;
   if (!w.load(slots[s], path[s], kk, cap)) return;
-  const int r0 = blockIdx.x * kTR, i0 = blockIdx.y * kTC, tid = threadIdx.x;
+  const int r0 = (blockIdx.x >> 1) * kTR, i0 = blockIdx.y * kTC, tid = threadIdx.x;
   if (r0 >= w.K || i0 >= w.K || r0 >= i0 + kTC || !w.graded()) return;  // uniform
   const double2 *x = side ? w.u : w.v;
   const int len = side ? w.M : w.N;
@@ -322,8 +322,8 @@ int launch_bd_rows(tebd_handle *h, const BidiagBatch &b) {
         b.slots_d, b.path_d, b.kk, b.cap, left);
     TEBD_LAUNCHED(h);
   }
-  k_bd_gram<<<dim3((b.kk + kTR - 1) / kTR, (b.kk + kTC - 1) / kTC, 2 * b.nb), 256, 0, h->stream>>>(b.slots_d, b.path_d,
-                                                                                               b.kk, b.cap);
+  k_bd_gram<<<dim3(2 * ((b.kk + kTR - 1) / kTR), (b.kk + kTC - 1) / kTC, b.nb), 256, 0, h->stream>>>(
+      b.slots_d, b.path_d, b.kk, b.cap);
   TEBD_LAUNCHED(h);
   k_bd_orthonormal<<<dim3((b.nmax + kFR - 1) / kFR, b.nb, 2), 256, 0, h->stream>>>(b.slots_d, b.path_d, b.kk, b.cap);
   TEBD_LAUNCHED(h);
