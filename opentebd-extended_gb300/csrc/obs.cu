@@ -134,7 +134,9 @@ __global__ void __launch_bounds__(kObsThreads) k_obs_rho2(const Slot *slots, dou
       row[u] = r;
       col[u] = r + q;
     }
-    const bool two = p0 + kObsThreads < pairs;
+    // of a warp: whether it has pairs at all (small d leaves most without, and the FP64 pipe free)
+    const int w0 = p0 + (threadIdx.x & ~31);
+    const bool one = w0 < pairs, two = w0 + kObsThreads < pairs;
     for (int e = e0; e < e1; e += kRhoE) {
       const int ne = min(kRhoE, e1 - e);
       __syncthreads();
@@ -149,7 +151,7 @@ __global__ void __launch_bounds__(kObsThreads) k_obs_rho2(const Slot *slots, dou
       }
       __syncthreads();
       for (int x = 0; x < ne; ++x) {
-        cacc(acc[0], th[x * d2 + row[0]], th[x * d2 + col[0]], 1.0);
+        if (one) cacc(acc[0], th[x * d2 + row[0]], th[x * d2 + col[0]], 1.0);
         if (two) cacc(acc[1], th[x * d2 + row[1]], th[x * d2 + col[1]], 1.0);
       }
     }
@@ -319,7 +321,9 @@ __global__ void k_obs_unit(double2 *E, int chi, double *e1) {  // E = e1 e1^T, e
 // for each of the two chains of an overlap, transfer matrices E, E' (chi^2 each) and T
 // (chi x d chi) with a unit vector (chi doubles), or the entropies (L+1).
 constexpr int kRho1Parts = 32;  // CTAs per site, per bond
-constexpr int kRho2Parts = 10;
+constexpr int kRho2Parts = 10;  // of a batch of 16 bonds or more; fewer bonds share out kRho2All
+constexpr int kRho2All = 152;
+static size_t rho2_parts(const tebd_handle *h) { return std::max(kRho2Parts * h->nslots, kRho2All); }
 static int obs_ws(tebd_handle *h, size_t bytes) {
   if (h->obs_bytes >= bytes) return TEBD_OK;
   cudaFree(h->obs_buf);
@@ -335,7 +339,7 @@ static int obs_begin(tebd_handle *h) {
   if (rc) return rc;
   const size_t n = (size_t)h->chi, d2 = (size_t)h->d * h->d;
   const size_t need = sizeof(double2) * std::max({(size_t)h->L * (d2 + kRho1Parts * d2),
-                                                  (size_t)h->nslots * (d2 * d2 + kRho2Parts * d2 * (d2 + 1) / 2),
+                                                  (size_t)h->nslots * d2 * d2 + rho2_parts(h) * d2 * (d2 + 1) / 2,
                                                   2 * (2 * n * n + n * h->d * n) + 1}) +
                       sizeof(double) * (n + h->L + 1) + 1024;
   return obs_ws(h, need);
@@ -374,7 +378,10 @@ static int obs_rho2(tebd_handle *h, const std::vector<int> &links, std::vector<d
       return rc;
     if ((rc = launch_dense_prepare(h, nb, false))) return rc;
     double2 *part = rho2_d + (size_t)h->nslots * d4;
-    const int nparts = std::max(1, std::min(kRho2Parts, 304 / nb));  // two CTAs per SM
+    // two CTAs per SM in a large batch, one in a small one (10 for a single bond of d = 3,
+    // chi = 200 took 2.1 ms, 0.34 now); at least two stages of pairs each
+    const int most = (int)cdiv((size_t)h->chi * h->chi, 2 * kRhoE);
+    const int nparts = std::max(1, std::min(most, std::max(std::min(kRho2Parts, 304 / nb), kRho2All / nb)));
     k_obs_rho2<<<dim3(nparts, nb), kObsThreads, sizeof(double2) * kRhoE * d2, h->stream>>>(h->slots_d, part, d);
     TEBD_LAUNCHED(h);
     k_obs_rho2_sum<<<dim3(cdiv(d4, kObsThreads), nb), kObsThreads, 0, h->stream>>>(h->slots_d, part, rho2_d, d, nparts);
