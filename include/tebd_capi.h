@@ -246,8 +246,10 @@ int tebd_set_rsvd_model(tebd_handle *h, tebd_mlp *m, double target);
 /* Theta formation (FormTheta, local_operations_module.f90:184-211) on the tensor
  * cores (no counterpart in the reference, which forms Theta in FP64 loops).
  * form 0, the default: CUDA cores (FP64, or double-float with TEBD_SVD_DF) for small
- * products, eight digit planes with balanced operands (at least FP64's accuracy) for
- * dense ones of 2^21 multiply-adds or more; 3:
+ * products, eight digit planes with balanced operands for dense ones of 2^21
+ * multiply-adds or more (error about 2^-56 of a row's largest factor times a column's
+ * per term, below FP64's where these meet in one product; an entry that is small because
+ * its row's and its column's large factors do not meet keeps that absolute error); 3:
  * 3xTF32 split-precision product with FP32 accumulation (~FP32 accuracy; the
  * precision tier's Theta; dense handles only); 100 + S, S = 3..7: S bf16 digit
  * planes (error ~2^(-7S) of the largest terms; S = 7 is FP64 class).  On

@@ -2,9 +2,9 @@
 // computing only the chi singular triplets the update keeps.
 //
 // Replaces SVDTruncation's ZGESVD('A','A') (local_operations_module.f90:322-345)
-// for bonds whose compacted Theta is m x n with m >= n >= max(256, 2 chi') (the
-// saturated regime, where the rank k approaches n and the Jacobi route's
-// O(n k^2)-per-sweep cost dominates).  FormLambda1/FormGamma1/FormGamma2 read
+// for bonds of 64 columns or more in a batch that holds a saturated one (where the rank
+// approaches n and the QR route's sweeps, O(k^3) each, dominate) or one above 384 columns, and
+// for the number-conserving update's blocks of 16 or more.  FormLambda1/FormGamma1/FormGamma2 read
 // only the first chi singular values and vectors, so only those are computed:
 //   1. (gebrd.cu) ZGEBD2 semantics: Q^H Theta P = B, B real upper bidiagonal (ZLARFG
 //      makes beta real), left reflectors H(i) = I - tauq v v^H below the diagonal,

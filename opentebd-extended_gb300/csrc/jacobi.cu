@@ -11,15 +11,14 @@
 //
 // Parallel schedule.  A sweep visits every column pair once in npad-1 rounds
 // of npad/2 disjoint pairs (round-robin "circle" tournament, npad = n rounded
-// up to even).  One kernel launch per round: every warp of the grid owns one
-// pair of one problem, so all pairs of all batched problems rotate concurrently
-// and the launch boundary is the only synchronisation.  Matrices stay in HBM
-// and are streamed through L2 (cfg: n <= 3072).
+// up to even).  One persistent launch runs all sweeps of a batch: a cluster of CTAs per
+// problem, a warp per pair, a cluster barrier between rounds; matrices are read through
+// L2.  The allocation-free entry point makes one launch per round instead, every warp of
+// the grid with one pair.
 //
 // Convergence.  A pair is rotated when |a^H b| > tol*|a||b|; a sweep without a
 // rotation ends the problem.  A problem that exceeds the sweep cap reports
-// TEBD_ERR_SVD_NOCONV.  Every wait is a host-side loop over bounded launches:
-// no kernel spins.
+// TEBD_ERR_SVD_NOCONV.  The loops are bounded by the cap: no kernel spins.
 #include <cooperative_groups.h>
 #include <math.h>
 

@@ -109,9 +109,10 @@ struct Slot {
   // QR-preconditioned SVD (qrj.cu)
   int *jpvt;                // n column permutation of the pivoted QR
   double2 *tau;             // n reflector scalars
-  double *vn;               // 2n partial column norms (later: the k singular values)
-  double2 *aux;             // 3 n^2: A = R^H (n x k), Z (k x k), Y = Q [Z; 0] (m x k);
-                            // bidiagonal path: right reflectors (n x n), partial sums
+  double *vn;               // 2n: Theta's balance, later the QR path's k singular values
+  double2 *aux;             // QR path, 3 n^2: A = R^H (n x k), Q2's reflectors, Z (k x k);
+                            // bidiagonal path: right reflectors (n x n), the fixed-point
+                            // matrix, the panel, a copy of Theta
   double2 *taup;            // n right-reflector scalars (bidiagonal path)
   double *bdws;             // bidiagonal path: d, e, sigma, inverse-iteration scratch, Z, U
 };

@@ -190,8 +190,10 @@ __global__ void __launch_bounds__(256) k_theta_operands(const double2 *__restric
 // the digit planes, so that the caller forms it on the CUDA cores.
 // The default form (0) takes this path for large products: 8 planes hold 56 bits below
 // each row's and column's largest magnitude, so that the error of a sum of r1 products,
-// about 2^-56 sqrt(r1) of the largest, is below FP64's own (640 x 128 x 640: 3e-17
-// against 1e-16 of the row and column maxima).  The CUDA cores' kernel is bound by the
+// about 2^-56 sqrt(r1) of the product of the two, is below FP64's own (640 x 128 x 640:
+// 3e-17 against 1e-16 of the row and column maxima).  It is normwise per row and column:
+// where a row's and a column's large factors lie at different inner indices the entry is
+// small and FP64 would keep it to its own size.  The CUDA cores' kernel is bound by the
 // FP64 pipe: 32 bonds of 640 x 640 (chi = 128) took 11.5 ms, 1.1 ms now, packs included.
 int launch_theta_tc(tebd_handle *h, int nb) {
   int rc;
