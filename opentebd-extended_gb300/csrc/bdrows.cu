@@ -14,7 +14,9 @@
 //      sigma_i, which step 1 mixes into single rows (1e-12 for values of 1e-8).  Each set
 //      is made orthonormal again: with G = U^H U, U <- U (I - T), T the part of G - I above
 //      the diagonal and half of it, vectors of larger values first; the square of G - I is
-//      below eps.  A row stays as accurate as it was: its larger entries lie at smaller
+//      below eps.  G(k, i), k < i, is off by eps sigma_0 / sigma_k at most, and only if step 1
+//      changed column k: T's rows k from 2^-8 sigma_0 down to the smallest row of Theta
+//      are formed.  A row stays as accurate as it was: its larger entries lie at smaller
 //      sigma_i, later in the order.
 // Below 2^-26 of the largest value, where that square would not be small, a row is replaced
 // only if the change is below eps: norm sigma_0 <= sigma_i^2.  The values keep the bisection's
@@ -132,9 +134,31 @@ struct Vectors {
     t = reinterpret_cast<double2 *>(base);
     return true;
   }
-  // whether step 2 has anything to do: down to 2^-14 of the largest value the rotations (1e-12 at
-  // 1e-8, in proportion) stay within a few eps
-  __device__ __forceinline__ bool graded() const { return sig[K - 1] < 6.103515625e-05 * sig[0]; }
+  // rows [ka, kb) of T, by the whole CTA: values below 2^-8 of the largest, down to the smallest
+  // norm of a line (side 1: row, 0: column) that is not zero
+  __device__ __forceinline__ void tail(const Slot &S, int side, int &ka, int &kb) const {
+    __shared__ int first[2];
+    __shared__ unsigned long long least;
+    if (threadIdx.x < 2) first[threadIdx.x] = K;
+    if (threadIdx.x == 0) least = ~0ull;
+    __syncthreads();
+    const Line *lines = lines_of(S, bd_theta_at(M, N), M, N, side);
+    unsigned long long low = ~0ull;
+    for (int l = threadIdx.x; l < (side ? M : N); l += blockDim.x) {
+      const double v = lines[l].norm;
+      if (v > 0.0) low = min(low, (unsigned long long)__double_as_longlong(v));
+    }
+    atomicMin(&least, low);
+    __syncthreads();
+    const double a = 0.00390625 * sig[0], b = __longlong_as_double((long long)least);
+    for (int i = threadIdx.x; i < K; i += blockDim.x) {
+      if (sig[i] < a) atomicMin(&first[0], i);
+      if (!(sig[i] >= b)) atomicMin(&first[1], i);
+    }
+    __syncthreads();
+    ka = first[0];
+    kb = first[1];
+  }
 };
 
 using Tile = Acc[4][2];  // rows tid % 16 + 16 q, vectors tid / 16 + 16 p
@@ -240,7 +264,10 @@ __global__ void __launch_bounds__(256, 2) k_bd_gram(Slot *slots, const int *path
   Vectors w;
   if (!w.load(slots[s], path[s], kk, cap)) return;
   const int r0 = (blockIdx.x >> 1) * kTR, i0 = blockIdx.y * kTC, tid = threadIdx.x;
-  if (r0 >= w.K || i0 >= w.K || r0 >= i0 + kTC || !w.graded()) return;  // uniform
+  if (r0 >= w.K || i0 >= w.K || r0 >= i0 + kTC) return;  // uniform
+  int ka, kb;
+  w.tail(slots[s], side, ka, kb);
+  if (r0 >= kb || r0 + kTR <= ka) return;  // uniform
   const double2 *x = side ? w.u : w.v;
   const int len = side ? w.M : w.N;
   __shared__ int ex[kTR];
@@ -255,7 +282,7 @@ __global__ void __launch_bounds__(256, 2) k_bd_gram(Slot *slots, const int *path
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int r = r0 + (tid & 15) + 16 * q, i = i0 + (tid >> 4) + 16 * p;
-      if (r > i || i >= w.K) continue;
+      if (r > i || i >= w.K || r < ka || r >= kb) continue;
       const longlong2 z = acc[q][p].value<1>();
       double2 t = make_double2((double)z.x * unit, (double)z.y * unit);
       if (r == i) t = make_double2(z.x ? 0.5 * (double)(z.x - (1ll << 61)) * unit : 0.0, 0.0);  // a zero vector stays
@@ -271,18 +298,20 @@ __global__ void __launch_bounds__(256) k_bd_orthonormal(Slot *slots, const int *
   Vectors w;
   if (!w.load(slots[s], path[s], kk, cap)) return;
   const int lim = side ? w.M : w.N, r0 = blockIdx.x * kFR, tid = threadIdx.x;
-  if (r0 >= lim || !w.graded()) return;  // uniform
+  if (r0 >= lim) return;  // uniform
+  int ka, kb;
+  w.tail(slots[s], side, ka, kb);
   double2 *x = side ? w.u : w.v;
   const double2 *T = w.t + (size_t)side * w.K * w.K;
   __shared__ float2 Us[kFC][kFR + 1], Ts[kFC][kFC + 1];
   const int r = tid & 31, c = tid >> 5;  // row; vectors c + 8 q
-  for (int i0 = (w.K - 1) / kFC * kFC; i0 >= 0; i0 -= kFC) {
+  for (int i0 = ka < kb ? (w.K - 1) / kFC * kFC : -1; i0 >= ka / kFC * kFC; i0 -= kFC) {
     float re[4] = {0.f, 0.f, 0.f, 0.f}, im[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k0 = 0; k0 <= i0; k0 += kFC) {
+    for (int k0 = ka / kFC * kFC; k0 <= i0 && k0 < kb; k0 += kFC) {
       for (int q = c; q < kFC; q += 8) {
         double2 a = make_double2(0.0, 0.0), t = a;
         if (r0 + r < lim && k0 + q < w.K) a = x[r0 + r + (size_t)lim * (k0 + q)];
-        if (k0 + r <= i0 + q && i0 + q < w.K) t = T[k0 + r + (size_t)w.K * (i0 + q)];
+        if (k0 + r >= ka && k0 + r < kb && k0 + r <= i0 + q && i0 + q < w.K) t = T[k0 + r + (size_t)w.K * (i0 + q)];
         Us[q][r] = make_float2((float)a.x, (float)a.y);
         Ts[q][r] = make_float2((float)t.x, (float)t.y);
       }
