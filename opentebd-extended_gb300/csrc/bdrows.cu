@@ -27,8 +27,8 @@
 // per k hide 10 shared-memory wavefronts, so that the integer pipe bounds it.  Tiles without
 // a row small enough for their values return at once.  Measured: rows of Gamma1 Lambda1
 // against extended precision, Lambdas down to 1e-8 (1e-4), 320 x 320: 1e-8 -> 3e-15 (2e-12 ->
-// 3e-15); 80 x 80: 8e-9 -> 6e-13 (1e-12 -> 3e-15).  32 bonds of 640 x 640, 128 vectors: 2.8 ms
-// beside 65; 10 of 270 x 270, 90 vectors: 0.3 beside 4.5.
+// 3e-15); 80 x 80: 8e-9 -> 6e-13 (1e-12 -> 3e-15).  32 bonds of 640 x 640, 128 vectors: 3.1 ms
+// beside 65; 10 of 270 x 270, 90 vectors: 0.7 beside 8.2.
 #include <algorithm>
 
 #include "bidiag.cuh"
